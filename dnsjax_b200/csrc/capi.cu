@@ -237,7 +237,9 @@ extern "C" int dnsb_periodic_create(const dnsb_periodic_desc* d,
     if (e1 || e2 || e3) rc = fail(DNSB_ERR_CUDA, "workspace allocation failed");
   }
   if (!rc) {
-    cudaError_t e = set_pass_attributes(smax);
+    cudaError_t e = cudaSuccess;
+    for (int L : {p->My, p->Mz, p->Mx})
+      if (e == cudaSuccess) e = set_pass_attributes(L, smax);
     if (e == cudaSuccess) e = set_solver_attributes(smax);
     if (e != cudaSuccess)
       rc = fail(DNSB_ERR_CUDA, std::string("cudaFuncSetAttribute: ") +
@@ -390,8 +392,7 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
   yi.tw = f32 ? reinterpret_cast<const double2*>(p->twy32) : p->twy;
   yi.fp32 = f32;
   yi.variant = p->var[0];
-  auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
-  if ((mask & 1u) && p->var[0] == 0 && fixed(p->My)) {
+  if ((mask & 1u) && p->var[0] == 0 && two_stage_length(p->My)) {
     // y inverse with the curl as a two-stage column pass: state
     // [comp][ky][kz][kx] -> A[f][y][kz][kx]
     ColPassArgs yc = periodic_ycurl(p, state);
@@ -435,7 +436,7 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
   yf.tw = f32 ? reinterpret_cast<const double2*>(p->twy32) : p->twy;
   yf.fp32 = f32;
   yf.variant = p->var[4];
-  if ((mask & 16u) && p->var[4] == 0 && fixed(p->My)) {
+  if ((mask & 16u) && p->var[4] == 0 && two_stage_length(p->My)) {
     // y forward as a two-stage column pass with truncation, A[f][y][kz][kx]
     // -> rhs[comp][ky][kz][kx] (complex128), then the projection in place
     ColPassArgs yc = periodic_yfwd_col(p, rhs);
@@ -461,8 +462,7 @@ extern "C" int dnsb_periodic_set_rhs_precision(dnsb_periodic* p, int fp32) {
   if (!p) return fail(DNSB_ERR_ARG, "null argument");
   if (fp32 && p->slab.nranks) return fail(DNSB_ERR_ARG, "slab contexts run the FP64 passes");
   if (fp32) {
-    auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
-    if (!fixed(p->My) || !fixed(p->Mz) || !fixed(p->Mx) || 3 * p->NKX != p->Mx)
+      if (!fp32_length(p->My) || !fp32_length(p->Mz) || !fp32_length(p->Mx) || 3 * p->NKX != p->Mx)
       return fail(DNSB_ERR_ARG,
                   "FP32 RHS passes need padded sizes in {48, 72, 96, 192} with nx_p = 3 nx / 2");
   }
@@ -712,8 +712,7 @@ static dnsb_step_graph* new_step_graph(size_t n) {
 // (the two-stage passes at the compiled sizes, the y forward as a column
 // pass plus the projection), at most max_iter; otherwise none.
 static int periodic_unroll(const dnsb_periodic* p, int max_iter) {
-  auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
-  if (p->graph_unroll <= 0 || !fixed(p->My) || !fixed(p->Mz) || !fixed(p->Mx) ||
+  if (p->graph_unroll <= 0 || !fp32_length(p->My) || !fp32_length(p->Mz) || !fp32_length(p->Mx) ||
       3 * p->NKX != p->Mx)
     return 0;
   for (int k = 0; k < 5; ++k)
@@ -1448,7 +1447,9 @@ extern "C" int dnsb_couette_create(const dnsb_couette_desc* d,
       rc = fail(DNSB_ERR_CUDA, "cudaMemset failed");
   }
   if (!rc) {
-    cudaError_t e = set_pass_attributes(smax);
+    cudaError_t e = cudaSuccess;
+    for (int L : {p->Mz, p->Mx})
+      if (e == cudaSuccess) e = set_pass_attributes(L, smax);
     if (e == cudaSuccess) e = set_solver_attributes(smax);
     if (e == cudaSuccess) e = set_imm_v2_attributes(smax);
     if (e == cudaSuccess) e = set_imm_batch_attributes(smax);
@@ -1659,8 +1660,7 @@ extern "C" int dnsb_couette_rhs(dnsb_couette* p, const void* state, void* rhs,
 // The FP32 passes are compiled for padded lengths 48, 72, 96 and 192 with
 // 3/2 oversampling in x.
 static bool couette_fp32_sizes(const dnsb_couette* p) {
-  auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
-  return fixed(p->Mz) && fixed(p->Mx) && 3 * p->NKX == p->Mx;
+  return fp32_length(p->Mz) && fp32_length(p->Mx) && 3 * p->NKX == p->Mx;
 }
 
 extern "C" int dnsb_couette_set_rhs_precision(dnsb_couette* p, int fp32) {
@@ -2519,7 +2519,6 @@ extern "C" int dnsb_banded_solve(const double* ab, const int* ipiv, double* b,
 // ===========================================================================
 static bool slab_sizes_ok(int nx_p, int nz_p, int nkxg, int nranks, int rank,
                           const char** why) {
-  auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
   if (nranks < 1 || nranks > kMaxRanks || rank < 0 || rank >= nranks) {
     *why = "nranks must be 1..8 and 0 <= rank < nranks";
     return false;
@@ -2528,7 +2527,7 @@ static bool slab_sizes_ok(int nx_p, int nz_p, int nkxg, int nranks, int rank,
     *why = "nx/2 and nz_p must be multiples of nranks";
     return false;
   }
-  if (!fixed(nx_p) || !fixed(nz_p) || 3 * nkxg != nx_p) {
+  if (!fp32_length(nx_p) || !fp32_length(nz_p) || 3 * nkxg != nx_p) {
     *why = "slab passes need padded sizes in {48, 72, 96, 192} with nx_p = 3 nx / 2";
     return false;
   }
@@ -2542,8 +2541,7 @@ extern "C" int dnsb_periodic_create_slab(const dnsb_periodic_desc* d, int nranks
   const int nkxg = d->nx / 2;
   const char* why = nullptr;
   if (!slab_sizes_ok(d->nx_p, d->nz_p, nkxg, nranks, rank, &why)) return fail(DNSB_ERR_ARG, why);
-  auto fixed = [](int L) { return L == 48 || L == 72 || L == 96 || L == 192; };
-  if (!fixed(d->ny_p)) return fail(DNSB_ERR_ARG, "slab passes need ny_p in {48, 72, 96, 192}");
+  if (!fp32_length(d->ny_p)) return fail(DNSB_ERR_ARG, "slab passes need ny_p in {48, 72, 96, 192}");
   // This rank's kx columns of the per-mode coefficients ([ky][kz][kx]).
   const int nkx = nkxg / nranks, ny1 = d->ny - 1, nz1 = d->nz - 1;
   std::vector<double> l1((size_t)ny1 * nz1 * nkx), l2(l1.size());

@@ -122,67 +122,26 @@ struct FFTPlan {
 };
 
 // ---- small DFTs in registers; sign = -1 forward, +1 inverse ------------
-// Generic over the complex type (double2, float2): the same operations in
-// either precision.
+// Generic over the value type: double2, float2, or cff (the compensated FP32
+// pair below); the same operations in each.
+// i * sign * v (exact)
 template <typename C>
-__device__ __forceinline__ void dft2(C* v) {
-  C a = v[0], b = v[1];
-  v[0] = cadd(a, b);
-  v[1] = csub(a, b);
+__device__ __forceinline__ C cisign(C v, int sign) {
+  return cmake<C>(-sign * v.y, sign * v.x);
 }
-
+// c v for a real constant c
 template <typename C>
-__device__ __forceinline__ void dft3(C* v, int sign) {
+__device__ __forceinline__ C cconst(C v, double c) {
+  return cscale(v, (typename cplx<C>::real)c);
+}
+// (c + i s) v for a constant
+template <typename C>
+__device__ __forceinline__ C crot(C v, double c, double s) {
   using R = typename cplx<C>::real;
-  const R s3 = (R)0.86602540378443864676;  // sin(2 pi / 3)
-  const R half = (R)0.5;
-  C t1 = cadd(v[1], v[2]);
-  C t2 = cmake<C>(v[0].x - half * t1.x, v[0].y - half * t1.y);
-  C d = csub(v[1], v[2]);
-  // i * sign * s3 * d
-  C t3 = cmake<C>(-sign * s3 * d.y, sign * s3 * d.x);
-  v[0] = cadd(v[0], t1);
-  v[1] = cadd(t2, t3);
-  v[2] = csub(t2, t3);
+  return cmake<C>(v.x * (R)c - v.y * (R)s, v.x * (R)s + v.y * (R)c);
 }
 
-template <typename C>
-__device__ __forceinline__ void dft4(C* v, int sign) {
-  C a = cadd(v[0], v[2]);
-  C b = csub(v[0], v[2]);
-  C c = cadd(v[1], v[3]);
-  C d = csub(v[1], v[3]);
-  // i * sign * d
-  C isd = cmake<C>(-sign * d.y, sign * d.x);
-  v[0] = cadd(a, c);
-  v[2] = csub(a, c);
-  v[1] = cadd(b, isd);
-  v[3] = csub(b, isd);
-}
-
-template <typename C>
-__device__ __forceinline__ void dft8(C* v, int sign) {
-  using R = typename cplx<C>::real;
-  const R h = (R)0.70710678118654752440;  // sqrt(2)/2
-  C e[4] = {v[0], v[2], v[4], v[6]};
-  C o[4] = {v[1], v[3], v[5], v[7]};
-  dft4(e, sign);
-  dft4(o, sign);
-  // twiddles w8^q = exp(sign * 2 pi i q / 8), q = 0..3
-  C t1 = cmake<C>(h * (o[1].x - sign * o[1].y), h * (o[1].y + sign * o[1].x));
-  C t2 = cmake<C>(-sign * o[2].y, sign * o[2].x);
-  C t3 = cmake<C>(h * (-o[3].x - sign * o[3].y), h * (-o[3].y + sign * o[3].x));
-  v[0] = cadd(e[0], o[0]);
-  v[4] = csub(e[0], o[0]);
-  v[1] = cadd(e[1], t1);
-  v[5] = csub(e[1], t1);
-  v[2] = cadd(e[2], t2);
-  v[6] = csub(e[2], t2);
-  v[3] = cadd(e[3], t3);
-  v[7] = csub(e[3], t3);
-}
-
-// ---- compensated FP32 butterflies (the cf2 overloads) -----------------------
+// ---- compensated FP32 values (the cf2 element type) -------------------------
 // Each FP32 value is carried as h + l: a sum or difference keeps its exact
 // rounding error (Knuth's two-sum) in l, a product by a constant keeps the
 // product's rounding error (from an FMA) and the constant's own FP32 rounding
@@ -212,6 +171,9 @@ __device__ __forceinline__ ffv ff_mulc(ffv a, float ch, float cl) {
   const float p = a.h * ch;
   return {p, fmaf(a.h, ch, -p) + (a.h * cl + a.l * ch)};
 }
+__device__ __forceinline__ ffv ff_mulc(ffv a, double c) {
+  return ff_mulc(a, (float)c, (float)(c - (double)(float)c));
+}
 struct cff {
   ffv x, y;
 };
@@ -219,86 +181,68 @@ __device__ __forceinline__ cff cff_of(float2 v) { return {{v.x, 0.0f}, {v.y, 0.0
 __device__ __forceinline__ cf2 cff_fold(cff v) {
   return cf2(make_float2(v.x.h + v.x.l, v.y.h + v.y.l));
 }
-__device__ __forceinline__ cff cff_add(cff a, cff b) { return {ff_add(a.x, b.x), ff_add(a.y, b.y)}; }
-__device__ __forceinline__ cff cff_sub(cff a, cff b) { return {ff_sub(a.x, b.x), ff_sub(a.y, b.y)}; }
-__device__ __forceinline__ cff cff_scale(cff a, float ch, float cl) {
-  return {ff_mulc(a.x, ch, cl), ff_mulc(a.y, ch, cl)};
-}
-// i * sign * a (exact)
-__device__ __forceinline__ cff cff_isign(cff a, int sign) {
+__device__ __forceinline__ cff cadd(cff a, cff b) { return {ff_add(a.x, b.x), ff_add(a.y, b.y)}; }
+__device__ __forceinline__ cff csub(cff a, cff b) { return {ff_sub(a.x, b.x), ff_sub(a.y, b.y)}; }
+__device__ __forceinline__ cff cisign(cff a, int sign) {
   const ffv nx = {-a.y.h, -a.y.l};
   return sign > 0 ? cff{nx, a.x} : cff{a.y, {-a.x.h, -a.x.l}};
 }
-// FP32 constant and its rounding error, evaluated in double at compile time.
-struct fconst {
-  float h, l;
-};
-__host__ __device__ constexpr fconst fsplit(double c) {
-  return {(float)c, (float)(c - (double)(float)c)};
+__device__ __forceinline__ cff cconst(cff a, double c) {
+  return {ff_mulc(a.x, c), ff_mulc(a.y, c)};
 }
-constexpr fconst kS3 = fsplit(0.86602540378443864676);  // sin(2 pi / 3)
-constexpr fconst kH8 = fsplit(0.70710678118654752440);  // sqrt(2) / 2
+__device__ __forceinline__ cff crot(cff a, double c, double s) {
+  return {ff_sub(ff_mulc(a.x, c), ff_mulc(a.y, s)), ff_add(ff_mulc(a.x, s), ff_mulc(a.y, c))};
+}
 
-__device__ __forceinline__ void cff_dft2(cff* v) {
-  const cff a = v[0], b = v[1];
-  v[0] = cff_add(a, b);
-  v[1] = cff_sub(a, b);
+template <typename V>
+__device__ __forceinline__ void dft2(V* v) {
+  const V a = v[0], b = v[1];
+  v[0] = cadd(a, b);
+  v[1] = csub(a, b);
 }
-__device__ __forceinline__ void cff_dft3(cff* v, int sign) {
-  const cff t1 = cff_add(v[1], v[2]);
-  const cff t2 = cff_sub(v[0], cff_scale(t1, 0.5f, 0.0f));
-  const cff t3 = cff_scale(cff_isign(cff_sub(v[1], v[2]), sign), kS3.h, kS3.l);
-  v[0] = cff_add(v[0], t1);
-  v[1] = cff_add(t2, t3);
-  v[2] = cff_sub(t2, t3);
+
+template <typename V>
+__device__ __forceinline__ void dft3(V* v, int sign) {
+  const V t1 = cadd(v[1], v[2]);
+  const V t2 = csub(v[0], cconst(t1, 0.5));
+  // sin(2 pi / 3)
+  const V t3 = cconst(cisign(csub(v[1], v[2]), sign), 0.86602540378443864676);
+  v[0] = cadd(v[0], t1);
+  v[1] = cadd(t2, t3);
+  v[2] = csub(t2, t3);
 }
-__device__ __forceinline__ void cff_dft4(cff* v, int sign) {
-  const cff a = cff_add(v[0], v[2]), b = cff_sub(v[0], v[2]);
-  const cff c = cff_add(v[1], v[3]), d = cff_sub(v[1], v[3]);
-  const cff isd = cff_isign(d, sign);
-  v[0] = cff_add(a, c);
-  v[2] = cff_sub(a, c);
-  v[1] = cff_add(b, isd);
-  v[3] = cff_sub(b, isd);
+
+template <typename V>
+__device__ __forceinline__ void dft4(V* v, int sign) {
+  const V a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
+  const V c = cadd(v[1], v[3]), d = csub(v[1], v[3]);
+  const V isd = cisign(d, sign);
+  v[0] = cadd(a, c);
+  v[2] = csub(a, c);
+  v[1] = cadd(b, isd);
+  v[3] = csub(b, isd);
 }
-__device__ __forceinline__ void cff_dft8(cff* v, int sign) {
-  cff e[4] = {v[0], v[2], v[4], v[6]};
-  cff o[4] = {v[1], v[3], v[5], v[7]};
-  cff_dft4(e, sign);
-  cff_dft4(o, sign);
+
+template <typename V>
+__device__ __forceinline__ void dft8(V* v, int sign) {
+  const double h = 0.70710678118654752440;  // sqrt(2)/2
+  V e[4] = {v[0], v[2], v[4], v[6]};
+  V o[4] = {v[1], v[3], v[5], v[7]};
+  dft4(e, sign);
+  dft4(o, sign);
   // twiddles w8^q = exp(sign 2 pi i q / 8): (1 + sign i) h, sign i, (-1 + sign i) h
-  const cff t1 = cff_scale(cff_add(o[1], cff_isign(o[1], sign)), kH8.h, kH8.l);
-  const cff t2 = cff_isign(o[2], sign);
-  const cff t3 = cff_scale(cff_sub(cff_isign(o[3], sign), o[3]), kH8.h, kH8.l);
-  v[0] = cff_add(e[0], o[0]);
-  v[4] = cff_sub(e[0], o[0]);
-  v[1] = cff_add(e[1], t1);
-  v[5] = cff_sub(e[1], t1);
-  v[2] = cff_add(e[2], t2);
-  v[6] = cff_sub(e[2], t2);
-  v[3] = cff_add(e[3], t3);
-  v[7] = cff_sub(e[3], t3);
+  const V t1 = cconst(cadd(o[1], cisign(o[1], sign)), h);
+  const V t2 = cisign(o[2], sign);
+  const V t3 = cconst(csub(cisign(o[3], sign), o[3]), h);
+  v[0] = cadd(e[0], o[0]);
+  v[4] = csub(e[0], o[0]);
+  v[1] = cadd(e[1], t1);
+  v[5] = csub(e[1], t1);
+  v[2] = cadd(e[2], t2);
+  v[6] = csub(e[2], t2);
+  v[3] = cadd(e[3], t3);
+  v[7] = csub(e[3], t3);
 }
-template <int P>
-__device__ __forceinline__ void cff_dft_small(cff* v, int sign) {
-  if constexpr (P == 2) cff_dft2(v);
-  else if constexpr (P == 3) cff_dft3(v, sign);
-  else if constexpr (P == 4) cff_dft4(v, sign);
-  else cff_dft8(v, sign);
-}
-template <int N>
-__device__ __forceinline__ void cf2_dft(cf2* v, int sign) {
-  cff w[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) w[i] = cff_of(v[i]);
-  cff_dft_small<N>(w, sign);
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = cff_fold(w[i]);
-}
-__device__ __forceinline__ void dft2(cf2* v) { cf2_dft<2>(v, 1); }
-__device__ __forceinline__ void dft3(cf2* v, int sign) { cf2_dft<3>(v, sign); }
-__device__ __forceinline__ void dft4(cf2* v, int sign) { cf2_dft<4>(v, sign); }
-__device__ __forceinline__ void dft8(cf2* v, int sign) { cf2_dft<8>(v, sign); }
 
 // One Stockham radix-R stage over C columns stored as buf[t * C + c].
 template <int R>
@@ -443,17 +387,7 @@ __device__ __forceinline__ CT* fft_cols(CT* a, CT* b, const FFTPlan& P, int sign
   }
 }
 
-// ---- register DFTs of size N = 3P (P in {2, 3, 4, 8}) --------------------
-// tw[m * TS] = exp(-2 pi i m / N) (a length-N*TS table); SIGN -1 forward,
-// +1 inverse; natural-order output in v.
-template <int P, typename C>
-__device__ __forceinline__ void dft_small(C* v, int sign) {
-  if constexpr (P == 2) dft2(v);
-  else if constexpr (P == 3) dft3(v, sign);
-  else if constexpr (P == 4) dft4(v, sign);
-  else dft8(v, sign);
-}
-
+// ---- register DFTs of composite size ---------------------------------------
 // Modular inverse of a mod m (a, m coprime), by search (compile time).
 __host__ __device__ constexpr int inv_mod(int a, int m) {
   int r = 1;
@@ -461,122 +395,154 @@ __host__ __device__ constexpr int inv_mod(int a, int m) {
   return r;
 }
 
+// cos(2 pi k / N) for the twiddles inside the 9-, 16- and 27-point DFTs
+// (a switch, so an unrolled index folds to the literal).
+template <int N>
+__host__ __device__ constexpr double cos_turn(int k) {
+  static_assert(27 % N == 0 || N == 16, "9, 16 and 27 points");
+  k = ((k % N) + N) % N;
+  k = k > N / 2 ? N - k : k;
+  if (N == 16) {
+    switch (k) {
+      case 0: return 1.0;
+      case 1: return 0.9238795325112867;
+      case 2: return 0.7071067811865476;
+      case 3: return 0.3826834323650898;
+      case 4: return 0.0;
+      case 5: return -0.3826834323650898;
+      case 6: return -0.7071067811865476;
+      case 7: return -0.9238795325112867;
+      default: return -1.0;
+    }
+  }
+  switch (k * (27 / N)) {
+    case 0: return 1.0;
+    case 1: return 0.9730448705798238;
+    case 2: return 0.8936326403234123;
+    case 3: return 0.766044443118978;
+    case 4: return 0.5971585917027862;
+    case 5: return 0.39607976603915684;
+    case 6: return 0.17364817766693036;
+    case 7: return -0.05814482891047583;
+    case 8: return -0.28680323271109026;
+    case 9: return -0.5;
+    case 10: return -0.6862416378687336;
+    case 11: return -0.8354878114129364;
+    case 12: return -0.9396926207859084;
+    default: return -0.993238357741943;
+  }
+}
+// sin(2 pi k / N)
+template <int N>
+__host__ __device__ constexpr double sin_turn(int k) {
+  k = ((k % N) + N) % N;
+  const double sg = 2 * k > N ? -1.0 : 1.0;
+  k = 2 * k > N ? N - k : k;
+  if (N == 16) return sg * cos_turn<16>(k - 4);
+  switch (k * (27 / N)) {
+    case 0: return 0.0;
+    case 1: return sg * 0.23061587074244017;
+    case 2: return sg * 0.44879918020046217;
+    case 3: return sg * 0.6427876096865394;
+    case 4: return sg * 0.8021231927550437;
+    case 5: return sg * 0.918216106880274;
+    case 6: return sg * 0.984807753012208;
+    case 7: return sg * 0.9983081582712682;
+    case 8: return sg * 0.9579895123154889;
+    case 9: return sg * 0.8660254037844386;
+    case 10: return sg * 0.7273736415730487;
+    case 11: return sg * 0.549508978070806;
+    case 12: return sg * 0.3420201433256687;
+    default: return sg * 0.11609291412523023;
+  }
+}
+
+// Natural-order DFT of N values in registers, SIGN -1 forward, +1 inverse.
+// N = A B with A, B coprime: the prime-factor (Good-Thomas) form, no twiddles:
+// input n = (B n1 + A n2) mod N, output k = (B (B^-1 mod A) k1 + A (A^-1 mod B)
+// k2) mod N.  9, 16 and 27 points: Cooley-Tukey with constant twiddles.
+template <int N, int SIGN, typename V>
+__device__ __forceinline__ void dft_n(V* v);
+
+template <int A, int B, int SIGN, typename V>
+__device__ __forceinline__ void dft_pfa(V* v) {
+  constexpr int N = A * B;
+  constexpr int KA = B * inv_mod(B % A, A), KB = A * inv_mod(A % B, B);
+  V a[B][A];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2)
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) a[n2][n1] = v[(B * n1 + A * n2) % N];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) dft_n<A, SIGN>(a[n2]);
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    V b[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) b[n2] = a[n2][k1];
+    dft_n<B, SIGN>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) v[(KA * k1 + KB * k2) % N] = b[k2];
+  }
+}
+
+template <int A, int B, int SIGN, typename V>
+__device__ __forceinline__ void dft_ct(V* v) {
+  constexpr int N = A * B;
+  V a[B][A];
+#pragma unroll
+  for (int b = 0; b < B; ++b)
+#pragma unroll
+    for (int n = 0; n < A; ++n) a[b][n] = v[B * n + b];
+#pragma unroll
+  for (int b = 0; b < B; ++b) dft_n<A, SIGN>(a[b]);
+#pragma unroll
+  for (int b = 1; b < B; ++b)
+#pragma unroll
+    for (int k = 1; k < A; ++k) {
+      if (N == 16 && b * k == 4) a[b][k] = cisign(a[b][k], SIGN);
+      else a[b][k] = crot(a[b][k], cos_turn<N>(b * k), SIGN * sin_turn<N>(b * k));
+    }
+#pragma unroll
+  for (int k = 0; k < A; ++k) {
+    V c[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) c[b] = a[b][k];
+    dft_n<B, SIGN>(c);
+#pragma unroll
+    for (int b = 0; b < B; ++b) v[k + A * b] = c[b];
+  }
+}
+
+template <int N, int SIGN, typename V>
+__device__ __forceinline__ void dft_n(V* v) {
+  if constexpr (N == 2) dft2(v);
+  else if constexpr (N == 3) dft3(v, SIGN);
+  else if constexpr (N == 4) dft4(v, SIGN);
+  else if constexpr (N == 8) dft8(v, SIGN);
+  else if constexpr (N == 9) dft_ct<3, 3, SIGN>(v);
+  else if constexpr (N == 16) dft_ct<4, 4, SIGN>(v);
+  else if constexpr (N == 27) dft_ct<9, 3, SIGN>(v);
+  else if constexpr (N == 18) dft_pfa<9, 2, SIGN>(v);
+  else {
+    static_assert(N == 6 || N == 12 || N == 24, "no register DFT of this size");
+    dft_pfa<N / 3, 3, SIGN>(v);
+  }
+}
+
+// The same on the pass kernels' element types: cf2 runs it on compensated
+// values.
 template <int N, int SIGN, typename C>
-__device__ __forceinline__ void dft_3p_ct(C* v, const C* __restrict__ tw, int TS);
-
-// PFA: with 3 and P coprime, the prime-factor form (no twiddles); else the
-// Cooley-Tukey form with the twiddle table.
-template <int N, int SIGN, bool PFA>
-__device__ __forceinline__ void dft_3p_comp(cf2* v, const cf2* __restrict__ tw, int TS);
-
-template <int N, int SIGN, typename C, bool PFA = false>
-__device__ __forceinline__ void dft_3p(C* v, const C* __restrict__ tw, int TS) {
-  constexpr int P = N / 3;
+__device__ __forceinline__ void dft_reg(C* v) {
   if constexpr (std::is_same<C, cf2>::value) {
-    dft_3p_comp<N, SIGN, PFA>(v, tw, TS);
-  } else if constexpr (PFA && P % 3 != 0) {
-    // 3 and P coprime: prime-factor (Good-Thomas) DFT, no twiddles.  Input
-    // n = (P n1 + 3 n2) mod N; P-point DFTs over n2, 3-point DFTs over n1;
-    // output k = (P (P^-1 mod 3) k1 + 3 (3^-1 mod P) k2) mod N (Chinese
-    // remainder map).
-    constexpr int A = P * inv_mod(P % 3, 3), B = 3 * inv_mod(3 % P, P);
-    (void)tw;
-    (void)TS;
-    C a[3][P];
+    cff w[N];
 #pragma unroll
-    for (int n1 = 0; n1 < 3; ++n1)
+    for (int i = 0; i < N; ++i) w[i] = cff_of(v[i]);
+    dft_n<N, SIGN>(w);
 #pragma unroll
-      for (int n2 = 0; n2 < P; ++n2) a[n1][n2] = v[(P * n1 + 3 * n2) % N];
-#pragma unroll
-    for (int n1 = 0; n1 < 3; ++n1) dft_small<P>(a[n1], SIGN);
-#pragma unroll
-    for (int k2 = 0; k2 < P; ++k2) {
-      C b[3] = {a[0][k2], a[1][k2], a[2][k2]};
-      dft3(b, SIGN);
-#pragma unroll
-      for (int k1 = 0; k1 < 3; ++k1) v[(A * k1 + B * k2) % N] = b[k1];
-    }
+    for (int i = 0; i < N; ++i) v[i] = cff_fold(w[i]);
   } else {
-    dft_3p_ct<N, SIGN>(v, tw, TS);
-  }
-}
-
-template <int N, int SIGN, typename C>
-__device__ __forceinline__ void dft_3p_ct(C* v, const C* __restrict__ tw, int TS) {
-  constexpr int P = N / 3;
-  C a[3][P];
-#pragma unroll
-  for (int q = 0; q < 3; ++q)
-#pragma unroll
-    for (int p = 0; p < P; ++p) a[q][p] = v[3 * p + q];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) dft_small<P>(a[q], SIGN);
-#pragma unroll
-  for (int q = 1; q < 3; ++q)
-#pragma unroll
-    for (int k1 = 1; k1 < P; ++k1) {
-      C w = tw[(q * k1) * TS];
-      if (SIGN > 0) w.y = -w.y;
-      a[q][k1] = cmul(a[q][k1], w);
-    }
-#pragma unroll
-  for (int k1 = 0; k1 < P; ++k1) {
-    C b[3] = {a[0][k1], a[1][k1], a[2][k1]};
-    dft3(b, SIGN);
-#pragma unroll
-    for (int k2 = 0; k2 < 3; ++k2) v[k1 + P * k2] = b[k2];
-  }
-}
-
-// The compensated form of dft_3p: the P-point and 3-point DFTs (and, in the
-// Cooley-Tukey form, the twiddle products between them) stay in h + l
-// until the outputs are stored.
-template <int N, int SIGN, bool PFA>
-__device__ __forceinline__ void dft_3p_comp(cf2* v, const cf2* __restrict__ tw, int TS) {
-  constexpr int P = N / 3;
-  cff a[3][P];
-  if constexpr (PFA && P % 3 != 0) {
-    constexpr int A = P * inv_mod(P % 3, 3), B = 3 * inv_mod(3 % P, P);
-    (void)tw;
-    (void)TS;
-#pragma unroll
-    for (int n1 = 0; n1 < 3; ++n1)
-#pragma unroll
-      for (int n2 = 0; n2 < P; ++n2) a[n1][n2] = cff_of(v[(P * n1 + 3 * n2) % N]);
-#pragma unroll
-    for (int n1 = 0; n1 < 3; ++n1) cff_dft_small<P>(a[n1], SIGN);
-#pragma unroll
-    for (int k2 = 0; k2 < P; ++k2) {
-      cff b[3] = {a[0][k2], a[1][k2], a[2][k2]};
-      cff_dft3(b, SIGN);
-#pragma unroll
-      for (int k1 = 0; k1 < 3; ++k1) v[(A * k1 + B * k2) % N] = cff_fold(b[k1]);
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-      for (int p = 0; p < P; ++p) a[q][p] = cff_of(v[3 * p + q]);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) cff_dft_small<P>(a[q], SIGN);
-#pragma unroll
-    for (int q = 1; q < 3; ++q)
-#pragma unroll
-      for (int k1 = 1; k1 < P; ++k1) {
-        float2 w = tw[(q * k1) * TS];
-        if (SIGN > 0) w.y = -w.y;
-        // (x + i y)(wx + i wy) with each product's rounding error kept
-        const cff z = a[q][k1];
-        a[q][k1] = {ff_sub(ff_mulc(z.x, w.x, 0.0f), ff_mulc(z.y, w.y, 0.0f)),
-                    ff_add(ff_mulc(z.x, w.y, 0.0f), ff_mulc(z.y, w.x, 0.0f))};
-      }
-#pragma unroll
-    for (int k1 = 0; k1 < P; ++k1) {
-      cff b[3] = {a[0][k1], a[1][k1], a[2][k1]};
-      cff_dft3(b, SIGN);
-#pragma unroll
-      for (int k2 = 0; k2 < 3; ++k2) v[k1 + P * k2] = cff_fold(b[k2]);
-    }
+    dft_n<N, SIGN>(v);
   }
 }
 

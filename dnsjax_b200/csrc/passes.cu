@@ -8,6 +8,8 @@
 // src/dnsjax/flows/monochromatic.py:366-386 (projection).
 #include "passes.cuh"
 
+#include <initializer_list>
+
 namespace dnsb {
 
 // Transform lengths with a compile-time FFT plan; others use the runtime
@@ -28,9 +30,6 @@ namespace dnsb {
     else                                                                    \
       DNSB_DISPATCH(L, KERNEL, GRID, SMEM, ST, __VA_ARGS__);                \
   } while (0)
-#define DNSB_ALL_SIZES(KERNEL)                                                \
-  (const void*)KERNEL<0>, (const void*)KERNEL<48>, (const void*)KERNEL<72>,   \
-      (const void*)KERNEL<96>, (const void*)KERNEL<192>
 
 FFTPlan make_plan(int L) {
   FFTPlan P{};
@@ -119,16 +118,59 @@ col_pass_kernel(ColPassArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Column pass, two register stages (M = 8 R1): stage 1 (radix R1, Ns = 1)
-// loads its inputs from global memory (zero-padding applied on load),
-// stage 2 (radix 8, Ns = R1) stores its outputs to global memory
-// (truncation applied on store); one shared buffer in between.
+// Column pass, two register stages (M = R1 R2): stage 1 (radix R1, Ns = 1)
+// loads its inputs from global memory (zero-padding applied on load), stage 2
+// (radix R2, Ns = R1) stores its outputs to global memory (truncation applied
+// on store); one shared buffer in between.  A CTA takes C columns with one
+// thread per stage-1 item.
+//
+// Shapes: R1 >= R2 as balanced as the register file allows (R1 <= 24 complex
+// values a thread), 16 columns (256-byte runs), 8 where 16 would leave two
+// CTAs per SM (M = 288, 384).  Against the Stockham stages with one radix <= 8
+// exchange each that the lengths beyond 48, 72, 96 and 192 ran before, one
+// shared-memory round trip replaces three to five: the four column passes of a
+// 256^3 periodic RHS (M = 384) took 5.3 ms, now 2.0 ms (all the passes of a
+// 144 x 192 x 108 predict_and_correct: 3.36 -> 2.25 ms).
 // ---------------------------------------------------------------------------
-constexpr int kC2Cols = 16;
-constexpr int kC2Threads = 128;
+constexpr int col_columns(int L) { return L >= 288 ? 8 : 16; }
+template <int M>
+struct ColShape;
+#define DNSB_COL_SHAPE(M_, R1_, R2_, C_, ZB_)                                     \
+  template <>                                                                     \
+  struct ColShape<M_> {                                                           \
+    static constexpr int R1 = R1_, R2 = R2_, C = C_, NT = R2_ * C_, ZB = ZB_;     \
+    static_assert(R1 * R2 == M_ && C == col_columns(M_), "two radices");          \
+  };
+// ZB: CTAs per SM that the Couette z inverse's registers are held to
+DNSB_COL_SHAPE(36, 6, 6, 16, 5)
+DNSB_COL_SHAPE(48, 6, 8, 16, 4)
+DNSB_COL_SHAPE(54, 9, 6, 16, 5)
+DNSB_COL_SHAPE(72, 9, 8, 16, 4)
+DNSB_COL_SHAPE(96, 12, 8, 16, 4)
+DNSB_COL_SHAPE(108, 12, 9, 16, 3)
+DNSB_COL_SHAPE(144, 12, 12, 16, 3)
+DNSB_COL_SHAPE(162, 18, 9, 16, 3)
+DNSB_COL_SHAPE(192, 24, 8, 16, 4)
+DNSB_COL_SHAPE(216, 18, 12, 16, 2)
+DNSB_COL_SHAPE(288, 24, 12, 8, 4)
+DNSB_COL_SHAPE(384, 24, 16, 8, 4)
+#undef DNSB_COL_SHAPE
+
+// f(std::integral_constant<int, L>) for a two-stage length L.
+template <typename F>
+static cudaError_t with_length(int L, F&& f) {
+  switch (L) {
+#define DNSB_LEN(LL) \
+  case LL: return f(std::integral_constant<int, LL>{});
+    DNSB_LEN(36) DNSB_LEN(48) DNSB_LEN(54) DNSB_LEN(72) DNSB_LEN(96) DNSB_LEN(108)
+    DNSB_LEN(144) DNSB_LEN(162) DNSB_LEN(192) DNSB_LEN(216) DNSB_LEN(288) DNSB_LEN(384)
+#undef DNSB_LEN
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 size_t col_pass2_smem(int M) {
-  return sizeof(double2) * (size_t)(M * kC2Cols + M);
+  return sizeof(double2) * (size_t)(M * col_columns(M) + M);
 }
 
 // T: the compute type and the element type of `in` (double, or float for the
@@ -141,7 +183,8 @@ template <int ML, int SIGN, typename T = double, bool OUT32 = false, bool CURL =
 __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int by, int bz) {
   using CT = typename pass_types<T>::C;
   using RT = typename pass_types<T>::R;
-  constexpr int M = ML, R1 = M / 8, C = kC2Cols;
+  constexpr int M = ML, R1 = ColShape<ML>::R1, R2 = ColShape<ML>::R2, C = ColShape<ML>::C;
+  constexpr int NT = ColShape<ML>::NT;
   extern __shared__ double2 sm_[];
   CT* X = reinterpret_cast<CT*>(sm_);  // [t][C]
   CT* tw = X + M * C;
@@ -157,12 +200,12 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
   const unsigned long long drop = l2_drop();
   load_twiddles(tw, reinterpret_cast<const CT*>(a.tw), M);
   __syncthreads();
-  for (int it = tid; it < 8 * C; it += kC2Threads) {
-    const int c = it % C, j = it / C;
+  {
+    const int c = tid % C, j = tid / C;
     CT v[R1];
 #pragma unroll
     for (int i = 0; i < R1; ++i) {
-      const int t = j + 8 * i;
+      const int t = j + R2 * i;
       CT z = cmake<CT>(0, 0);
       if (c < ni) {
         if (SIGN > 0) {
@@ -209,27 +252,27 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
       }
       v[i] = z;
     }
-    dft_3p<R1, SIGN>(v, tw, 8);
+    dft_reg<R1, SIGN>(v);
 #pragma unroll
     for (int i = 0; i < R1; ++i) X[(j * R1 + i) * C + c] = v[i];
   }
   __syncthreads();
   const double sc = 1.0 / M;
-  for (int it = tid; it < R1 * C; it += kC2Threads) {
+  for (int it = tid; it < R1 * C; it += NT) {
     const int c = it % C, k = it / C;
-    CT z[8];
+    CT z[R2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) z[i] = X[(k + R1 * i) * C + c];
+    for (int i = 0; i < R2; ++i) z[i] = X[(k + R1 * i) * C + c];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) {
+    for (int i = 1; i < R2; ++i) {
       CT w = tw[i * k];
       if (SIGN > 0) w.y = -w.y;
       z[i] = cmul(z[i], w);
     }
-    dft8(z, SIGN);
+    dft_reg<R2, SIGN>(z);
     if (c < ni) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < R2; ++i) {
         const int t = k + R1 * i;
         if (SIGN > 0) {
           if constexpr (SLAB) {
@@ -255,21 +298,22 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
 }
 
 // Block (bx, by, bz) = (column tile, outer index, field) of the grid
-// ((nI + 15) / 16, nO, nfields); the work-list ensemble kernels call the body
+// ((nI + C - 1) / C, nO, nfields); the work-list ensemble kernels call the body
 // with their own block numbering.
 template <int ML, int SIGN, typename T = double, bool OUT32 = false, bool CURL = false,
           bool SLAB = false>
-__global__ void __launch_bounds__(kC2Threads)
+__global__ void __launch_bounds__(ColShape<ML>::NT)
 col_pass2_kernel(ColPassArgs a) {
   if (a.skip && *a.skip) return;
   col_pass2_body<ML, SIGN, T, OUT32, CURL, SLAB>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// The FP64 pass held to 128 registers, so 4 CTAs fit per SM instead of 3
-// (ColPassArgs::occ4: the periodic flows' column passes, measured faster so;
-// the Couette z forward measured slower).
+// The FP64 pass held to 512 threads' worth of 128 registers per SM, so 4 CTAs
+// of 128 threads fit instead of 3 (ColPassArgs::occ4: the periodic flows'
+// column passes, measured faster so; the Couette z forward at 192 measured
+// slower, the lengths compiled for FP64 alone take it always).
 template <int ML, int SIGN, bool CURL>
-__global__ void __launch_bounds__(kC2Threads, 4)
+__global__ void __launch_bounds__(ColShape<ML>::NT, 512 / ColShape<ML>::NT)
 col_pass2_occ4_kernel(ColPassArgs a) {
   if (a.skip && *a.skip) return;
   col_pass2_body<ML, SIGN, double, false, CURL, false>(a, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -278,48 +322,51 @@ col_pass2_occ4_kernel(ColPassArgs a) {
 cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
                             cudaStream_t st) {
   const int L = a.plan.L;
-  if (a.variant == 0 && (L == 48 || L == 72 || L == 96 || L == 192)) {
-    dim3 g2((a.nI + kC2Cols - 1) / kC2Cols, nO, nfields);
+  if (a.variant == 0 && two_stage_length(L)) {
+    const int C = col_columns(L);
+    const dim3 g2((a.nI + C - 1) / C, nO, nfields);
     const size_t sm2 = a.fp32 ? col_pass2_smem(L) / 2 : col_pass2_smem(L);
-    if (a.fp32 && a.inverse && !a.out32) return cudaErrorInvalidValue;
     const bool slab = a.slab.buf[0] != nullptr;
+    if ((a.fp32 || slab) && !fp32_length(L)) return cudaErrorInvalidValue;
+    if (a.fp32 && a.inverse && !a.out32) return cudaErrorInvalidValue;
     if (slab && (a.fp32 || a.curl || !a.inverse)) return cudaErrorInvalidValue;
-#define DNSB_C2(LL)                                                                     \
-  case LL:                                                                              \
-    if (slab)                                                                           \
-      col_pass2_kernel<LL, 1, double, false, false, true><<<g2, kC2Threads, sm2, st>>>(a); \
-    else if (a.curl && a.fp32 == 2)                                                     \
-      col_pass2_kernel<LL, 1, fcomp, true, true><<<g2, kC2Threads, sm2, st>>>(a);       \
-    else if (a.fp32 == 2 && a.inverse)                                                  \
-      col_pass2_kernel<LL, 1, fcomp, true><<<g2, kC2Threads, sm2, st>>>(a);             \
-    else if (a.fp32 == 2 && a.out32)                                                    \
-      col_pass2_kernel<LL, -1, fcomp, true><<<g2, kC2Threads, sm2, st>>>(a);            \
-    else if (a.fp32 == 2)                                                               \
-      col_pass2_kernel<LL, -1, fcomp><<<g2, kC2Threads, sm2, st>>>(a);                  \
-    else if (a.curl && a.fp32)                                                          \
-      col_pass2_kernel<LL, 1, float, true, true><<<g2, kC2Threads, sm2, st>>>(a);       \
-    else if (a.occ4 && !a.fp32 && a.curl)                                               \
-      col_pass2_occ4_kernel<LL, 1, true><<<g2, kC2Threads, sm2, st>>>(a);               \
-    else if (a.occ4 && !a.fp32 && a.inverse)                                            \
-      col_pass2_occ4_kernel<LL, 1, false><<<g2, kC2Threads, sm2, st>>>(a);              \
-    else if (a.occ4 && !a.fp32)                                                         \
-      col_pass2_occ4_kernel<LL, -1, false><<<g2, kC2Threads, sm2, st>>>(a);             \
-    else if (a.curl)                                                                    \
-      col_pass2_kernel<LL, 1, double, false, true><<<g2, kC2Threads, sm2, st>>>(a);     \
-    else if (a.fp32 && a.inverse)                                                       \
-      col_pass2_kernel<LL, 1, float, true><<<g2, kC2Threads, sm2, st>>>(a);             \
-    else if (a.fp32 && a.out32)                                                         \
-      col_pass2_kernel<LL, -1, float, true><<<g2, kC2Threads, sm2, st>>>(a);            \
-    else if (a.fp32)                                                                    \
-      col_pass2_kernel<LL, -1, float><<<g2, kC2Threads, sm2, st>>>(a);                  \
-    else if (a.inverse)                                                                 \
-      col_pass2_kernel<LL, 1><<<g2, kC2Threads, sm2, st>>>(a);                          \
-    else                                                                                \
-      col_pass2_kernel<LL, -1><<<g2, kC2Threads, sm2, st>>>(a);                         \
-    break;
-    switch (L) { DNSB_C2(48) DNSB_C2(72) DNSB_C2(96) DNSB_C2(192) }
-#undef DNSB_C2
-    return cudaGetLastError();
+    return with_length(L, [&](auto len) {
+      constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;
+      if constexpr (fp32_length(LL)) {
+        if (slab)
+          col_pass2_kernel<LL, 1, double, false, false, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.curl && a.fp32 == 2)
+          col_pass2_kernel<LL, 1, fcomp, true, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32 == 2 && a.inverse)
+          col_pass2_kernel<LL, 1, fcomp, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32 == 2 && a.out32)
+          col_pass2_kernel<LL, -1, fcomp, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32 == 2)
+          col_pass2_kernel<LL, -1, fcomp><<<g2, NT, sm2, st>>>(a);
+        else if (a.curl && a.fp32)
+          col_pass2_kernel<LL, 1, float, true, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32 && a.inverse)
+          col_pass2_kernel<LL, 1, float, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32 && a.out32)
+          col_pass2_kernel<LL, -1, float, true><<<g2, NT, sm2, st>>>(a);
+        else if (a.fp32)
+          col_pass2_kernel<LL, -1, float><<<g2, NT, sm2, st>>>(a);
+        else if (!a.occ4 && a.curl)
+          col_pass2_kernel<LL, 1, double, false, true><<<g2, NT, sm2, st>>>(a);
+        else if (!a.occ4 && a.inverse)
+          col_pass2_kernel<LL, 1><<<g2, NT, sm2, st>>>(a);
+        else if (!a.occ4)
+          col_pass2_kernel<LL, -1><<<g2, NT, sm2, st>>>(a);
+        if (slab || a.fp32 || !a.occ4) return cudaGetLastError();
+      }
+      if (a.curl)
+        col_pass2_occ4_kernel<LL, 1, true><<<g2, NT, sm2, st>>>(a);
+      else if (a.inverse)
+        col_pass2_occ4_kernel<LL, 1, false><<<g2, NT, sm2, st>>>(a);
+      else
+        col_pass2_occ4_kernel<LL, -1, false><<<g2, NT, sm2, st>>>(a);
+      return cudaGetLastError();
+    });
   }
   // two-stage compile-time passes only
   if (a.fp32 || a.curl || a.slab.buf[0]) return cudaErrorInvalidValue;
@@ -659,7 +706,7 @@ __device__ __forceinline__ void x_pass2_body(const XPassArgs& a, int bx) {
     }
     __syncthreads();  // S read by every thread before X is written over it
     if (act) {
-      dft_3p<R1, 1, CT, true>(v, tw, 8);
+      dft_reg<R1, 1>(v);
 #pragma unroll
       for (int i = 0; i < R1; ++i) X[(j * R1 + i) * CI + col + XS * j] = v[i];
     }
@@ -684,7 +731,7 @@ __device__ __forceinline__ void x_pass2_body(const XPassArgs& a, int bx) {
           w.y = -w.y;
           z[pr][i] = cmul(z[pr][i], w);
         }
-        dft8(z[pr], 1);
+        dft_reg<8, 1>(z[pr]);
       }
       const bool live = r < nr;
       const int y = s_y[r];
@@ -708,8 +755,8 @@ __device__ __forceinline__ void x_pass2_body(const XPassArgs& a, int bx) {
         F0[i] = live ? cmake<CT>(n0 + b0, n1 + b1) : cmake<CT>(0, 0);
         F1[i] = live ? cmake<CT>(n2 + b2, 0) : cmake<CT>(0, 0);
       }
-      dft8(F0, -1);
-      dft8(F1, -1);
+      dft_reg<8, -1>(F0);
+      dft_reg<8, -1>(F1);
     }
     __syncthreads();  // X read by every thread before Y is written over it
     if (act) {
@@ -738,7 +785,7 @@ __device__ __forceinline__ void x_pass2_body(const XPassArgs& a, int bx) {
     if (act) {
 #pragma unroll
       for (int i = 1; i < R1; ++i) v[i] = cmul(v[i], tw[i * j]);
-      dft_3p<R1, -1, CT, true>(v, tw, 8);
+      dft_reg<R1, -1>(v);
 #pragma unroll
       for (int i = 0; i < R1; ++i) X[xrow(j + 8 * i) + col] = v[i];
     }
@@ -802,8 +849,14 @@ __device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int
   return lo;
 }
 
+// the fp32_length lengths all run 128 threads on 16 columns
+constexpr int kEnsColThreads = ColShape<192>::NT;
+static_assert(ColShape<48>::NT == kEnsColThreads && ColShape<72>::NT == kEnsColThreads &&
+                  ColShape<96>::NT == kEnsColThreads,
+              "one CTA shape for every member");
+
 template <int SIGN, bool CURL>
-__global__ void __launch_bounds__(kC2Threads)
+__global__ void __launch_bounds__(kEnsColThreads)
 ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict__ base, int n,
                      int total, const int* __restrict__ active) {
   __shared__ int s_k;
@@ -850,10 +903,11 @@ ens_x_pass2_kernel(const EnsXItem* __restrict__ items, const int* __restrict__ b
   }
 }
 
-bool ens_pass_supported(int L) { return L == 48 || L == 72 || L == 96 || L == 192; }
+bool ens_pass_supported(int L) { return fp32_length(L); }
 
 int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy) {
-  *gx = (a.nI + kC2Cols - 1) / kC2Cols;
+  const int C = col_columns(a.plan.L);
+  *gx = (a.nI + C - 1) / C;
   *gy = nO;
   return *gx * nO * nfields;
 }
@@ -879,7 +933,7 @@ int ens_pass_grid(int kind, size_t smem, int total, int max_smem) {
   const void* f = ens_kernel(kind);
   if (allow_dynamic_smem(f, max_smem) != cudaSuccess) return 0;
   int per_sm = 0, dev = 0, nsm = 0;
-  const int threads = kind == 3 ? kX2Threads : kC2Threads;
+  const int threads = kind == 3 ? kX2Threads : kEnsColThreads;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess)
     return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -893,15 +947,15 @@ cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n,
                             const int* active, int grid, size_t smem, cudaStream_t st) {
   switch (kind) {
     case 0:
-      ens_col_pass2_kernel<1, true><<<grid, kC2Threads, smem, st>>>(
+      ens_col_pass2_kernel<1, true><<<grid, kEnsColThreads, smem, st>>>(
           static_cast<const EnsColItem*>(items), base, n, total, active);
       break;
     case 1:
-      ens_col_pass2_kernel<1, false><<<grid, kC2Threads, smem, st>>>(
+      ens_col_pass2_kernel<1, false><<<grid, kEnsColThreads, smem, st>>>(
           static_cast<const EnsColItem*>(items), base, n, total, active);
       break;
     case 2:
-      ens_col_pass2_kernel<-1, false><<<grid, kC2Threads, smem, st>>>(
+      ens_col_pass2_kernel<-1, false><<<grid, kEnsColThreads, smem, st>>>(
           static_cast<const EnsColItem*>(items), base, n, total, active);
       break;
     default:
@@ -1405,39 +1459,36 @@ zinv_curl_kernel(ZInvCurlArgs a, int span_max) {
 }
 
 // ---------------------------------------------------------------------------
-// Couette z-inverse pass, two register stages (M = 8 R1): a CTA takes 16
-// consecutive (kx, y) columns -- contiguous in the (nz-1, nx/2, ny) layout --
-// fills each field's zero-padded z column into shared memory (all of a
-// thread's loads of a batch in flight together), runs the inverse radix-R1
-// stage in registers, exchanges once through shared memory, and stores the
-// inverse radix-8 stage's outputs straight to global memory.
+// Couette z-inverse pass, two register stages (M = R1 R2, the shapes of the
+// column pass): a CTA takes C consecutive (kx, y) columns -- contiguous in the
+// (nz-1, nx/2, ny) layout -- fills each field's zero-padded z column into
+// shared memory (all of a thread's loads of a batch in flight together), runs
+// the inverse radix-R1 stage in registers, exchanges once through shared
+// memory, and stores the inverse radix-R2 stage's outputs straight to global
+// memory.
 // ---------------------------------------------------------------------------
-constexpr int kZ2Cols = 16;
-constexpr int kZ2Threads = 8 * kZ2Cols;  // stage 1: one thread per (j, column)
-
-size_t zinv_curl2_smem(int M) {
-  return sizeof(double2) * (size_t)(M * kZ2Cols + M);
-}
+size_t zinv_curl2_smem(int M) { return col_pass2_smem(M); }
 
 template <int M, int F, typename CT>
 __device__ __forceinline__ void zinv2_fill(const ZInvCurlArgs& a, CT* X,
                                            const double2* U, const double2* V,
                                            const double2* Wc, long long sstride,
                                            int y, double kx, bool live) {
-  constexpr int NE = M * kZ2Cols / kZ2Threads;  // elements per thread (= M / 8)
+  constexpr int C = ColShape<M>::C, NT = ColShape<M>::NT;
+  constexpr int NE = M * C / NT;  // elements per thread (= R1)
   constexpr int B = (NE % 6 == 0) ? 6 : ((NE % 3 == 0) ? 3 : 1);
   const int tid = threadIdx.x;
   for (int e0 = 0; e0 < NE; e0 += B) {
     double2 v[B];
 #pragma unroll
     for (int e = 0; e < B; ++e) {
-      const int t = (tid + (e0 + e) * kZ2Threads) / kZ2Cols;
+      const int t = (tid + (e0 + e) * NT) / C;
       const int s = pos_to_stored(t, a.NZ1, M);
       v[e] = make_double2(0.0, 0.0);
       if (live && s >= 0) v[e] = zinv_field<F>(a, U, V, Wc, s * sstride, s, y, kx);
     }
 #pragma unroll
-    for (int e = 0; e < B; ++e) X[tid + (e0 + e) * kZ2Threads] = to_c(v[e], (CT*)nullptr);
+    for (int e = 0; e < B; ++e) X[tid + (e0 + e) * NT] = to_c(v[e], (CT*)nullptr);
   }
 }
 
@@ -1445,12 +1496,14 @@ __device__ __forceinline__ void zinv2_fill(const ZInvCurlArgs& a, CT* X,
 // (double, or float for the FP32 form of the Couette RHS); the state is
 // read, and the curl's fill computed, in FP64.
 template <int ML, typename T = double, bool SLAB = false>
-__global__ void __launch_bounds__(kZ2Threads, std::is_same<T, float>::value ? 6 : 4)
+__global__ void __launch_bounds__(ColShape<ML>::NT,
+                                  std::is_same<T, float>::value ? 6 : ColShape<ML>::ZB)
 zinv_curl2_kernel(ZInvCurlArgs a) {
   if (a.skip && *a.skip) return;
   using CT = typename pass_types<T>::C;
   using RT = typename pass_types<T>::R;
-  constexpr int M = ML, R1 = M / 8, C = kZ2Cols;
+  constexpr int M = ML, R1 = ColShape<ML>::R1, R2 = ColShape<ML>::R2, C = ColShape<ML>::C;
+  constexpr int NT = ColShape<ML>::NT;
   extern __shared__ double2 sm_[];
   CT* X = reinterpret_cast<CT*>(sm_);  // [t][C]
   CT* tw = X + M * C;
@@ -1462,7 +1515,7 @@ zinv_curl2_kernel(ZInvCurlArgs a) {
   const long long q0 = (long long)blockIdx.x * C;
   const int nq = (int)min((long long)C, ncol - q0);
   const long long cs = (long long)NZ1 * ncol;
-  for (int i = tid; i < M; i += kZ2Threads) cp_async_elem(tw + i, gtw + i);
+  for (int i = tid; i < M; i += NT) cp_async_elem(tw + i, gtw + i);
   cp_async_commit();
   // The fill column of this thread (the same for all its elements).
   const int cf = tid % C;
@@ -1490,34 +1543,34 @@ zinv_curl2_kernel(ZInvCurlArgs a) {
     }
     cp_async_wait_all();  // twiddles
     __syncthreads();
-    // Stage 1: inverse radix R1 (Ns = 1) on positions t = j + 8 i of column c.
+    // Stage 1: inverse radix R1 (Ns = 1) on positions t = j + R2 i of column c.
     {
       const int c = tid % C, j = tid / C;
       CT v[R1];
 #pragma unroll
-      for (int i = 0; i < R1; ++i) v[i] = X[(j + 8 * i) * C + c];
-      dft_3p<R1, 1>(v, tw, 8);
+      for (int i = 0; i < R1; ++i) v[i] = X[(j + R2 * i) * C + c];
+      dft_reg<R1, 1>(v);
       __syncthreads();  // every read done before the in-place writes
 #pragma unroll
       for (int i = 0; i < R1; ++i) X[(j * R1 + i) * C + c] = v[i];
     }
     __syncthreads();
-    // Stage 2: inverse radix 8 (Ns = R1) -> positions t = k + R1 i.
-    for (int it = tid; it < R1 * C; it += kZ2Threads) {
+    // Stage 2: inverse radix R2 (Ns = R1) -> positions t = k + R1 i.
+    for (int it = tid; it < R1 * C; it += NT) {
       const int c = it % C, k = it / C;
-      CT z[8];
+      CT z[R2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) z[i] = X[(k + R1 * i) * C + c];
+      for (int i = 0; i < R2; ++i) z[i] = X[(k + R1 * i) * C + c];
 #pragma unroll
-      for (int i = 1; i < 8; ++i) {
+      for (int i = 1; i < R2; ++i) {
         CT w = tw[i * k];
         w.y = -w.y;
         z[i] = cmul(z[i], w);
       }
-      dft8(z, 1);
+      dft_reg<R2, 1>(z);
       if (c < nq) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < R2; ++i) {
           if constexpr (SLAB) {
             // position t belongs to rank t / blk (its padded-z share)
             const int t = k + R1 * i, r = t / a.slab.blk;
@@ -1537,50 +1590,25 @@ cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,
                              cudaStream_t st) {
   const int L = a.plan.L;
   const bool slab = a.slab.buf[0] != nullptr;
-  const bool fixed = L == 48 || L == 72 || L == 96 || L == 192;
-  if (slab && (a.fp32 || a.variant != 0 || !fixed)) return cudaErrorInvalidValue;
-  if (a.variant == 0 && fixed) {
+  if (slab && (a.fp32 || a.variant != 0 || !fp32_length(L))) return cudaErrorInvalidValue;
+  if (a.variant == 0 && two_stage_length(L)) {
+    if (a.fp32 && !fp32_length(L)) return cudaErrorInvalidValue;
     const long long ncol = (long long)a.NKX * a.Ny;
+    const int C = col_columns(L);
     // one field per CTA along y
-    const dim3 grid((unsigned)((ncol + kZ2Cols - 1) / kZ2Cols), a.curl ? 6 : 3);
-    if (slab) {
-      const size_t sm = zinv_curl2_smem(L);
-      switch (L) {
-        case 48: zinv_curl2_kernel<48, double, true><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 72: zinv_curl2_kernel<72, double, true><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 96: zinv_curl2_kernel<96, double, true><<<grid, kZ2Threads, sm, st>>>(a); break;
-        default: zinv_curl2_kernel<192, double, true><<<grid, kZ2Threads, sm, st>>>(a); break;
+    const dim3 grid((unsigned)((ncol + C - 1) / C), a.curl ? 6 : 3);
+    const size_t sm = a.fp32 ? zinv_curl2_smem(L) / 2 : zinv_curl2_smem(L);
+    return with_length(L, [&](auto len) {
+      constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;
+      if constexpr (fp32_length(LL)) {
+        if (slab) zinv_curl2_kernel<LL, double, true><<<grid, NT, sm, st>>>(a);
+        else if (a.fp32 == 2) zinv_curl2_kernel<LL, fcomp><<<grid, NT, sm, st>>>(a);
+        else if (a.fp32) zinv_curl2_kernel<LL, float><<<grid, NT, sm, st>>>(a);
+        if (slab || a.fp32) return cudaGetLastError();
       }
+      zinv_curl2_kernel<LL><<<grid, NT, sm, st>>>(a);
       return cudaGetLastError();
-    }
-    if (a.fp32 == 2) {
-      const size_t sm = zinv_curl2_smem(L) / 2;
-      switch (L) {
-        case 48: zinv_curl2_kernel<48, fcomp><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 72: zinv_curl2_kernel<72, fcomp><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 96: zinv_curl2_kernel<96, fcomp><<<grid, kZ2Threads, sm, st>>>(a); break;
-        default: zinv_curl2_kernel<192, fcomp><<<grid, kZ2Threads, sm, st>>>(a); break;
-      }
-      return cudaGetLastError();
-    }
-    if (a.fp32) {
-      const size_t sm = zinv_curl2_smem(L) / 2;
-      switch (L) {
-        case 48: zinv_curl2_kernel<48, float><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 72: zinv_curl2_kernel<72, float><<<grid, kZ2Threads, sm, st>>>(a); break;
-        case 96: zinv_curl2_kernel<96, float><<<grid, kZ2Threads, sm, st>>>(a); break;
-        default: zinv_curl2_kernel<192, float><<<grid, kZ2Threads, sm, st>>>(a); break;
-      }
-      return cudaGetLastError();
-    }
-    const size_t sm = zinv_curl2_smem(L);
-    switch (L) {
-      case 48: zinv_curl2_kernel<48><<<grid, kZ2Threads, sm, st>>>(a); break;
-      case 72: zinv_curl2_kernel<72><<<grid, kZ2Threads, sm, st>>>(a); break;
-      case 96: zinv_curl2_kernel<96><<<grid, kZ2Threads, sm, st>>>(a); break;
-      default: zinv_curl2_kernel<192><<<grid, kZ2Threads, sm, st>>>(a); break;
-    }
-    return cudaGetLastError();
+    });
   }
   if (a.fp32) return cudaErrorInvalidValue;  // two-stage compile-time passes only
   dim3 grid((a.Ny + kZTile - 1) / kZTile, a.NKX);
@@ -1589,59 +1617,46 @@ cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,
   return cudaGetLastError();
 }
 
-cudaError_t set_pass_attributes(int max_smem) {
+// Raises the dynamic shared-memory limit of every pass kernel that a
+// transform of length L can launch (a context calls it for its own lengths).
+cudaError_t set_pass_attributes(int L, int max_smem) {
   cudaError_t e = cudaSuccess;
-  const void* fns[] = {DNSB_ALL_SIZES(col_pass_kernel), DNSB_ALL_SIZES(x_pass_kernel),
-                       DNSB_ALL_SIZES(x_phys_kernel), DNSB_ALL_SIZES(x_fwd_kernel),
-                       DNSB_ALL_SIZES(yinv_kernel), DNSB_ALL_SIZES(yfwd_kernel),
-                       DNSB_ALL_SIZES(zinv_curl_kernel),
-                       (const void*)zinv_curl2_kernel<48>, (const void*)zinv_curl2_kernel<72>,
-                       (const void*)zinv_curl2_kernel<96>, (const void*)zinv_curl2_kernel<192>,
-                       (const void*)zinv_curl2_kernel<48, float>,
-                       (const void*)zinv_curl2_kernel<72, float>,
-                       (const void*)zinv_curl2_kernel<96, float>,
-                       (const void*)zinv_curl2_kernel<192, float>,
-                       (const void*)zinv_curl2_kernel<48, double, true>,
-                       (const void*)zinv_curl2_kernel<72, double, true>,
-                       (const void*)zinv_curl2_kernel<96, double, true>,
-                       (const void*)zinv_curl2_kernel<192, double, true>,
-                       (const void*)x_pass2_kernel<48, double, true>,
-                       (const void*)x_pass2_kernel<72, double, true>,
-                       (const void*)x_pass2_kernel<96, double, true>,
-                       (const void*)x_pass2_kernel<192, double, true>,
-                       (const void*)x_pass2_kernel<48>, (const void*)x_pass2_kernel<72>,
-                       (const void*)x_pass2_kernel<96>, (const void*)x_pass2_kernel<192>,
-                       (const void*)x_pass2_kernel<48, float>, (const void*)x_pass2_kernel<72, float>,
-                       (const void*)x_pass2_kernel<96, float>, (const void*)x_pass2_kernel<192, float>,
-                       (const void*)col_pass2_kernel<48, -1, float>,
-                       (const void*)col_pass2_kernel<72, -1, float>,
-                       (const void*)col_pass2_kernel<96, -1, float>,
-                       (const void*)col_pass2_kernel<192, -1, float>,
-                       (const void*)col_pass2_kernel<48, 1>, (const void*)col_pass2_kernel<48, -1>,
-                       (const void*)col_pass2_kernel<72, 1>, (const void*)col_pass2_kernel<72, -1>,
-                       (const void*)col_pass2_kernel<96, 1>, (const void*)col_pass2_kernel<96, -1>,
-                       (const void*)col_pass2_kernel<192, 1>, (const void*)col_pass2_kernel<192, -1>,
-#define DNSB_OCC4_PASSES(L)                                                         \
-  (const void*)col_pass2_occ4_kernel<L, 1, true>,                                   \
-      (const void*)col_pass2_occ4_kernel<L, 1, false>,                              \
-      (const void*)col_pass2_occ4_kernel<L, -1, false>
-                       DNSB_OCC4_PASSES(48), DNSB_OCC4_PASSES(72), DNSB_OCC4_PASSES(96),
-                       DNSB_OCC4_PASSES(192),
-#undef DNSB_OCC4_PASSES
-#define DNSB_F32_PASSES(L)                                                          \
-  (const void*)yinv_kernel<L, float>, (const void*)yfwd_kernel<L, float>,           \
-      (const void*)col_pass2_kernel<L, 1, float, true>,                             \
-      (const void*)col_pass2_kernel<L, -1, float, true>,                            \
-      (const void*)col_pass2_kernel<L, 1, float, true, true>,                       \
-      (const void*)col_pass2_kernel<L, 1, double, false, true>,                     \
-      (const void*)col_pass2_kernel<L, 1, double, false, false, true>
-                       DNSB_F32_PASSES(48), DNSB_F32_PASSES(72), DNSB_F32_PASSES(96),
-                       DNSB_F32_PASSES(192)};
-#undef DNSB_F32_PASSES
-  for (const void* f : fns) {
-    cudaError_t r = allow_dynamic_smem(f, max_smem);
-    if (r != cudaSuccess) e = r;
-  }
+  auto allow = [&](std::initializer_list<const void*> fns) {
+    for (const void* f : fns) {
+      const cudaError_t r = allow_dynamic_smem(f, max_smem);
+      if (r != cudaSuccess) e = r;
+    }
+  };
+#define DNSB_STOCKHAM(N)                                                               \
+  {(const void*)col_pass_kernel<N>, (const void*)x_pass_kernel<N>,                     \
+   (const void*)x_phys_kernel<N>, (const void*)x_fwd_kernel<N>,                        \
+   (const void*)yinv_kernel<N>, (const void*)yfwd_kernel<N>, (const void*)zinv_curl_kernel<N>}
+  allow(DNSB_STOCKHAM(0));
+  if (!two_stage_length(L)) return e;
+  with_length(L, [&](auto len) {
+    constexpr int LL = decltype(len)::value;
+    allow({(const void*)col_pass2_occ4_kernel<LL, 1, true>,
+           (const void*)col_pass2_occ4_kernel<LL, 1, false>,
+           (const void*)col_pass2_occ4_kernel<LL, -1, false>,
+           (const void*)zinv_curl2_kernel<LL>});
+    if constexpr (fp32_length(LL)) {
+      allow(DNSB_STOCKHAM(LL));
+      allow({(const void*)x_pass2_kernel<LL>, (const void*)x_pass2_kernel<LL, float>,
+             (const void*)x_pass2_kernel<LL, double, true>,
+             (const void*)zinv_curl2_kernel<LL, float>,
+             (const void*)zinv_curl2_kernel<LL, double, true>,
+             (const void*)yinv_kernel<LL, float>, (const void*)yfwd_kernel<LL, float>,
+             (const void*)col_pass2_kernel<LL, 1>, (const void*)col_pass2_kernel<LL, -1>,
+             (const void*)col_pass2_kernel<LL, -1, float>,
+             (const void*)col_pass2_kernel<LL, 1, float, true>,
+             (const void*)col_pass2_kernel<LL, -1, float, true>,
+             (const void*)col_pass2_kernel<LL, 1, float, true, true>,
+             (const void*)col_pass2_kernel<LL, 1, double, false, true>,
+             (const void*)col_pass2_kernel<LL, 1, double, false, false, true>});
+    }
+    return cudaSuccess;
+  });
+#undef DNSB_STOCKHAM
   return e;
 }
 

@@ -19,6 +19,18 @@ constexpr int kX2Rows = 4;       // physical rows per CTA in the two-stage x pas
 constexpr int kX2Threads = 96;   // one item per thread in every stage
 size_t x_pass2_smem(int M, int nkx);
 
+// Padded lengths with two-stage register passes in FP64: 3 m for every m =
+// 2^a 3^b from 12 to 72 and 96, 128 (mode counts 24 to 256); the others run
+// Stockham stages.  The FP32, slab and work-list forms are compiled for
+// fp32_length alone.
+__host__ __device__ constexpr bool fp32_length(int L) {
+  return L == 48 || L == 72 || L == 96 || L == 192;
+}
+__host__ __device__ constexpr bool two_stage_length(int L) {
+  return fp32_length(L) || L == 36 || L == 54 || L == 108 || L == 144 || L == 162 ||
+         L == 216 || L == 288 || L == 384;
+}
+
 // Slab exchange (the reference's slab scheme over several GPUs): a pass
 // that feeds the other layout stores each output straight into the
 // buffer of the rank that owns it, through that rank's pointer (peer
@@ -56,7 +68,7 @@ struct ColPassArgs {
   const double* kx;
   const double* ky;
   const double* kz;
-  int occ4;  // FP64 two-stage pass held to 4 CTAs per SM (128 registers)
+  int occ4;  // FP64 two-stage pass held to 4 CTAs per SM (always beyond fp32_length)
   // Slab store (inverse, FP64 two-stage pass): position t goes to
   // slab.buf[t / blk] + f*fs + o*out_os + (t % blk)*ts + off + i, instead of
   // out + f*out_fs + o*out_os + t*out_ts + i.
@@ -209,7 +221,7 @@ cudaError_t launch_x_phys(const XPhysArgs& a, cudaStream_t st);
 cudaError_t launch_x_fwd(const XPhysArgs& a, const double* phys, double2* spec,
                          cudaStream_t st);
 size_t x_fwd_smem(int Mx);
-cudaError_t set_pass_attributes(int max_smem);
+cudaError_t set_pass_attributes(int L, int max_smem);
 cudaError_t launch_yinv(const YInvArgs& a, cudaStream_t st);
 cudaError_t launch_yfwd(const YFwdArgs& a, cudaStream_t st);
 cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,

@@ -1,0 +1,74 @@
+"""Every padded length of the two-stage passes on each axis, against the
+oracle: the RHS and the transforms, both flow families.  The other axes stay
+at 16 modes (padded 24, Stockham stages), so one length is tested at a time;
+nx/2 = n/2 columns leave the last column tile partly filled."""
+
+from math import pi
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# mode counts of the lengths beyond 48, 72, 96 and 192 (3 n / 2)
+MODES = [24, 36, 72, 96, 108, 144, 192, 256]
+
+
+def dev(a):
+    import torch
+
+    return torch.as_tensor(np.ascontiguousarray(a), device="cuda")
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("n", MODES)
+def test_periodic_lengths(n, axis):
+    from dnsjax_b200 import initial
+    from dnsjax_b200.flows.monochromatic import TriplyPeriodicFlow
+    from dnsjax_b200.parameters import Parameters
+    from oracle.config import Config
+    from oracle.fft import spec_to_phys
+    from oracle.periodic import PeriodicSetup
+
+    g = [16, 16, 16]
+    g[axis] = n
+    p = Parameters(phys=dict(system="waleffe", re=60.0),
+                   geo=dict(lx=2 * pi, lz=2 * pi, tilt_degree=30.0),
+                   res=dict(nx=g[0], ny=g[1], nz=g[2]), step=dict(dt=0.01))
+    cfg = Config(system="waleffe", nx=g[0], ny=g[1], nz=g[2], lx=2 * pi, lz=2 * pi, ly=2 * pi,
+                 re=60.0, dt=0.01, tilt_degree=30.0)
+    flow, orc = TriplyPeriodicFlow(p, ly=2 * pi), PeriodicSetup(cfg)
+    u0 = initial.periodic_field(*g, 2 * pi, 2 * pi, 2 * pi, n + axis,
+                                initial.kolmogorov_spectrum_k53, 0.1)
+    assert rel_l2(flow.get_rhs(dev(u0)).cpu(), orc.get_rhs(u0)) < 1e-12
+    phys = spec_to_phys(u0, cfg)
+    assert rel_l2(flow.spec_to_phys(dev(u0)).cpu(), phys) < 1e-13
+    assert rel_l2(flow.phys_to_spec(dev(phys)).cpu(), u0) < 1e-13
+
+
+@pytest.mark.parametrize("axis", [0, 2])
+@pytest.mark.parametrize("n", MODES)
+def test_couette_lengths(n, axis):
+    from dnsjax_b200 import initial
+    from dnsjax_b200.flows.plane_couette import PlaneCouetteFlow
+    from dnsjax_b200.parameters import Parameters
+    from oracle.config import Config
+    from oracle.couette import CouetteSetup
+    from oracle.fft import spec_to_phys_2d
+
+    g = [16, 19, 16]
+    g[axis] = n
+    p = Parameters(phys=dict(system="plane-couette", re=400.0), geo=dict(lx=2 * pi, lz=pi),
+                   res=dict(nx=g[0], ny=g[1], nz=g[2], fd_order=4), step=dict(dt=0.01))
+    cfg = Config(system="plane-couette", nx=g[0], ny=g[1], nz=g[2], lx=2 * pi, lz=pi,
+                 re=400.0, dt=0.01, fd_order=4)
+    flow = PlaneCouetteFlow(p)
+    imm = {k: v.cpu().numpy() for k, v in flow.imm.items()}
+    orc = CouetteSetup(cfg, imm=dict(imm, D1=flow.D1, D2=flow.D2))
+    u0 = initial.couette_field(*g, 2 * pi, pi, 4, n + axis, 8.0, 1e-2)
+    assert rel_l2(flow.get_rhs(dev(u0)).cpu(), orc.get_rhs(u0)) < 1e-12
+    phys = spec_to_phys_2d(u0, cfg)
+    assert rel_l2(flow.spec_to_phys(dev(u0)).cpu(), phys) < 1e-13
+    assert rel_l2(flow.phys_to_spec(dev(phys)).cpu(), u0) < 1e-13
