@@ -237,9 +237,7 @@ extern "C" int dnsb_periodic_create(const dnsb_periodic_desc* d,
     if (e1 || e2 || e3) rc = fail(DNSB_ERR_CUDA, "workspace allocation failed");
   }
   if (!rc) {
-    cudaError_t e = cudaSuccess;
-    for (int L : {p->My, p->Mz, p->Mx})
-      if (e == cudaSuccess) e = set_pass_attributes(L, smax);
+    cudaError_t e = set_pass_attributes(smax);
     if (e == cudaSuccess) e = set_solver_attributes(smax);
     if (e != cudaSuccess)
       rc = fail(DNSB_ERR_CUDA, std::string("cudaFuncSetAttribute: ") +
@@ -712,8 +710,8 @@ static dnsb_step_graph* new_step_graph(size_t n) {
 // (the two-stage passes at the compiled sizes, the y forward as a column
 // pass plus the projection), at most max_iter; otherwise none.
 static int periodic_unroll(const dnsb_periodic* p, int max_iter) {
-  if (p->graph_unroll <= 0 || !fp32_length(p->My) || !fp32_length(p->Mz) || !fp32_length(p->Mx) ||
-      3 * p->NKX != p->Mx)
+  if (p->graph_unroll <= 0 || !two_stage_length(p->My) || !two_stage_length(p->Mz) ||
+      !two_stage_length(p->Mx) || 3 * p->NKX != p->Mx)
     return 0;
   for (int k = 0; k < 5; ++k)
     if (p->var[k] != 0) return 0;
@@ -1447,9 +1445,7 @@ extern "C" int dnsb_couette_create(const dnsb_couette_desc* d,
       rc = fail(DNSB_ERR_CUDA, "cudaMemset failed");
   }
   if (!rc) {
-    cudaError_t e = cudaSuccess;
-    for (int L : {p->Mz, p->Mx})
-      if (e == cudaSuccess) e = set_pass_attributes(L, smax);
+    cudaError_t e = set_pass_attributes(smax);
     if (e == cudaSuccess) e = set_solver_attributes(smax);
     if (e == cudaSuccess) e = set_imm_v2_attributes(smax);
     if (e == cudaSuccess) e = set_imm_batch_attributes(smax);
@@ -1814,7 +1810,9 @@ extern "C" int dnsb_couette_phys_to_spec(dnsb_couette* p, const double* phys,
 // two-stage passes at the compiled sizes and the batched IMM), at most
 // max_iter; otherwise none.
 static int couette_unroll(const dnsb_couette* p, int max_iter) {
-  if (p->graph_unroll <= 0 || !couette_fp32_sizes(p) || !p->batch_ready) return 0;
+  if (p->graph_unroll <= 0 || !two_stage_length(p->Mz) || !two_stage_length(p->Mx) ||
+      3 * p->NKX != p->Mx || !p->batch_ready)
+    return 0;
   for (int k = 0; k < 4; ++k)
     if (p->var[k] != 0) return 0;
   return std::min(p->graph_unroll, std::max(max_iter, 0));

@@ -201,8 +201,27 @@ __device__ __forceinline__ void dft2(V* v) {
   v[1] = csub(a, b);
 }
 
+// zero: bit i set where v[i] is known to be zero (one at most)
 template <typename V>
-__device__ __forceinline__ void dft3(V* v, int sign) {
+__device__ __forceinline__ void dft3(V* v, int sign, unsigned zero = 0) {
+  if (zero == 1u || zero == 2u || zero == 4u) {
+    const double s3 = 0.86602540378443864676;  // sin(2 pi / 3)
+    if (zero == 1u) {
+      const V t1 = cadd(v[1], v[2]), t2 = cconst(t1, -0.5);
+      const V t3 = cconst(cisign(csub(v[1], v[2]), sign), s3);
+      v[0] = t1;
+      v[1] = cadd(t2, t3);
+      v[2] = csub(t2, t3);
+    } else {
+      const V x = zero == 2u ? v[2] : v[1];
+      const V t2 = csub(v[0], cconst(x, 0.5));
+      const V t3 = cconst(cisign(x, zero == 2u ? -sign : sign), s3);
+      v[0] = cadd(v[0], x);
+      v[1] = cadd(t2, t3);
+      v[2] = csub(t2, t3);
+    }
+    return;
+  }
   const V t1 = cadd(v[1], v[2]);
   const V t2 = csub(v[0], cconst(t1, 0.5));
   // sin(2 pi / 3)
@@ -461,20 +480,27 @@ __host__ __device__ constexpr double sin_turn(int k) {
 // N = A B with A, B coprime: the prime-factor (Good-Thomas) form, no twiddles:
 // input n = (B n1 + A n2) mod N, output k = (B (B^-1 mod A) k1 + A (A^-1 mod B)
 // k2) mod N.  9, 16 and 27 points: Cooley-Tukey with constant twiddles.
+// zero: bit i set where v[i] is known to be zero; folded away once unrolled.
+// The 3-point DFTs that see such an input (the padded middle third of an
+// inverse transform) skip its operations.
 template <int N, int SIGN, typename V>
-__device__ __forceinline__ void dft_n(V* v);
+__device__ __forceinline__ void dft_n(V* v, unsigned zero = 0);
 
 template <int A, int B, int SIGN, typename V>
-__device__ __forceinline__ void dft_pfa(V* v) {
+__device__ __forceinline__ void dft_pfa(V* v, unsigned zero) {
   constexpr int N = A * B;
   constexpr int KA = B * inv_mod(B % A, A), KB = A * inv_mod(A % B, B);
   V a[B][A];
 #pragma unroll
-  for (int n2 = 0; n2 < B; ++n2)
+  for (int n2 = 0; n2 < B; ++n2) {
+    unsigned z = 0;
 #pragma unroll
-    for (int n1 = 0; n1 < A; ++n1) a[n2][n1] = v[(B * n1 + A * n2) % N];
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) dft_n<A, SIGN>(a[n2]);
+    for (int n1 = 0; n1 < A; ++n1) {
+      a[n2][n1] = v[(B * n1 + A * n2) % N];
+      z |= ((zero >> ((B * n1 + A * n2) % N)) & 1u) << n1;
+    }
+    dft_n<A, SIGN>(a[n2], z);
+  }
 #pragma unroll
   for (int k1 = 0; k1 < A; ++k1) {
     V b[B];
@@ -487,15 +513,19 @@ __device__ __forceinline__ void dft_pfa(V* v) {
 }
 
 template <int A, int B, int SIGN, typename V>
-__device__ __forceinline__ void dft_ct(V* v) {
+__device__ __forceinline__ void dft_ct(V* v, unsigned zero) {
   constexpr int N = A * B;
   V a[B][A];
 #pragma unroll
-  for (int b = 0; b < B; ++b)
+  for (int b = 0; b < B; ++b) {
+    unsigned z = 0;
 #pragma unroll
-    for (int n = 0; n < A; ++n) a[b][n] = v[B * n + b];
-#pragma unroll
-  for (int b = 0; b < B; ++b) dft_n<A, SIGN>(a[b]);
+    for (int n = 0; n < A; ++n) {
+      a[b][n] = v[B * n + b];
+      z |= ((zero >> (B * n + b)) & 1u) << n;
+    }
+    dft_n<A, SIGN>(a[b], z);
+  }
 #pragma unroll
   for (int b = 1; b < B; ++b)
 #pragma unroll
@@ -515,35 +545,43 @@ __device__ __forceinline__ void dft_ct(V* v) {
 }
 
 template <int N, int SIGN, typename V>
-__device__ __forceinline__ void dft_n(V* v) {
+__device__ __forceinline__ void dft_n(V* v, unsigned zero) {
   if constexpr (N == 2) dft2(v);
-  else if constexpr (N == 3) dft3(v, SIGN);
+  else if constexpr (N == 3) dft3(v, SIGN, zero);
   else if constexpr (N == 4) dft4(v, SIGN);
   else if constexpr (N == 8) dft8(v, SIGN);
-  else if constexpr (N == 9) dft_ct<3, 3, SIGN>(v);
-  else if constexpr (N == 16) dft_ct<4, 4, SIGN>(v);
-  else if constexpr (N == 27) dft_ct<9, 3, SIGN>(v);
-  else if constexpr (N == 18) dft_pfa<9, 2, SIGN>(v);
+  else if constexpr (N == 9) dft_ct<3, 3, SIGN>(v, zero);
+  else if constexpr (N == 16) dft_ct<4, 4, SIGN>(v, zero);
+  else if constexpr (N == 27) dft_ct<9, 3, SIGN>(v, zero);
+  else if constexpr (N == 18) dft_pfa<9, 2, SIGN>(v, zero);
   else {
     static_assert(N == 6 || N == 12 || N == 24, "no register DFT of this size");
-    dft_pfa<N / 3, 3, SIGN>(v);
+    // 3 points first where they see the zeros, else last (a caller that drops
+    // the middle third of the outputs drops one of each three there)
+    if (zero) dft_pfa<3, N / 3, SIGN>(v, zero);
+    else dft_pfa<N / 3, 3, SIGN>(v, 0);
   }
 }
 
 // The same on the pass kernels' element types: cf2 runs it on compensated
 // values.
 template <int N, int SIGN, typename C>
-__device__ __forceinline__ void dft_reg(C* v) {
+__device__ __forceinline__ void dft_reg(C* v, unsigned zero = 0) {
   if constexpr (std::is_same<C, cf2>::value) {
     cff w[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) w[i] = cff_of(v[i]);
-    dft_n<N, SIGN>(w);
+    dft_n<N, SIGN>(w, zero);
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = cff_fold(w[i]);
   } else {
-    dft_n<N, SIGN>(v);
+    dft_n<N, SIGN>(v, zero);
   }
+}
+
+// The middle third of N inputs: what 3/2 zero-padding leaves zero.
+__host__ __device__ constexpr unsigned middle_third(int N) {
+  return N % 3 ? 0u : ((1u << (N / 3)) - 1u) << (N / 3);
 }
 
 // Stored index -> padded FFT position for a Nyquist-free complex axis of

@@ -156,19 +156,6 @@ DNSB_COL_SHAPE(288, 24, 12, 8, 4)
 DNSB_COL_SHAPE(384, 24, 16, 8, 4)
 #undef DNSB_COL_SHAPE
 
-// f(std::integral_constant<int, L>) for a two-stage length L.
-template <typename F>
-static cudaError_t with_length(int L, F&& f) {
-  switch (L) {
-#define DNSB_LEN(LL) \
-  case LL: return f(std::integral_constant<int, LL>{});
-    DNSB_LEN(36) DNSB_LEN(48) DNSB_LEN(54) DNSB_LEN(72) DNSB_LEN(96) DNSB_LEN(108)
-    DNSB_LEN(144) DNSB_LEN(162) DNSB_LEN(192) DNSB_LEN(216) DNSB_LEN(288) DNSB_LEN(384)
-#undef DNSB_LEN
-    default: return cudaErrorInvalidValue;
-  }
-}
-
 size_t col_pass2_smem(int M) {
   return sizeof(double2) * (size_t)(M * col_columns(M) + M);
 }
@@ -514,321 +501,16 @@ x_pass_kernel(XPassArgs a) {
   }
 }
 
-template <int ML, typename T = double, bool SLAB = false>
-__global__ void __launch_bounds__(kX2Threads, std::is_same<T, float>::value ? 8 : 5)
-x_pass2_kernel(XPassArgs a);
-
 cudaError_t launch_x_pass(const XPassArgs& a, cudaStream_t st) {
   dim3 grid((a.nrows + kXRows - 1) / kXRows);
   // The compile-time variants assume nx/2 = M/3 (3/2 oversampling).
   const int L = (a.nkx * 3 == a.plan.L) ? a.plan.L : -1;
   const bool slab = a.slab.buf[0] != nullptr;
   if (slab && (a.fp32 || a.variant != 0 || L < 0)) return cudaErrorInvalidValue;
-  if (a.variant == 0 && (L == 48 || L == 72 || L == 96 || L == 192)) {
-    dim3 g2((a.nrows + kX2Rows - 1) / kX2Rows);
-    if (slab) {
-      const size_t sm2 = x_pass2_smem(L, a.nkx);
-      switch (L) {
-        case 48: x_pass2_kernel<48, double, true><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 72: x_pass2_kernel<72, double, true><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 96: x_pass2_kernel<96, double, true><<<g2, kX2Threads, sm2, st>>>(a); break;
-        default: x_pass2_kernel<192, double, true><<<g2, kX2Threads, sm2, st>>>(a); break;
-      }
-      return cudaGetLastError();
-    }
-    if (a.fp32 == 2) {
-      const size_t sm2 = x_pass2_smem(L, a.nkx) / 2;
-      switch (L) {
-        case 48: x_pass2_kernel<48, fcomp><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 72: x_pass2_kernel<72, fcomp><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 96: x_pass2_kernel<96, fcomp><<<g2, kX2Threads, sm2, st>>>(a); break;
-        default: x_pass2_kernel<192, fcomp><<<g2, kX2Threads, sm2, st>>>(a); break;
-      }
-      return cudaGetLastError();
-    }
-    if (a.fp32) {
-      const size_t sm2 = x_pass2_smem(L, a.nkx) / 2;
-      switch (L) {
-        case 48: x_pass2_kernel<48, float><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 72: x_pass2_kernel<72, float><<<g2, kX2Threads, sm2, st>>>(a); break;
-        case 96: x_pass2_kernel<96, float><<<g2, kX2Threads, sm2, st>>>(a); break;
-        default: x_pass2_kernel<192, float><<<g2, kX2Threads, sm2, st>>>(a); break;
-      }
-      return cudaGetLastError();
-    }
-    const size_t sm2 = x_pass2_smem(L, a.nkx);
-    switch (L) {
-      case 48: x_pass2_kernel<48><<<g2, kX2Threads, sm2, st>>>(a); break;
-      case 72: x_pass2_kernel<72><<<g2, kX2Threads, sm2, st>>>(a); break;
-      case 96: x_pass2_kernel<96><<<g2, kX2Threads, sm2, st>>>(a); break;
-      default: x_pass2_kernel<192><<<g2, kX2Threads, sm2, st>>>(a); break;
-    }
-    return cudaGetLastError();
-  }
+  if (a.variant == 0 && two_stage_length(L)) return launch_x_pass2(a, st);
   if (a.fp32) return cudaErrorInvalidValue;  // two-stage compile-time passes only
   DNSB_DISPATCH_V(a.variant, L, x_pass_kernel, grid, x_pass_smem(a.plan.L), st, a);
   return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// x pass, two register stages (M = 8 R1, R1 = M/8 = 3P): inverse radix-R1
-// stage straight from the staged half spectra; inverse radix-8 stage, the
-// rotational product and the first forward radix-8 stage fused in one
-// thread (the 8 positions k + R1 i a radix-8 output holds are the inputs of
-// the forward radix-8 stage); forward radix-R1 stage; unpack and store.
-// ---------------------------------------------------------------------------
-// One work region holds, in turn, the staged half spectra, the inverse
-// stage-A output, the forward stage-1 output and the stage-C output: each
-// stage reads its input into registers, waits for every thread, then writes
-// its output over it.
-size_t x_pass2_smem(int M, int nkx) {
-  // the stage-B output: M / 8 blocks of 8 * CF + 16 slots (CF = 2 rows x 4)
-  const size_t S = (size_t)6 * nkx * kX2Rows, Y = (size_t)(M / 8) * (8 * 2 * kX2Rows + 16);
-  const size_t X = (size_t)M * 3 * kX2Rows + 4 * 8;  // + the stage-A skew
-  size_t W = S > Y ? S : Y;
-  W = W > X ? W : X;
-  return sizeof(double2) * (W + M);
-}
-
-// T: the compute type and the element type of the pass buffer (double, or
-// float for the FP32 form of the Couette RHS).
-template <int ML, typename T, bool SLAB = false>
-__device__ __forceinline__ void x_pass2_body(const XPassArgs& a, int bx) {
-  using CT = typename pass_types<T>::C;
-  using RT = typename pass_types<T>::R;
-  constexpr int M = ML, R1 = M / 8, R = kX2Rows, NKX = ML / 3;
-  constexpr int CI = 3 * R, CF = 2 * R;
-  // Shared-memory layouts keep the stages' accesses free of bank conflicts
-  // for 16-byte (FP64, 8 lanes per 128-byte wavefront) and 8-byte (FP32, 16
-  // lanes) elements alike:
-  //  * the stage-A output carries a skew of XS slots per block of R1
-  //    positions;
-  //  * the stage-B output, position t = 8 k + i, lives in blocks of YB
-  //    slots (a multiple of 16, so the banks depend on the skew alone), with
-  //    a skew of (k & 1) + 8 ((k >> 1) & 1) slots per block;
-  //  * the stage-C output's row t starts at slot 9 t, which the final
-  //    unpack reads without conflicts, rows or modes fastest (for 8-byte
-  //    elements unpacked rows fastest, rows of CF slots measured faster).
-  constexpr int XS = 4;
-  constexpr int YB = 8 * CF + 16;
-  static_assert(R == 4, "the stage-A lane map assumes 4 rows");
-  static_assert(YB % 16 == 0 && YB >= 8 * CF + 10, "stage-B blocks hold their skew");
-  constexpr int SZ_S = 6 * NKX * R, SZ_Y = R1 * YB, SZ_X = M * CI + XS * 8;
-  static_assert(9 * M <= SZ_X, "the stage-C rows fit the work region");
-  // 9 slots per row, except 8-byte elements unpacked rows fastest (CF:
-  // 1% faster there); the mapping is fixed per launch
-  const int xstride = (sizeof(CT) == 16 || !a.rows_fast) ? 9 : CF;
-  auto xrow = [xstride](int t) { return xstride * t; };
-  constexpr int SZ_SY = SZ_S > SZ_Y ? SZ_S : SZ_Y;
-  constexpr int SZ_W = SZ_SY > SZ_X ? SZ_SY : SZ_X;
-  // every stage has at most one item per thread, so a thread can hold its
-  // item's inputs in registers across the barrier before the in-place write
-  static_assert(8 * CI <= kX2Threads && R1 * R <= kX2Threads && 8 * CF <= kX2Threads,
-                "one item per thread in every stage");
-  extern __shared__ double2 sm_[];
-  CT* sm = reinterpret_cast<CT*>(sm_);
-  CT* S = sm;                 // staged half spectra, S[(f*NKX + k)*R + r]
-  CT* X = sm;                 // inverse stage-A output [t][CI] (over S); later [t][CF]
-  CT* Y = sm;                 // forward stage-1 output [t][CF] (over X)
-  CT* tw = sm + SZ_W;
-  const CT* gin = reinterpret_cast<const CT*>(a.in);
-  const CT* gtw = reinterpret_cast<const CT*>(a.tw);
-  CT* gout = reinterpret_cast<CT*>(a.out);
-  const int tid = threadIdx.x;
-  const int r0 = bx * R;
-  const int nr = min(R, a.nrows - r0);
-  __shared__ long long s_off[kX2Rows];
-  __shared__ long long s_doff[kX2Rows];  // SLAB: the row in the destination layout
-  __shared__ int s_y[kX2Rows];
-  if (tid < R) {
-    const int row = r0 + tid;
-    const int outer = row / a.inner_n, inner = row % a.inner_n;
-    s_off[tid] = (long long)outer * a.so + (long long)inner * a.si;
-    s_y[tid] = a.y_outer ? outer : inner;
-    if (SLAB)
-      s_doff[tid] = (long long)(outer + a.slab.oo) * a.slab.so +
-                    (long long)(inner + a.slab.io) * a.slab.si;
-  }
-  for (int i = tid; i < M; i += kX2Threads) cp_async_elem(tw + i, gtw + i);
-  __syncthreads();
-  // The input's last use (evict_first); the output is the next pass's input
-  // (evict_last).
-  const unsigned long long drop = l2_drop(), keep = l2_keep();
-  for (int idx = tid; idx < 6 * NKX * R; idx += kX2Threads) {
-    int r, k, f;
-    if (a.rows_fast) {
-      r = idx % R;
-      k = (idx / R) % NKX;
-      f = idx / (R * NKX);
-    } else {
-      k = idx % NKX;
-      r = (idx / NKX) % R;
-      f = idx / (R * NKX);
-    }
-    CT* dst = S + (f * NKX + k) * R + r;
-    if (r < nr) cp_async_elem_l2(dst, gin + f * a.in_fs + s_off[r] + k * a.ks, drop);
-    else *dst = cmake<CT>(0, 0);
-  }
-  cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
-  // Stage A: inverse radix R1 (Ns = 1) on Z = A + iB, built on the fly.
-  {
-    // lanes of a half warp: 4 rows x 4 values of j, one field pair, where
-    // the stage-A output's stride per j (R1 CI + XS slots) spreads the four
-    // j over the banks; else (M = 72) 4 rows x 2 values of j x 2 pairs
-    constexpr bool J4 = (R1 * CI + XS) % 16 != 0;
-    const int it = tid;
-    const bool act = it < 8 * CI;
-    const int r = it & 3, rest = J4 ? it >> 4 : it >> 3;
-    const int pr = rest % 3;
-    const int j = J4 ? ((it >> 2) & 3) + 4 * (rest / 3) : ((it >> 2) & 1) + 2 * (rest / 3);
-    const int col = 3 * r + pr;
-    CT v[R1];
-    if (act) {
-      const CT* A = S + (2 * pr) * NKX * R + r;
-      const CT* B = S + (2 * pr + 1) * NKX * R + r;
-#pragma unroll
-      for (int i = 0; i < R1; ++i) {
-        const int t = j + 8 * i;
-        CT z = cmake<CT>(0, 0);
-        if (t == 0) {
-          z = cmake<CT>(A[0].x, B[0].x);
-        } else if (t < NKX) {
-          const CT av = A[t * R], bv = B[t * R];
-          z = cmake<CT>(av.x - bv.y, av.y + bv.x);
-        } else if (M - t < NKX) {
-          const CT av = A[(M - t) * R], bv = B[(M - t) * R];
-          z = cmake<CT>(av.x + bv.y, -av.y + bv.x);
-        }
-        v[i] = z;
-      }
-    }
-    __syncthreads();  // S read by every thread before X is written over it
-    if (act) {
-      dft_reg<R1, 1>(v);
-#pragma unroll
-      for (int i = 0; i < R1; ++i) X[(j * R1 + i) * CI + col + XS * j] = v[i];
-    }
-  }
-  __syncthreads();
-  // Stage B: inverse radix 8 (Ns = R1) -> physical values at t = k + R1 i;
-  // rotational product there; forward radix-8 stage (Ns = 1) on the same t.
-  {
-    const int it = tid;
-    const bool act = it < R1 * R;
-    const int r = it % R, k = it / R;
-    CT F0[8], F1[8];
-    if (act) {
-      CT z[3][8];
-#pragma unroll
-      for (int pr = 0; pr < 3; ++pr) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) z[pr][i] = X[(k + R1 * i) * CI + 3 * r + pr + XS * i];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) {
-          CT w = tw[i * k];
-          w.y = -w.y;
-          z[pr][i] = cmul(z[pr][i], w);
-        }
-        dft_reg<8, 1>(z[pr]);
-      }
-      const bool live = r < nr;
-      const int y = s_y[r];
-      const int ny = a.ny_grid;
-      const RT U0 = live ? (RT)a.U[y] : RT(0), U1 = live ? (RT)a.U[ny + y] : RT(0),
-              U2 = live ? (RT)a.U[2 * ny + y] : RT(0);
-      const RT C0 = live ? (RT)a.cU[y] : RT(0), C1 = live ? (RT)a.cU[ny + y] : RT(0),
-              C2 = live ? (RT)a.cU[2 * ny + y] : RT(0);
-      const RT N0 = live ? (RT)a.nU[y] : RT(0), N1 = live ? (RT)a.nU[ny + y] : RT(0),
-              N2 = live ? (RT)a.nU[2 * ny + y] : RT(0);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const RT u0 = z[0][i].x, u1 = z[0][i].y, u2 = z[1][i].x;
-        const RT w0 = z[1][i].y, w1 = z[2][i].x, w2 = z[2][i].y;
-        const RT n0 = u1 * w2 - u2 * w1;
-        const RT n1 = u2 * w0 - u0 * w2;
-        const RT n2 = u0 * w1 - u1 * w0;
-        const RT b0 = (u1 * C2 - u2 * C1) + (U1 * w2 - U2 * w1) + N0;
-        const RT b1 = (u2 * C0 - u0 * C2) + (U2 * w0 - U0 * w2) + N1;
-        const RT b2 = (u0 * C1 - u1 * C0) + (U0 * w1 - U1 * w0) + N2;
-        F0[i] = live ? cmake<CT>(n0 + b0, n1 + b1) : cmake<CT>(0, 0);
-        F1[i] = live ? cmake<CT>(n2 + b2, 0) : cmake<CT>(0, 0);
-      }
-      dft_reg<8, -1>(F0);
-      dft_reg<8, -1>(F1);
-    }
-    __syncthreads();  // X read by every thread before Y is written over it
-    if (act) {
-      CT* yk = Y + k * YB + (k & 1) + 8 * ((k >> 1) & 1);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        yk[i * CF + 2 * r] = F0[i];
-        yk[i * CF + 2 * r + 1] = F1[i];
-      }
-    }
-  }
-  __syncthreads();
-  // Stage C: forward radix R1 (Ns = 8), natural order into X[t][CF].
-  {
-    const int it = tid;
-    const bool act = it < 8 * CF;
-    const int col = it % CF, j = it / CF;
-    CT v[R1];
-    if (act) {
-      // position t = j + 8 i is entry j of stage-B block i
-#pragma unroll
-      for (int i = 0; i < R1; ++i)
-        v[i] = Y[i * YB + (i & 1) + 8 * ((i >> 1) & 1) + j * CF + col];
-    }
-    __syncthreads();  // Y read by every thread before X is written over it
-    if (act) {
-#pragma unroll
-      for (int i = 1; i < R1; ++i) v[i] = cmul(v[i], tw[i * j]);
-      dft_reg<R1, -1>(v);
-#pragma unroll
-      for (int i = 0; i < R1; ++i) X[xrow(j + 8 * i) + col] = v[i];
-    }
-  }
-  __syncthreads();
-  // Unpack the real-field spectra, truncate to NKX, scale 1/M, store.
-  const RT h = (RT)0.5 / M;
-  for (int idx = tid; idx < 3 * NKX * R; idx += kX2Threads) {
-    int r, k, f;
-    if (a.rows_fast) {
-      r = idx % R;
-      k = (idx / R) % NKX;
-      f = idx / (R * NKX);
-    } else {
-      k = idx % NKX;
-      r = (idx / NKX) % R;
-      f = idx / (R * NKX);
-    }
-    if (r >= nr) continue;
-    const int col = 2 * r + (f == 2 ? 1 : 0);
-    const CT Z = X[xrow(k) + col];
-    const CT Zm = X[xrow((M - k) % M) + col];
-    CT v;
-    if (f == 1) {
-      v = cmake<CT>((Z.y + Zm.y) * h, (Zm.x - Z.x) * h);
-    } else {
-      v = cmake<CT>((Z.x + Zm.x) * h, (Z.y - Zm.y) * h);
-    }
-    if constexpr (SLAB) {
-      // mode k belongs to rank k / blk (its kx share)
-      const int q = k / a.slab.blk;
-      a.slab.buf[q][f * a.slab.fs + s_doff[r] + (k - q * a.slab.blk) * a.slab.ks] = to_d(v);
-    } else {
-      st_l2(gout + f * a.out_fs + s_off[r] + k * a.ks, v, keep);
-    }
-  }
-}
-
-template <int ML, typename T, bool SLAB>
-__global__ void __launch_bounds__(kX2Threads, std::is_same<T, float>::value ? 8 : 5)
-x_pass2_kernel(XPassArgs a) {
-  if (a.skip && *a.skip) return;
-  x_pass2_body<ML, T, SLAB>(a, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -839,16 +521,6 @@ x_pass2_kernel(XPassArgs a) {
 // runs the member's body on its block, so each member computes exactly what
 // its own launch computes.  Members whose `active` flag is 0 are skipped.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int vb) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (base[mid] <= vb) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 // the fp32_length lengths all run 128 threads on 16 columns
 constexpr int kEnsColThreads = ColShape<192>::NT;
 static_assert(ColShape<48>::NT == kEnsColThreads && ColShape<72>::NT == kEnsColThreads &&
@@ -880,29 +552,6 @@ ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict
   }
 }
 
-__global__ void __launch_bounds__(kX2Threads)
-ens_x_pass2_kernel(const EnsXItem* __restrict__ items, const int* __restrict__ base, int n,
-                   int total, const int* __restrict__ active) {
-  __shared__ int s_k;
-  for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
-    if (threadIdx.x == 0) s_k = ens_find(base, n, vb);
-    __syncthreads();
-    const int k = s_k;
-    const int m = items[k].member;
-    if (!active || active[m]) {
-      const XPassArgs a = items[k].a;
-      const int bx = vb - base[k];
-      switch (a.plan.L) {
-        case 48: x_pass2_body<48, double>(a, bx); break;
-        case 72: x_pass2_body<72, double>(a, bx); break;
-        case 96: x_pass2_body<96, double>(a, bx); break;
-        default: x_pass2_body<192, double>(a, bx); break;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 bool ens_pass_supported(int L) { return fp32_length(L); }
 
 int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy) {
@@ -912,10 +561,7 @@ int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy) 
   return *gx * nO * nfields;
 }
 
-int ens_x_blocks(const XPassArgs& a) { return (a.nrows + kX2Rows - 1) / kX2Rows; }
-
 size_t ens_col_smem(int maxL) { return col_pass2_smem(maxL); }
-size_t ens_x_smem(int maxL, int maxNKX) { return x_pass2_smem(maxL, maxNKX); }
 
 // kind 0: inverse with the curl, 1: inverse, 2: forward (col_pass2); 3: x pass.
 static const void* ens_kernel(int kind) {
@@ -923,7 +569,7 @@ static const void* ens_kernel(int kind) {
     case 0: return (const void*)ens_col_pass2_kernel<1, true>;
     case 1: return (const void*)ens_col_pass2_kernel<1, false>;
     case 2: return (const void*)ens_col_pass2_kernel<-1, false>;
-    default: return (const void*)ens_x_pass2_kernel;
+    default: return ens_x_kernel();
   }
 }
 
@@ -933,7 +579,7 @@ int ens_pass_grid(int kind, size_t smem, int total, int max_smem) {
   const void* f = ens_kernel(kind);
   if (allow_dynamic_smem(f, max_smem) != cudaSuccess) return 0;
   int per_sm = 0, dev = 0, nsm = 0;
-  const int threads = kind == 3 ? kX2Threads : kEnsColThreads;
+  const int threads = kind == 3 ? kEnsXThreads : kEnsColThreads;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess)
     return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -959,8 +605,8 @@ cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n,
           static_cast<const EnsColItem*>(items), base, n, total, active);
       break;
     default:
-      ens_x_pass2_kernel<<<grid, kX2Threads, smem, st>>>(static_cast<const EnsXItem*>(items),
-                                                          base, n, total, active);
+      return launch_ens_x(static_cast<const EnsXItem*>(items), base, n, total, active, grid,
+                          smem, st);
   }
   return cudaGetLastError();
 }
@@ -1617,9 +1263,9 @@ cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,
   return cudaGetLastError();
 }
 
-// Raises the dynamic shared-memory limit of every pass kernel that a
-// transform of length L can launch (a context calls it for its own lengths).
-cudaError_t set_pass_attributes(int L, int max_smem) {
+// Raises the dynamic shared-memory limit of every pass kernel that needs more
+// than the default 48 KB.
+cudaError_t set_pass_attributes(int max_smem) {
   cudaError_t e = cudaSuccess;
   auto allow = [&](std::initializer_list<const void*> fns) {
     for (const void* f : fns) {
@@ -1632,32 +1278,27 @@ cudaError_t set_pass_attributes(int L, int max_smem) {
    (const void*)x_phys_kernel<N>, (const void*)x_fwd_kernel<N>,                        \
    (const void*)yinv_kernel<N>, (const void*)yfwd_kernel<N>, (const void*)zinv_curl_kernel<N>}
   allow(DNSB_STOCKHAM(0));
-  if (!two_stage_length(L)) return e;
-  with_length(L, [&](auto len) {
+  for_each_length([&](auto len) {
     constexpr int LL = decltype(len)::value;
+    if constexpr (fp32_length(LL)) {
+      allow(DNSB_STOCKHAM(LL));
+      if constexpr (LL > 72)
+        allow({(const void*)yinv_kernel<LL, float>, (const void*)yfwd_kernel<LL, float>});
+    }
+    if (col_pass2_smem(LL) <= kDefaultSmem) return;
     allow({(const void*)col_pass2_occ4_kernel<LL, 1, true>,
            (const void*)col_pass2_occ4_kernel<LL, 1, false>,
            (const void*)col_pass2_occ4_kernel<LL, -1, false>,
            (const void*)zinv_curl2_kernel<LL>});
-    if constexpr (fp32_length(LL)) {
-      allow(DNSB_STOCKHAM(LL));
-      allow({(const void*)x_pass2_kernel<LL>, (const void*)x_pass2_kernel<LL, float>,
-             (const void*)x_pass2_kernel<LL, double, true>,
-             (const void*)zinv_curl2_kernel<LL, float>,
-             (const void*)zinv_curl2_kernel<LL, double, true>,
-             (const void*)yinv_kernel<LL, float>, (const void*)yfwd_kernel<LL, float>,
+    if constexpr (fp32_length(LL))
+      allow({(const void*)zinv_curl2_kernel<LL, double, true>,
              (const void*)col_pass2_kernel<LL, 1>, (const void*)col_pass2_kernel<LL, -1>,
-             (const void*)col_pass2_kernel<LL, -1, float>,
-             (const void*)col_pass2_kernel<LL, 1, float, true>,
-             (const void*)col_pass2_kernel<LL, -1, float, true>,
-             (const void*)col_pass2_kernel<LL, 1, float, true, true>,
              (const void*)col_pass2_kernel<LL, 1, double, false, true>,
              (const void*)col_pass2_kernel<LL, 1, double, false, false, true>});
-    }
-    return cudaSuccess;
   });
 #undef DNSB_STOCKHAM
-  return e;
+  const cudaError_t x = set_x_pass_attributes(max_smem);
+  return x != cudaSuccess ? x : e;
 }
 
 }  // namespace dnsb

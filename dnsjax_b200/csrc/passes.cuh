@@ -8,6 +8,8 @@
 // data they need.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace dnsb {
@@ -15,9 +17,6 @@ namespace dnsb {
 constexpr int kTile = 8;     // columns per CTA in the column passes
 constexpr int kXRows = 4;    // physical rows per CTA in the x pass
 constexpr int kPassThreads = 256;
-constexpr int kX2Rows = 4;       // physical rows per CTA in the two-stage x pass
-constexpr int kX2Threads = 96;   // one item per thread in every stage
-size_t x_pass2_smem(int M, int nkx);
 
 // Padded lengths with two-stage register passes in FP64: 3 m for every m =
 // 2^a 3^b from 12 to 72 and 96, 128 (mode counts 24 to 256); the others run
@@ -30,6 +29,29 @@ __host__ __device__ constexpr bool two_stage_length(int L) {
   return fp32_length(L) || L == 36 || L == 54 || L == 108 || L == 144 || L == 162 ||
          L == 216 || L == 288 || L == 384;
 }
+
+// f(std::integral_constant<int, L>) for a two-stage length L, or for each.
+#define DNSB_LENGTHS(X) \
+  X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(162) X(192) X(216) X(288) X(384)
+template <typename F>
+inline cudaError_t with_length(int L, F&& f) {
+  switch (L) {
+#define DNSB_LEN(LL) \
+  case LL: return f(std::integral_constant<int, LL>{});
+    DNSB_LENGTHS(DNSB_LEN)
+#undef DNSB_LEN
+    default: return cudaErrorInvalidValue;
+  }
+}
+template <typename F>
+inline void for_each_length(F&& f) {
+#define DNSB_LEN(LL) f(std::integral_constant<int, LL>{});
+  DNSB_LENGTHS(DNSB_LEN)
+#undef DNSB_LEN
+}
+// Shared memory a kernel may use without raising its limit (less a margin for
+// its static arrays).
+constexpr size_t kDefaultSmem = 47 * 1024;
 
 // Slab exchange (the reference's slab scheme over several GPUs): a pass
 // that feeds the other layout stores each output straight into the
@@ -193,6 +215,10 @@ size_t zinv_curl2_smem(int M);
 cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
                             cudaStream_t st);
 cudaError_t launch_x_pass(const XPassArgs& a, cudaStream_t st);
+// The register-stage x pass (csrc/x_pass.cu): two_stage_length(plan.L) with
+// nkx = plan.L / 3.
+cudaError_t launch_x_pass2(const XPassArgs& a, cudaStream_t st);
+cudaError_t set_x_pass_attributes(int max_smem);
 
 // Work lists of the ensemble form (one launch per pass for every member;
 // FP64 two-stage passes, padded lengths 48, 72, 96, 192).
@@ -208,6 +234,20 @@ struct EnsXItem {
 bool ens_pass_supported(int L);
 int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy);
 int ens_x_blocks(const XPassArgs& a);
+constexpr int kEnsXThreads = 96;
+const void* ens_x_kernel();
+cudaError_t launch_ens_x(const EnsXItem* items, const int* base, int n, int total,
+                         const int* active, int grid, size_t smem, cudaStream_t st);
+// Item of virtual block vb: the last k with base[k] <= vb.
+__device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int vb) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (base[mid] <= vb) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
 size_t ens_col_smem(int maxL);
 size_t ens_x_smem(int maxL, int maxNKX);
 // kind 0: inverse pass with the spectral curl, 1: inverse, 2: forward
@@ -221,7 +261,7 @@ cudaError_t launch_x_phys(const XPhysArgs& a, cudaStream_t st);
 cudaError_t launch_x_fwd(const XPhysArgs& a, const double* phys, double2* spec,
                          cudaStream_t st);
 size_t x_fwd_smem(int Mx);
-cudaError_t set_pass_attributes(int L, int max_smem);
+cudaError_t set_pass_attributes(int max_smem);
 cudaError_t launch_yinv(const YInvArgs& a, cudaStream_t st);
 cudaError_t launch_yfwd(const YFwdArgs& a, cudaStream_t st);
 cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,

@@ -72,3 +72,35 @@ def test_couette_lengths(n, axis):
     phys = spec_to_phys_2d(u0, cfg)
     assert rel_l2(flow.spec_to_phys(dev(u0)).cpu(), phys) < 1e-13
     assert rel_l2(flow.phys_to_spec(dev(phys)).cpu(), u0) < 1e-13
+
+
+@pytest.mark.parametrize("system", ["kolmogorov", "plane-couette"])
+def test_unrolled_step_graph_lengths(system):
+    """Unrolled step graphs on grids of these lengths alone: every kernel of an
+    iteration has to honour the skip flag, so the states equal the host loop's
+    bit for bit with more iterations unrolled than the step takes."""
+    from dnsjax_b200 import driver, initial
+    from dnsjax_b200.flows.monochromatic import TriplyPeriodicFlow
+    from dnsjax_b200.flows.plane_couette import PlaneCouetteFlow
+    from dnsjax_b200.parameters import Parameters
+
+    wall = system == "plane-couette"
+    lz = pi if wall else 2 * pi
+    p = Parameters(phys=dict(system=system, re=60.0), geo=dict(lx=2 * pi, lz=lz),
+                   res=dict(nx=36, ny=33 if wall else 24, nz=72, fd_order=4),
+                   step=dict(dt=0.01, corrector_tolerance=1e-10, max_corrector_iterations=60))
+    if wall:
+        flow = PlaneCouetteFlow(p)
+        u0 = initial.couette_field(36, 33, 72, 2 * pi, lz, 4, 1, 8.0, 1e-3)
+    else:
+        flow = TriplyPeriodicFlow(p, ly=2 * pi)
+        u0 = initial.periodic_field(36, 24, 72, 2 * pi, 2 * pi, 2 * pi, 1,
+                                    initial.kolmogorov_spectrum_cfg0, 1e-2)
+    s_graph, s_host = dev(u0), dev(u0)
+    g = flow.make_step_graph(s_graph, unroll=64)
+    steppers = flow.make_stepper()
+    for _ in range(2):
+        s_host, c, e = driver.step(flow, steppers, s_host, 1e-10, 60)
+        g.launch()
+        assert g.status() == (c, e)
+        assert bool((s_graph == s_host).all())
