@@ -32,7 +32,12 @@ namespace {
 
 constexpr int kTile = 16;       // items per substitution CTA (two sides per item)
 constexpr int kStageWarps = 4;  // modes per CTA in the stage kernels
-constexpr int kSYM = 5;         // y values per lane: y = lane + 32 k, Ny <= 160
+// y values per lane that the stage kernels hold in registers, y = lane + 32 k:
+// kSYM for Ny <= 160, so that all of a mode's inputs are in flight at once; for
+// taller grids (YM = 0) they are read where they are used (96 x 193 x 72, fd 4:
+// 1207 us in the one-warp kernel that ran before, 133 us so).
+constexpr int kSYM = 5;
+constexpr int kMaxNy = 512;  // stage-0 rows of kStageWarps modes fit in shared memory
 
 // L2 residency of the workspaces F and R (K Ny and 3 K Ny complex, 67 MB at
 // 128x129x128, each touched about three times per call): their writes and
@@ -124,13 +129,13 @@ cudaError_t launch_imm_repack(const double* ab, const int* piv, int Ny, int kl, 
 // inputs: f_hat -> F, and Q = H_k^- u^n + c N_j + (1-c) N_n -> R (wall rows
 // zero), so u^n, N_j and N_n are read once per call.
 // ---------------------------------------------------------------------------
-template <int KL>
+template <int KL, int YM>
 __global__ void __launch_bounds__(32 * kStageWarps)
 imm_stage013_kernel(ImmArgs a, const double2* __restrict__ vel_n,
                     const double2* __restrict__ nl_n, const double2* __restrict__ nl_j,
                     double2* __restrict__ F, double2* __restrict__ R) {
   if (a.skip && *a.skip) return;
-  constexpr int S1 = KL + 1, S2 = KL + 2, YM = kSYM;
+  constexpr int S1 = KL + 1, S2 = KL + 2, YR = YM > 0 ? YM : 1;
   extern __shared__ double2 sm[];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
@@ -152,23 +157,25 @@ imm_stage013_kernel(ImmArgs a, const double2* __restrict__ vel_n,
   const double k2 = kx * kx + kz * kz;
   const double c = a.c, dt = a.dt, omc = 1.0 - c, omc_nu = omc * a.nu, idt = 1.0 / dt;
   const unsigned long long keep = l2_keep();
-  double2 nj[3][YM], nn[3][YM];
+  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
+  double2 nj[3][YR], nn[3][YR];
+  auto load = [&](int k, int y) {
+#pragma unroll
+    for (int cpt = 0; cpt < 3; ++cpt) {
+      nj[cpt][k] = nl_j[cpt * CS + mo + y];
+      nn[cpt][k] = nl_n[cpt * CS + mo + y];
+    }
+  };
 #pragma unroll
   for (int k = 0; k < YM; ++k) {
     const int y = lane + 32 * k;
-    if (y < Ny) {
-#pragma unroll
-      for (int cpt = 0; cpt < 3; ++cpt) {
-        nj[cpt][k] = nl_j[cpt * CS + mo + y];
-        nn[cpt][k] = nl_n[cpt * CS + mo + y];
-      }
-    }
+    if (y < Ny) load(k, y);
   }
   cp_async_wait_all();
   __syncwarp();
   // Stage 0: d_hat^n = div u^n
 #pragma unroll
-  for (int k = 0; k < YM; ++k) {
+  for (int k = 0; k < nk; ++k) {
     const int y = lane + 32 * k;
     if (y < Ny)
       D[y] = cadd(cadd(cik(kx, T[y]), band_row<S1>(T + Ny, a.d1_j0, a.d1_wT, Ny, y)),
@@ -176,9 +183,10 @@ imm_stage013_kernel(ImmArgs a, const double2* __restrict__ vel_n,
   }
   __syncwarp();
 #pragma unroll
-  for (int k = 0; k < YM; ++k) {
-    const int y = lane + 32 * k;
+  for (int kk = 0; kk < nk; ++kk) {
+    const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
     if (y >= Ny) continue;
+    if (YM == 0) load(0, y);
     double2 fy = make_double2(0.0, 0.0), qu = fy, qv = fy, qw = fy;
     if (y > 0 && y < Ny - 1) {
       // Stage 1: f_hat
@@ -215,11 +223,11 @@ imm_stage013_kernel(ImmArgs a, const double2* __restrict__ vel_n,
 // Stage 3's pressure gradient: R -= grad p_P on the interior rows (the wall
 // rows of R stay zero), p_P = L_k^-1 f_hat from the L_k substitution in F.
 // ---------------------------------------------------------------------------
-template <int KL>
+template <int KL, int YM>
 __global__ void __launch_bounds__(32 * kStageWarps)
 imm_grad_kernel(ImmArgs a, const double2* __restrict__ P, double2* __restrict__ R) {
   if (a.skip && *a.skip) return;
-  constexpr int S1 = KL + 1, YM = kSYM;
+  constexpr int S1 = KL + 1, YR = YM > 0 ? YM : 1;
   extern __shared__ double2 sm[];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
@@ -232,21 +240,24 @@ imm_grad_kernel(ImmArgs a, const double2* __restrict__ P, double2* __restrict__ 
   cp_async_commit();
   const int iz = m / NKX, ix = m % NKX;
   const double kx = a.kx[ix], kz = a.kz[iz];
-  double2 q[3][YM];
+  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
+  double2 q[3][YR];
+  auto load = [&](int k, int y) {
+#pragma unroll
+    for (int cpt = 0; cpt < 3; ++cpt) q[cpt][k] = ld_l2(R + cpt * CS + mo + y, keep);
+  };
 #pragma unroll
   for (int k = 0; k < YM; ++k) {
     const int y = lane + 32 * k;
-    if (y > 0 && y < Ny - 1) {
-#pragma unroll
-      for (int cpt = 0; cpt < 3; ++cpt) q[cpt][k] = ld_l2(R + cpt * CS + mo + y, keep);
-    }
+    if (y > 0 && y < Ny - 1) load(k, y);
   }
   cp_async_wait_all();
   __syncwarp();
 #pragma unroll
-  for (int k = 0; k < YM; ++k) {
-    const int y = lane + 32 * k;
+  for (int kk = 0; kk < nk; ++kk) {
+    const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
     if (y <= 0 || y >= Ny - 1) continue;
+    if (YM == 0) load(0, y);
     const double2 p = Pp[y];
     st_l2(R + mo + y, csub(q[0][k], cik(kx, p)), keep);
     st_l2(R + CS + mo + y, csub(q[1][k], band_row<S1>(Pp, a.d1_j0, a.d1_wT, Ny, y)), keep);
@@ -257,13 +268,13 @@ imm_grad_kernel(ImmArgs a, const double2* __restrict__ P, double2* __restrict__ 
 // ---------------------------------------------------------------------------
 // Stages 4-6: vel_new, correction, per-mode norm partial.
 // ---------------------------------------------------------------------------
-template <int KL>
+template <int KL, int YM>
 __global__ void __launch_bounds__(32 * kStageWarps)
 imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j,
                   double2* vel_new, double2* __restrict__ corr_out,
                   double* __restrict__ partials) {
   if (a.skip && *a.skip) return;
-  constexpr int S1 = KL + 1, YM = kSYM;
+  constexpr int S1 = KL + 1, YR = YM > 0 ? YM : 1;
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
   const int m = blockIdx.x * kStageWarps + wq;
@@ -272,23 +283,25 @@ imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j
   const int iz = m / NKX, ix = m % NKX;
   const double kx = a.kx[ix], kz = a.kz[iz];
   const double k2 = kx * kx + kz * kz;
-  double2 vj[3][YM], ra[3][YM];
-  double c1[YM], c2[YM], e1[YM], e2[YM];
+  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
+  double2 vj[3][YR], ra[3][YR];
+  double c1[YR], c2[YR], e1[YR], e2[YR];
   const unsigned long long drop = l2_drop();
+  auto load = [&](int k, int y) {
+#pragma unroll
+    for (int cpt = 0; cpt < 3; ++cpt) {
+      vj[cpt][k] = vel_j[cpt * CS + mo + y];
+      ra[cpt][k] = ld_l2(R + cpt * CS + mo + y, drop);
+    }
+    c1[k] = a.v1[mo + y];
+    c2[k] = a.v2[mo + y];
+    e1[k] = a.q1[mo + y];
+    e2[k] = a.q2[mo + y];
+  };
 #pragma unroll
   for (int k = 0; k < YM; ++k) {
     const int y = lane + 32 * k;
-    if (y < Ny) {
-#pragma unroll
-      for (int cpt = 0; cpt < 3; ++cpt) {
-        vj[cpt][k] = vel_j[cpt * CS + mo + y];
-        ra[cpt][k] = ld_l2(R + cpt * CS + mo + y, drop);
-      }
-      c1[k] = a.v1[mo + y];
-      c2[k] = a.v2[mo + y];
-      e1[k] = a.q1[mo + y];
-      e2[k] = a.q2[mo + y];
-    }
+    if (y < Ny) load(k, y);
   }
   // Stages 4-5: wall divergence and influence-matrix weights
   const double2* va = R + CS + mo;
@@ -304,9 +317,10 @@ imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j
   const double km = (ix == 0 && a.kx0) ? 1.0 : 2.0;
   double acc = 0.0;
 #pragma unroll
-  for (int k = 0; k < YM; ++k) {
-    const int y = lane + 32 * k;
+  for (int kk = 0; kk < nk; ++kk) {
+    const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
     if (y >= Ny) continue;
+    if (YM == 0) load(0, y);
     const double2 vnew = cadd(cadd(ra[1][k], cscale(a1, c1[k])), cscale(a2, c2[k]));
     const double2 qq = cadd(cscale(a1, e1[k]), cscale(a2, e2[k]));
     const double2 unew = csub(ra[0][k], cik(kx, qq));
@@ -734,7 +748,7 @@ static size_t imm_batch_grad_smem(int Ny) {
 }
 
 bool imm_batch_supported(int kl, int ny) {
-  return (kl == 2 || kl == 4 || kl == 6 || kl == 8) && ny <= 32 * kSYM;
+  return (kl == 2 || kl == 4 || kl == 6 || kl == 8) && ny <= kMaxNy;
 }
 
 // Ring slot bytes of one substitution launch: the larger of a forward block
@@ -788,7 +802,7 @@ static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, int ncom
   return cudaGetLastError();
 }
 
-template <int K>
+template <int K, int YM>
 static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2* vel_n,
                            const double2* vel_j, const double2* nl_n, const double2* nl_j,
                            double2* vel_new, double2* corr_out, double* partials,
@@ -797,15 +811,15 @@ static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2*
   const int grid = (NM + kStageWarps - 1) / kStageWarps;
   const size_t sm = imm_batch_stage_smem(Ny);
   cudaError_t e;
-  imm_stage013_kernel<K><<<grid, 32 * kStageWarps, sm, st>>>(a, vel_n, nl_n, nl_j, bt.F, bt.R);
+  imm_stage013_kernel<K, YM><<<grid, 32 * kStageWarps, sm, st>>>(a, vel_n, nl_n, nl_j, bt.F, bt.R);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = solve_launch<K>(bt, 0, bt.F, 1, NM, Ny, a.NKX, a.NZ1, a.skip, st);
   if (e != cudaSuccess) return e;
-  imm_grad_kernel<K><<<grid, 32 * kStageWarps, imm_batch_grad_smem(Ny), st>>>(a, bt.F, bt.R);
+  imm_grad_kernel<K, YM><<<grid, 32 * kStageWarps, imm_batch_grad_smem(Ny), st>>>(a, bt.F, bt.R);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = solve_launch<K>(bt, 1, bt.R, 3, NM, Ny, a.NKX, a.NZ1, a.skip, st);
   if (e != cudaSuccess) return e;
-  imm_stage6_kernel<K><<<grid, 32 * kStageWarps, 0, st>>>(a, bt.R, vel_j, vel_new, corr_out,
+  imm_stage6_kernel<K, YM><<<grid, 32 * kStageWarps, 0, st>>>(a, bt.R, vel_j, vel_new, corr_out,
                                                           partials);
   return cudaGetLastError();
 }
@@ -815,21 +829,26 @@ cudaError_t launch_imm_batch(const ImmArgs& a, const ImmBatch& bt, const double2
                              const double2* vel_j, const double2* nl_n,
                              const double2* nl_j, double2* vel_new, double2* corr_out,
                              double* partials, cudaStream_t st) {
+  const bool regs = a.Ny <= 32 * kSYM;
   switch (a.kl) {
-    case 2: return pipeline<2>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
-    case 4: return pipeline<4>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
-    case 6: return pipeline<6>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
-    case 8: return pipeline<8>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
+#define DNSB_PIPE(K)                                                                          \
+  case K:                                                                                     \
+    return regs ? pipeline<K, kSYM>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out,       \
+                                    partials, st)                                             \
+                : pipeline<K, 0>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
+    DNSB_PIPE(2) DNSB_PIPE(4) DNSB_PIPE(6) DNSB_PIPE(8)
+#undef DNSB_PIPE
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t set_imm_batch_attributes(int max_smem) {
   const void* fns[] = {
-      (const void*)imm_stage013_kernel<2>, (const void*)imm_stage013_kernel<4>,
-      (const void*)imm_stage013_kernel<6>, (const void*)imm_stage013_kernel<8>,
-      (const void*)imm_grad_kernel<2>,     (const void*)imm_grad_kernel<4>,
-      (const void*)imm_grad_kernel<6>,     (const void*)imm_grad_kernel<8>,
+#define DNSB_STAGE_FNS(K)                                                        \
+  (const void*)imm_stage013_kernel<K, kSYM>, (const void*)imm_stage013_kernel<K, 0>, \
+      (const void*)imm_grad_kernel<K, kSYM>, (const void*)imm_grad_kernel<K, 0>
+      DNSB_STAGE_FNS(2), DNSB_STAGE_FNS(4), DNSB_STAGE_FNS(6), DNSB_STAGE_FNS(8),
+#undef DNSB_STAGE_FNS
 #define DNSB_SOLVE_FNS(K) \
   (const void*)imm_solve_kernel<K, K + 1>, (const void*)imm_solve_kernel<K, 2 * K>
       DNSB_SOLVE_FNS(2), DNSB_SOLVE_FNS(4), DNSB_SOLVE_FNS(6), DNSB_SOLVE_FNS(8)};

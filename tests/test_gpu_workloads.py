@@ -99,8 +99,8 @@ def test_couette_64_one_step():
 
 
 def test_couette_tall_wall_normal_grid():
-    """ny = 193 is beyond the batched IMM's wall-normal limit (160), so the
-    one-kernel IMM runs, and nx = nz = 16 (padded 24) takes the
+    """ny = 193 is beyond the heights whose inputs the IMM's stage kernels hold
+    in registers (160), and nx = nz = 16 (padded 24) takes the
     runtime-planned passes: two steps against the oracle."""
     from dnsjax_b200 import driver, initial
     from oracle.stepper import run
