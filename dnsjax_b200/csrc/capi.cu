@@ -1278,6 +1278,8 @@ struct dnsb_couette {
   unsigned char* dp = nullptr;
   double2* Fw = nullptr;
   double2* Rw = nullptr;
+  double *w1x = nullptr, *w2x = nullptr;  // stage-kernel windows (null: not batched)
+  int* wbase = nullptr;
   ImmBatch batch{};
   bool batch_ready = false;
   int wait_limit = 1 << 20;  // substitution ring: polls before a wait gives up
@@ -1327,7 +1329,7 @@ struct dnsb_couette {
 static void couette_free(dnsb_couette* p) {
   void* ptrs[] = {p->twz, p->twx, p->twz32, p->twx32, p->kx, p->kz, p->d1w, p->d2w, p->d1wT, p->d2wT, p->d1j0,
                   p->d2j0, p->U, p->cU, p->nU, p->simpson, p->B, p->partials,
-                  p->status, p->fac, p->dp, p->Fw, p->Rw, p->slab.Bx};
+                  p->status, p->fac, p->dp, p->Fw, p->Rw, p->w1x, p->w2x, p->wbase, p->slab.Bx};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   delete p;
@@ -1424,6 +1426,15 @@ extern "C" int dnsb_couette_create(const dnsb_couette_desc* d,
     chk(upload(&p->d1wT, t1.data(), t1.size()));
     chk(upload(&p->d2wT, t2.data(), t2.size()));
   }
+  if (imm_batch_supported(pord, p->Ny) &&
+      imm_batch_windows_ok(p->Ny, pord, d->d1_j0, d->d2_j0)) {
+    std::vector<int> base;
+    std::vector<double> w1x, w2x;
+    imm_batch_windows(p->Ny, pord, d->d1_j0, d->d1_w, d->d2_j0, d->d2_w, &base, &w1x, &w2x);
+    chk(upload(&p->wbase, base.data(), base.size()));
+    chk(upload(&p->w1x, w1x.data(), w1x.size()));
+    chk(upload(&p->w2x, w2x.data(), w2x.size()));
+  }
   chk(upload(&p->U, d->base_flow, 3 * (size_t)p->Ny));
   chk(upload(&p->cU, d->curl_base_flow, 3 * (size_t)p->Ny));
   chk(upload(&p->nU, d->nonlin_base_flow, 3 * (size_t)p->Ny));
@@ -1495,10 +1506,15 @@ static int bind_batch(dnsb_couette* p) {
   const size_t fac_bytes = 2 * (nL + nU) * sizeof(double);
   cudaError_t e1 = cudaMalloc(&p->fac, fac_bytes);
   cudaError_t e2 = cudaMalloc(&p->dp, 2 * nP);
-  cudaError_t e3 = cudaMalloc(&p->Fw, (size_t)p->NM * p->Ny * sizeof(double2));
-  cudaError_t e4 = cudaMalloc(&p->Rw, 3 * (size_t)p->NM * p->Ny * sizeof(double2));
+  // [tile][y][32 lanes], zero in the lanes of no mode
+  const size_t wbytes = (size_t)ntiles * p->Ny * 2 * tile * sizeof(double2);
+  cudaError_t e3 = cudaMalloc(&p->Fw, wbytes);
+  cudaError_t e4 = cudaMalloc(&p->Rw, 3 * wbytes);
   if (e1 || e2 || e3 || e4) return fail(DNSB_ERR_CUDA, "IMM workspace allocation failed");
-  if (cudaMemset(p->fac, 0, fac_bytes) != cudaSuccess || cudaMemset(p->dp, 0, 2 * nP) != cudaSuccess)
+  if (cudaMemset(p->fac, 0, fac_bytes) != cudaSuccess ||
+      cudaMemset(p->dp, 0, 2 * nP) != cudaSuccess ||
+      cudaMemset(p->Fw, 0, wbytes) != cudaSuccess ||
+      cudaMemset(p->Rw, 0, 3 * wbytes) != cudaSuccess)
     return fail(DNSB_ERR_CUDA, "cudaMemset failed");
   ImmBatch& b = p->batch;
   const double* abs_[2] = {p->ops.Lk_ab, p->ops.Hk_ab};
@@ -1524,6 +1540,9 @@ static int bind_batch(dnsb_couette* p) {
   b.wait_limit = p->wait_limit;
   b.F = p->Fw;
   b.R = p->Rw;
+  b.w1x = p->w1x;
+  b.w2x = p->w2x;
+  b.base = p->wbase;
   p->batch_ready = true;
   return 0;
 }
@@ -1573,7 +1592,7 @@ extern "C" int dnsb_couette_bind_imm(dnsb_couette* p, const dnsb_imm_ops* ops) {
   p->ab_row0 = h_row;
   p->bound = true;
   p->batch_ready = false;
-  if (imm_batch_supported(p->p, p->Ny)) {
+  if (p->w1x) {
     rc = bind_batch(p);
     if (rc) return rc;
   }

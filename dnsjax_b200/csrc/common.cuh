@@ -681,6 +681,14 @@ __device__ __forceinline__ float2 ld_l2(const float2* g, unsigned long long pol)
                : "memory");
   return v;
 }
+// A load of data used once: no line allocated in L1.
+__device__ __forceinline__ double2 ld_stream(const double2* g) {
+  double2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];\n"
+               : "=d"(v.x), "=d"(v.y)
+               : "l"(g));
+  return v;
+}
 __device__ __forceinline__ void cp_async16_l2(void* smem, const void* g, unsigned long long pol) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g),

@@ -4,26 +4,35 @@
 // dgbtrs-'N' substitution of src/dnsjax/geometries/cartesian.py:360-441.
 //
 //   stages 0-1   one warp per (kz, kx) mode: d_hat = div u^n, then f_hat
-//   (+ 3)        (D1 / D2 along y from shared memory) -> F      [NM][Ny],
-//                and in the same pass the part of stage 3 that does not
-//                need p_P, Q = H_k^- u^n + c N_j + (1-c) N_n -> R [3][NM][Ny]
-//   L_k solve    p_P = L_k^-1 f_hat in place in F: a CTA per 16 items, one
-//                warp per component, lane = side * 16 + item (side 1 is the
+//   (+ 3)        (D1 / D2 along y) -> F, and in the same pass the part of
+//                stage 3 that does not need p_P, Q = H_k^- u^n + c N_j + (1-c)
+//                N_n -> R, so u^n, N_j and N_n are read once per call
+//   L_k solve    p_P = L_k^-1 f_hat in place in F: a CTA per tile of 16 items,
+//                one warp per component, lane = side * 16 + item (side 1 is the
 //                mirror mode (nz-1-s, kx) of item (s, kx) when it shares the
 //                item's factors), each lane one complex column
-//   stage 3      one warp per mode: R = Q - grad p_P (interior rows)
+//   stage 3      R -= grad p_P on the interior rows
 //   H_k solve    as the L_k solve, three components, in place in R
 //   stages 4-6   one warp per mode: wall divergence, influence-matrix
 //                weights, u^{j+1}, the correction and its Simpson norm
 //
+// The workspaces F and R[3] are laid out for the substitutions, [tile][y][32
+// lanes]: a row of a tile is 512 contiguous bytes, so the rows that enter a
+// block of substitution steps are one bulk copy and every result row one
+// coalesced store.  (As [mode][y], which the kernels ran on before, each lane's
+// 16 bytes were a sector of their own, read and written twice per solve: the
+// L_k / H_k launches took 38 / 68 us at 128 x 129 x 128.)  The stage kernels
+// transpose through shared memory, four modes (64 bytes of a row) at a time.
+//
 // The LU factors are repacked once, when the operators are bound, into
 // 16-item tiles whose rows are contiguous (layout below), so a block of
-// substitution steps of one tile is one bulk copy into shared memory; the
-// substitution kernels stream those blocks through a ring of slots, each
-// lane fetching its own entering rows with cp.async.
+// substitution steps of one tile is one bulk copy into shared memory.
 // An item is mode (s, kx) with s <= (nz-1)/2; when the factors of (s, kx)
 // and its mirror (nz-1-s, kx) are bit-identical (same k^2; checked at bind
 // time) the mirror reads the item's records, else every mode is an item.
+#include <algorithm>
+#include <vector>
+
 #include "solver.cuh"
 
 namespace dnsb {
@@ -31,37 +40,26 @@ namespace dnsb {
 namespace {
 
 constexpr int kTile = 16;       // items per substitution CTA (two sides per item)
+constexpr int kLanes = 2 * kTile;  // lanes of a tile row (two sides)
 constexpr int kStageWarps = 4;  // modes per CTA in the stage kernels
-// y values per lane that the stage kernels hold in registers, y = lane + 32 k:
-// kSYM for Ny <= 160, so that all of a mode's inputs are in flight at once; for
-// taller grids (YM = 0) they are read where they are used (96 x 193 x 72, fd 4:
-// 1207 us in the one-warp kernel that ran before, 133 us so).
-constexpr int kSYM = 5;
-constexpr int kMaxNy = 512;  // stage-0 rows of kStageWarps modes fit in shared memory
 
 // L2 residency of the workspaces F and R (K Ny and 3 K Ny complex, 67 MB at
-// 128x129x128, each touched about three times per call): their writes and
-// the substitutions' accesses carry an evict_last policy, and their last
-// reads (F in the gradient kernel, R in stage 6) evict_first, so the streamed
-// inputs do not push them out of the 126 MB L2 between the kernels of one call
-// (l2_keep / l2_drop and the hinted accesses are in common.cuh).
+// 128x129x128, each touched about three times per call): their writes carry an
+// evict_last policy, and their last reads (F in the gradient kernel, R in stage
+// 6) evict_first, so the streamed inputs do not push them out of the 126 MB L2
+// between the kernels of one call (l2_keep / l2_drop and the hinted accesses
+// are in common.cuh).
 
-// Banded stencil row y applied to x: sum_m w[m][y] x[j0[y] + m], with the
-// weights stored tap-major ([S][Ny]) so the lanes of a warp (consecutive y)
-// read each tap's weights contiguously.
-template <int S>
-__device__ __forceinline__ double2 band_row(const double2* x, const int* __restrict__ j0,
-                                            const double* __restrict__ wT, int Ny, int y) {
-  const int j = j0[y];
-  double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int m = 0; m < S; ++m) {
-    const double wm = wT[m * Ny + y];
-    const double2 v = x[j + m];
-    acc.x += wm * v.x;
-    acc.y += wm * v.y;
-  }
-  return acc;
+// Tile and lane of mode m: item p on side 0, or the mirror of item p on side 1.
+struct ModeSlot {
+  long long tile;
+  int lane;
+};
+__device__ __forceinline__ ModeSlot mode_slot(int m, int NKX, int NZ1, int paired) {
+  const int s = m / NKX, ix = m % NKX;
+  const bool mirror = paired && s >= (NZ1 + 1) / 2;
+  const int p = mirror ? (NZ1 - s) * NKX + ix : m;
+  return {p / kTile, (mirror ? kTile : 0) + p % kTile};
 }
 
 }  // namespace
@@ -125,174 +123,261 @@ cudaError_t launch_imm_repack(const double* ab, const int* piv, int Ny, int kl, 
 }
 
 // ---------------------------------------------------------------------------
-// Stages 0-1 and the pressure-free part of stage 3, in one pass over the
-// inputs: f_hat -> F, and Q = H_k^- u^n + c N_j + (1-c) N_n -> R (wall rows
-// zero), so u^n, N_j and N_n are read once per call.
+// Stages 0-1 and the pressure-free part of stage 3.  One warp per mode, lane l
+// the YM consecutive rows y = YM l + o, four modes per CTA.
+//
+// With N = c N_j + (1-c) N_n, f_hat = d/dt + div N + (1-c) nu (D2 - k2) d and
+// Q = u/dt + (1-c) nu (D2 - k2) u + N.  A lane walks the W = S2 + YM - 1 rows its
+// YM rows' stencils reach, adding each row to the YM sums it belongs to: one
+// shared-memory read per row of the window instead of one per tap and row, and
+// 2 YM or more independent sums in flight.  The weights come window-relative
+// ([o][W][32 lanes], zero outside the stencil), so rows whose stencils are
+// shifted at the walls run the same code.  YM is odd, so lanes YM rows apart
+// read without bank conflicts.  All rows live in place in 7 Ny complex values a
+// mode (3 CTAs per SM at 129 rows): Q_u, Q_v, Q_w over N, f over d.
 // ---------------------------------------------------------------------------
+// Values per mode in shared memory: 7 Ny, rounded so that the four modes of a
+// row fall on other banks when the CTA writes it out.
+__host__ __device__ constexpr int stage_stride(int Ny) { return ((7 * Ny + 5) / 8) * 8 + 2; }
+
+__device__ __forceinline__ void axpy(double2& acc, double w, double2 x) {
+  acc.x += w * x.x;
+  acc.y += w * x.y;
+}
+
 template <int KL, int YM>
-__global__ void __launch_bounds__(32 * kStageWarps)
-imm_stage013_kernel(ImmArgs a, const double2* __restrict__ vel_n,
-                    const double2* __restrict__ nl_n, const double2* __restrict__ nl_j,
-                    double2* __restrict__ F, double2* __restrict__ R) {
+__global__ void __launch_bounds__(32 * kStageWarps, YM == 5 ? 3 : 1)
+imm_stage013_kernel(ImmArgs a, int paired, const double* __restrict__ w1x,
+                    const double* __restrict__ w2x, const int* __restrict__ base,
+                    const double2* __restrict__ vel_n, const double2* __restrict__ nl_n,
+                    const double2* __restrict__ nl_j, double2* __restrict__ F,
+                    double2* __restrict__ R, long long cs) {
   if (a.skip && *a.skip) return;
-  constexpr int S1 = KL + 1, S2 = KL + 2, YR = YM > 0 ? YM : 1;
+  constexpr int W = KL + 2 + YM - 1;
   extern __shared__ double2 sm[];
+  __shared__ long long s_dst[kStageWarps];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
   const int m = blockIdx.x * kStageWarps + wq;
-  if (m >= NM) return;  // no CTA-wide barrier below
-  double2* T = sm + wq * 6 * Ny;  // u^n, v^n, w^n, N^j_v, N^n_v, d_hat^n
-  double2* D = T + 5 * Ny;
-  const long long CS = (long long)NM * Ny, mo = (long long)m * Ny;
-  for (int y = lane; y < Ny; y += 32) {
-    cp_async16(T + y, vel_n + mo + y);
-    cp_async16(T + Ny + y, vel_n + CS + mo + y);
-    cp_async16(T + 2 * Ny + y, vel_n + 2 * CS + mo + y);
-    cp_async16(T + 3 * Ny + y, nl_j + CS + mo + y);
-    cp_async16(T + 4 * Ny + y, nl_n + CS + mo + y);
+  const bool act = m < NM;
+  const int SS = stage_stride(Ny);
+  if (act) {
+    double2* T = sm + wq * SS;  // u, v, w, N_u, N_v, N_w, d
+    double2 *Nr = T + 3 * Ny, *D = T + 6 * Ny;
+    const long long CS = (long long)NM * Ny, mo = (long long)m * Ny;
+    if (lane == 0) {
+      const ModeSlot ms = mode_slot(m, NKX, a.NZ1, paired);
+      s_dst[wq] = ms.tile * Ny * kLanes + ms.lane;
+    }
+    for (int y = lane; y < Ny; y += 32) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cp_async16(T + c * Ny + y, vel_n + c * CS + mo + y);
+    }
+    cp_async_commit();
+    const int iz = m / NKX, ix = m % NKX;
+    const double kx = a.kx[ix], kz = a.kz[iz];
+    const double k2 = kx * kx + kz * kz;
+    const double c = a.c, omc = 1.0 - c, omc_nu = omc * a.nu, idt = 1.0 / a.dt;
+    {
+      double2 nj[3][YM], nn[3][YM];
+#pragma unroll
+      for (int k = 0; k < YM; ++k) {
+        const int y = lane + 32 * k;
+        if (y < Ny) {
+#pragma unroll
+          for (int cpt = 0; cpt < 3; ++cpt) {
+            // streamed once: keep the weights in L1
+            nj[cpt][k] = ld_stream(nl_j + cpt * CS + mo + y);
+            nn[cpt][k] = ld_stream(nl_n + cpt * CS + mo + y);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < YM; ++k) {
+        const int y = lane + 32 * k;
+        if (y < Ny) {
+#pragma unroll
+          for (int cpt = 0; cpt < 3; ++cpt)
+            Nr[cpt * Ny + y] = cadd(cscale(nj[cpt][k], c), cscale(nn[cpt][k], omc));
+        }
+      }
+    }
+    cp_async_wait_all();
+    __syncwarp();
+    const int y0 = YM * lane, b = base[lane];
+    const double *w1 = w1x + lane, *w2 = w2x + lane;
+    double2 f[YM], qv[YM];
+    {
+      // d_hat = div u^n, Q, and div N but for D1 N_v
+      double2 su[YM], sv[YM], sw[YM], dv[YM];
+#pragma unroll
+      for (int o = 0; o < YM; ++o) su[o] = sv[o] = sw[o] = dv[o] = make_double2(0.0, 0.0);
+#pragma unroll 2
+      for (int i = 0; i < W; ++i) {
+        const int r = min(b + i, Ny - 1);
+        const double2 xu = T[r], xv = T[Ny + r], xw = T[2 * Ny + r];
+#pragma unroll
+        for (int o = 0; o < YM; ++o) {
+          const double c1 = w1[(o * W + i) * 32], c2 = w2[(o * W + i) * 32];
+          axpy(dv[o], c1, xv);
+          axpy(su[o], c2, xu);
+          axpy(sv[o], c2, xv);
+          axpy(sw[o], c2, xw);
+        }
+      }
+#pragma unroll
+      for (int o = 0; o < YM; ++o) {
+        const int y = y0 + o;
+        if (y < Ny) {
+          const bool in = y > 0 && y < Ny - 1;
+          const double2 zero = make_double2(0.0, 0.0);
+          const double2 u = T[y], v = T[Ny + y], w = T[2 * Ny + y];
+          const double2 nu = Nr[y], nv = Nr[Ny + y], nw = Nr[2 * Ny + y];
+          D[y] = cadd(cadd(cik(kx, u), dv[o]), cik(kz, w));
+          f[o] = cadd(cik(kx, nu), cik(kz, nw));
+          const double2 hu = cadd(cscale(u, idt), cscale(csub(su[o], cscale(u, k2)), omc_nu));
+          const double2 hv = cadd(cscale(v, idt), cscale(csub(sv[o], cscale(v, k2)), omc_nu));
+          const double2 hw = cadd(cscale(w, idt), cscale(csub(sw[o], cscale(w, k2)), omc_nu));
+          Nr[y] = in ? cadd(hu, nu) : zero;
+          qv[o] = in ? cadd(hv, nv) : zero;
+          Nr[2 * Ny + y] = in ? cadd(hw, nw) : zero;
+        }
+      }
+    }
+    __syncwarp();  // every D row written
+    {
+      double2 dn[YM], sd[YM];
+#pragma unroll
+      for (int o = 0; o < YM; ++o) dn[o] = sd[o] = make_double2(0.0, 0.0);
+#pragma unroll 2
+      for (int i = 0; i < W; ++i) {
+        const int r = min(b + i, Ny - 1);
+        const double2 xn = Nr[Ny + r], xd = D[r];
+#pragma unroll
+        for (int o = 0; o < YM; ++o) {
+          axpy(dn[o], w1[(o * W + i) * 32], xn);
+          axpy(sd[o], w2[(o * W + i) * 32], xd);
+        }
+      }
+#pragma unroll
+      for (int o = 0; o < YM; ++o) {
+        const int y = y0 + o;
+        if (y < Ny) {
+          const double2 d = D[y];
+          const double2 Lkd = csub(sd[o], cscale(d, k2));
+          f[o] = cadd(cadd(cscale(d, idt), cadd(f[o], dn[o])), cscale(Lkd, omc_nu));
+        }
+      }
+    }
+    __syncwarp();  // every D and N_v row read
+#pragma unroll
+    for (int o = 0; o < YM; ++o) {
+      const int y = y0 + o;
+      if (y < Ny) {
+        D[y] = (y > 0 && y < Ny - 1) ? f[o] : make_double2(0.0, 0.0);
+        Nr[Ny + y] = qv[o];
+      }
+    }
   }
-  cp_async_commit();
-  const int iz = m / NKX, ix = m % NKX;
-  const double kx = a.kx[ix], kz = a.kz[iz];
-  const double k2 = kx * kx + kz * kz;
-  const double c = a.c, dt = a.dt, omc = 1.0 - c, omc_nu = omc * a.nu, idt = 1.0 / dt;
+  __syncthreads();
+  // Out to the tiles, four modes of a row at a time.
   const unsigned long long keep = l2_keep();
-  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
-  double2 nj[3][YR], nn[3][YR];
-  auto load = [&](int k, int y) {
+  const int nm = min(kStageWarps, NM - (int)blockIdx.x * kStageWarps);
+  const int q = threadIdx.x & 3;
+  if (q < nm) {
+    const double2* src = sm + q * SS + 3 * Ny;
+    const long long dst = s_dst[q];
+    for (int y = threadIdx.x >> 2; y < Ny; y += 8 * kStageWarps) {
+      const long long d = dst + (long long)y * kLanes;
 #pragma unroll
-    for (int cpt = 0; cpt < 3; ++cpt) {
-      nj[cpt][k] = nl_j[cpt * CS + mo + y];
-      nn[cpt][k] = nl_n[cpt * CS + mo + y];
+      for (int cpt = 0; cpt < 3; ++cpt) st_l2(R + cpt * cs + d, src[cpt * Ny + y], keep);
+      st_l2(F + d, src[3 * Ny + y], keep);
     }
-  };
-#pragma unroll
-  for (int k = 0; k < YM; ++k) {
-    const int y = lane + 32 * k;
-    if (y < Ny) load(k, y);
-  }
-  cp_async_wait_all();
-  __syncwarp();
-  // Stage 0: d_hat^n = div u^n
-#pragma unroll
-  for (int k = 0; k < nk; ++k) {
-    const int y = lane + 32 * k;
-    if (y < Ny)
-      D[y] = cadd(cadd(cik(kx, T[y]), band_row<S1>(T + Ny, a.d1_j0, a.d1_wT, Ny, y)),
-                  cik(kz, T[2 * Ny + y]));
-  }
-  __syncwarp();
-#pragma unroll
-  for (int kk = 0; kk < nk; ++kk) {
-    const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
-    if (y >= Ny) continue;
-    if (YM == 0) load(0, y);
-    double2 fy = make_double2(0.0, 0.0), qu = fy, qv = fy, qw = fy;
-    if (y > 0 && y < Ny - 1) {
-      // Stage 1: f_hat
-      const double2 divNj = cadd(cadd(cik(kx, nj[0][k]),
-                                      band_row<S1>(T + 3 * Ny, a.d1_j0, a.d1_wT, Ny, y)),
-                                 cik(kz, nj[2][k]));
-      const double2 divNn = cadd(cadd(cik(kx, nn[0][k]),
-                                      band_row<S1>(T + 4 * Ny, a.d1_j0, a.d1_wT, Ny, y)),
-                                 cik(kz, nn[2][k]));
-      const double2 dy = D[y];
-      const double2 Lkd = csub(band_row<S2>(D, a.d2_j0, a.d2_wT, Ny, y), cscale(dy, k2));
-      const double2 dd = make_double2(dy.x / dt, dy.y / dt);
-      fy = cadd(cadd(cadd(dd, cscale(divNj, c)), cscale(divNn, omc)), cscale(Lkd, omc_nu));
-      // Stage 3 without the pressure gradient
-      const double2 u = T[y], v = T[Ny + y], w = T[2 * Ny + y];
-      const double2 D2u = band_row<S2>(T, a.d2_j0, a.d2_wT, Ny, y);
-      const double2 D2v = band_row<S2>(T + Ny, a.d2_j0, a.d2_wT, Ny, y);
-      const double2 D2w = band_row<S2>(T + 2 * Ny, a.d2_j0, a.d2_wT, Ny, y);
-      const double2 hu = cadd(cscale(u, idt), cscale(csub(D2u, cscale(u, k2)), omc_nu));
-      const double2 hv = cadd(cscale(v, idt), cscale(csub(D2v, cscale(v, k2)), omc_nu));
-      const double2 hw = cadd(cscale(w, idt), cscale(csub(D2w, cscale(w, k2)), omc_nu));
-      qu = cadd(cadd(hu, cscale(nj[0][k], c)), cscale(nn[0][k], omc));
-      qv = cadd(cadd(hv, cscale(nj[1][k], c)), cscale(nn[1][k], omc));
-      qw = cadd(cadd(hw, cscale(nj[2][k], c)), cscale(nn[2][k], omc));
-    }
-    st_l2(F + mo + y, fy, keep);
-    st_l2(R + mo + y, qu, keep);
-    st_l2(R + CS + mo + y, qv, keep);
-    st_l2(R + 2 * CS + mo + y, qw, keep);
   }
 }
 
 // ---------------------------------------------------------------------------
 // Stage 3's pressure gradient: R -= grad p_P on the interior rows (the wall
 // rows of R stay zero), p_P = L_k^-1 f_hat from the L_k substitution in F.
+// Thread = (row, lane) of a tile: every access is a whole tile row, and the
+// rows of p that a block's stencils share come from L1.
 // ---------------------------------------------------------------------------
+constexpr int kGradRows = 8;
+
+template <int KL>
+__global__ void __launch_bounds__(kLanes * kGradRows)
+imm_grad_kernel(ImmArgs a, int paired, int NP, const double2* __restrict__ P,
+                double2* __restrict__ R, long long cs) {
+  if (a.skip && *a.skip) return;
+  constexpr int S1 = KL + 1;
+  const int lane = threadIdx.x & 31, side = lane / kTile, Ny = a.Ny;
+  const int y = blockIdx.x * kGradRows + (threadIdx.x >> 5) + 1;
+  if (y >= Ny - 1) return;
+  const long long t0 = (long long)blockIdx.y * Ny * kLanes + lane;
+  const int p = blockIdx.y * kTile + lane % kTile, s = p / a.NKX;
+  const bool live = p < NP && (side == 0 || (paired && s != 0));
+  if (!live) return;
+  const double kx = a.kx[p % a.NKX], kz = a.kz[side ? a.NZ1 - s : s];
+  const unsigned long long keep = l2_keep();
+  double2* r = R + t0 + (long long)y * kLanes;
+  const double2 r0 = ld_l2(r, keep), r1 = ld_l2(r + cs, keep), r2 = ld_l2(r + 2 * cs, keep);
+  const double2 pc = P[t0 + (long long)y * kLanes];
+  const double2* pw = P + t0 + (long long)a.d1_j0[y] * kLanes;
+  double2 dp = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int i = 0; i < S1; ++i) {
+    const double w = a.d1_w[y * S1 + i];
+    const double2 v = pw[i * kLanes];
+    dp.x += w * v.x;
+    dp.y += w * v.y;
+  }
+  st_l2(r, csub(r0, cik(kx, pc)), keep);
+  st_l2(r + cs, csub(r1, dp), keep);
+  st_l2(r + 2 * cs, csub(r2, cik(kz, pc)), keep);
+}
+
+// ---------------------------------------------------------------------------
+// Stages 4-6: vel_new, correction, per-mode norm partial.  One warp per mode,
+// y over the lanes; R comes out of the tiles through shared memory, four modes
+// of a row at a time.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int assemble_stride(int Ny) { return ((3 * Ny + 5) / 8) * 8 + 2; }
+
+// YM: rows per lane whose inputs are held in registers (all in flight at once;
+// Ny <= 32 YM), or 0: read where they are used.
 template <int KL, int YM>
 __global__ void __launch_bounds__(32 * kStageWarps)
-imm_grad_kernel(ImmArgs a, const double2* __restrict__ P, double2* __restrict__ R) {
+imm_stage6_kernel(ImmArgs a, int paired, const double2* __restrict__ R, long long cs,
+                  const double2* vel_j, double2* vel_new, double2* __restrict__ corr_out,
+                  double* __restrict__ partials) {
   if (a.skip && *a.skip) return;
   constexpr int S1 = KL + 1, YR = YM > 0 ? YM : 1;
   extern __shared__ double2 sm[];
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
+  const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX, SS = assemble_stride(Ny);
   const int m = blockIdx.x * kStageWarps + wq;
-  if (m >= NM) return;
-  double2* Pp = sm + wq * Ny;
-  const long long CS = (long long)NM * Ny, mo = (long long)m * Ny;
-  const unsigned long long keep = l2_keep(), drop = l2_drop();
-  for (int y = lane; y < Ny; y += 32) cp_async16_l2(Pp + y, P + mo + y, drop);
-  cp_async_commit();
-  const int iz = m / NKX, ix = m % NKX;
-  const double kx = a.kx[ix], kz = a.kz[iz];
-  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
-  double2 q[3][YR];
-  auto load = [&](int k, int y) {
-#pragma unroll
-    for (int cpt = 0; cpt < 3; ++cpt) q[cpt][k] = ld_l2(R + cpt * CS + mo + y, keep);
-  };
-#pragma unroll
-  for (int k = 0; k < YM; ++k) {
-    const int y = lane + 32 * k;
-    if (y > 0 && y < Ny - 1) load(k, y);
-  }
-  cp_async_wait_all();
-  __syncwarp();
-#pragma unroll
-  for (int kk = 0; kk < nk; ++kk) {
-    const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
-    if (y <= 0 || y >= Ny - 1) continue;
-    if (YM == 0) load(0, y);
-    const double2 p = Pp[y];
-    st_l2(R + mo + y, csub(q[0][k], cik(kx, p)), keep);
-    st_l2(R + CS + mo + y, csub(q[1][k], band_row<S1>(Pp, a.d1_j0, a.d1_wT, Ny, y)), keep);
-    st_l2(R + 2 * CS + mo + y, csub(q[2][k], cik(kz, p)), keep);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Stages 4-6: vel_new, correction, per-mode norm partial.
-// ---------------------------------------------------------------------------
-template <int KL, int YM>
-__global__ void __launch_bounds__(32 * kStageWarps)
-imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j,
-                  double2* vel_new, double2* __restrict__ corr_out,
-                  double* __restrict__ partials) {
-  if (a.skip && *a.skip) return;
-  constexpr int S1 = KL + 1, YR = YM > 0 ? YM : 1;
-  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  const int NKX = a.NKX, Ny = a.Ny, NM = a.NZ1 * a.NKX;
-  const int m = blockIdx.x * kStageWarps + wq;
-  if (m >= NM) return;
-  const long long CS = (long long)NM * Ny, mo = (long long)m * Ny;
-  const int iz = m / NKX, ix = m % NKX;
-  const double kx = a.kx[ix], kz = a.kz[iz];
-  const double k2 = kx * kx + kz * kz;
-  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
-  double2 vj[3][YR], ra[3][YR];
-  double c1[YR], c2[YR], e1[YR], e2[YR];
   const unsigned long long drop = l2_drop();
+  {
+    const int q = threadIdx.x & 3, mq = blockIdx.x * kStageWarps + q;
+    if (mq < NM) {
+      const ModeSlot ms = mode_slot(mq, NKX, a.NZ1, paired);
+      const double2* src = R + ms.tile * Ny * kLanes + ms.lane;
+      for (int y = threadIdx.x >> 2; y < Ny; y += 8 * kStageWarps) {
+#pragma unroll
+        for (int cpt = 0; cpt < 3; ++cpt)
+          cp_async16_l2(sm + q * SS + cpt * Ny + y, src + cpt * cs + (long long)y * kLanes, drop);
+      }
+    }
+    cp_async_commit();
+  }
+  const bool act = m < NM;
+  const long long CS = (long long)NM * Ny, mo = (long long)m * Ny;
+  const int iz = m / NKX, ix = m % NKX;
+  double2 vj[3][YR];
+  double c1[YR], c2[YR], e1[YR], e2[YR];
   auto load = [&](int k, int y) {
 #pragma unroll
-    for (int cpt = 0; cpt < 3; ++cpt) {
-      vj[cpt][k] = vel_j[cpt * CS + mo + y];
-      ra[cpt][k] = ld_l2(R + cpt * CS + mo + y, drop);
-    }
+    for (int cpt = 0; cpt < 3; ++cpt) vj[cpt][k] = vel_j[cpt * CS + mo + y];
     c1[k] = a.v1[mo + y];
     c2[k] = a.v2[mo + y];
     e1[k] = a.q1[mo + y];
@@ -301,12 +386,25 @@ imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j
 #pragma unroll
   for (int k = 0; k < YM; ++k) {
     const int y = lane + 32 * k;
-    if (y < Ny) load(k, y);
+    if (act && y < Ny) load(k, y);
   }
+  cp_async_wait_all();
+  __syncthreads();
+  if (!act) return;  // no CTA-wide barrier below
+  const double kx = a.kx[ix], kz = a.kz[iz];
+  const double k2 = kx * kx + kz * kz;
+  const double2 *ra = sm + wq * SS, *va = ra + Ny;
   // Stages 4-5: wall divergence and influence-matrix weights
-  const double2* va = R + CS + mo;
-  double2 dw0 = band_row<S1>(va, a.d1_j0, a.d1_wT, Ny, 0);
-  const double2 dw1 = band_row<S1>(va, a.d1_j0, a.d1_wT, Ny, Ny - 1);
+  double2 dw0 = make_double2(0.0, 0.0), dw1 = dw0;
+#pragma unroll
+  for (int i = 0; i < S1; ++i) {
+    const double b0 = a.d1_w[i], b1 = a.d1_w[(Ny - 1) * S1 + i];
+    const double2 x0 = va[a.d1_j0[0] + i], x1 = va[a.d1_j0[Ny - 1] + i];
+    dw0.x += b0 * x0.x;
+    dw0.y += b0 * x0.y;
+    dw1.x += b1 * x1.x;
+    dw1.y += b1 * x1.y;
+  }
   if (k2 == 0.0) dw0 = make_double2(0.0, 0.0);
   const double* Mi = a.M_inv + (long long)m * 4;
   const double2 a1 = make_double2(-(Mi[0] * dw0.x + Mi[1] * dw1.x),
@@ -315,16 +413,17 @@ imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j
                                   -(Mi[2] * dw0.y + Mi[3] * dw1.y));
   // Stage 6: assemble, store, correction norm
   const double km = (ix == 0 && a.kx0) ? 1.0 : 2.0;
+  const int nk = YM > 0 ? YM : (Ny + 31) / 32;
   double acc = 0.0;
 #pragma unroll
   for (int kk = 0; kk < nk; ++kk) {
     const int y = lane + 32 * kk, k = YM > 0 ? kk : 0;
     if (y >= Ny) continue;
     if (YM == 0) load(0, y);
-    const double2 vnew = cadd(cadd(ra[1][k], cscale(a1, c1[k])), cscale(a2, c2[k]));
+    const double2 vnew = cadd(cadd(va[y], cscale(a1, c1[k])), cscale(a2, c2[k]));
     const double2 qq = cadd(cscale(a1, e1[k]), cscale(a2, e2[k]));
-    const double2 unew = csub(ra[0][k], cik(kx, qq));
-    const double2 wnew = csub(ra[2][k], cik(kz, qq));
+    const double2 unew = csub(ra[y], cik(kx, qq));
+    const double2 wnew = csub(ra[2 * Ny + y], cik(kz, qq));
     const double2 cu = csub(unew, vj[0][k]);
     const double2 cv = csub(vnew, vj[1][k]);
     const double2 cw = csub(wnew, vj[2][k]);
@@ -347,33 +446,38 @@ imm_stage6_kernel(ImmArgs a, const double2* __restrict__ R, const double2* vel_j
 
 // ---------------------------------------------------------------------------
 // Batched banded substitution: one CTA per tile of 16 items, one warp per
-// component (1 for L_k: p_P; 3 for H_k); lane = (side, item) (lanes 0-15 the
-// items' own modes, 16-31 their mirrors), and each thread solves both real
-// columns (re, im) of its mode's component as two recurrences sharing every
-// factor load; the warps share the tile's factor stream.  Lane 0 streams each block of
-// steps' factors (and pivots) for the tile -- one contiguous chunk each --
-// into a ring of shared-memory slots with bulk copies completing on the
-// slot's mbarrier; every thread copies the right-hand-side rows entering its
-// windows during the block into the same slot with cp.async.  Both run
-// ring-1 blocks ahead of the block being computed.
+// component (1 for L_k: p_P; 3 for H_k) and one copying warp; lane = (side,
+// item) (lanes 0-15 the items' own modes, 16-31 their mirrors), and each thread
+// solves both real columns (re, im) of its mode's component as two recurrences
+// sharing every factor load; the warps share the tile's factor stream.  Lane 0
+// of the copying warp streams each block of steps -- its factors and pivots and,
+// per component, the right-hand-side rows that enter the windows during the
+// block, each one contiguous bulk copy -- into a ring of shared-memory slots
+// (`full` barriers, by bytes); the component warps hand a slot back one by one
+// (`empty` barriers), so no warp waits for another but for the data.  Lanes of
+// no mode (padding items, the mirror side of s = 0 or of unpaired items) run on
+// the workspace's zeros.
 //
 // Forward elimination (dgbtrs 'N'): windows b[j..j+KL] in registers,
 // slot(o, ph) = (o + ph) % W, W = KL + 1; the row interchange is chosen per
 // block for the warp: none, with the next row only (two selects), or
 // general (switch).  Back substitution: windows b[j-NU..j], slot(o, ph) =
-// (o - ph) mod WB, WB = NU + 1, one FMA deep per step (U pre-scaled).
-// A ring wait that does not complete within its bound sets bit 2 of the
-// status word and the CTA stops computing.
+// (o - ph) mod WB, WB = NU + 1, one FMA deep per step (U pre-scaled).  Its rows
+// are the forward results, read back by bulk copies: every lane fences its
+// stores towards the copies' proxy before the copying warp is told.
+// A wait that does not complete within its bound sets bit 2 of the status word
+// and the CTA stops computing.
 // ---------------------------------------------------------------------------
 
 struct SolveArgs {
   const double* facL;
   const double* facU;
   const unsigned char* dp;
-  double2* X;  // [ncomp][NM][Ny]
+  double2* X;    // [ncomp][tiles][Ny][32]
+  long long cs;  // component stride of X
   int* status;
-  int NP, NM, Ny, NKX, NZ1, paired, ring, slot_bytes;
-  int wait_limit;  // polls before a ring wait gives up (the drain after it uses kDrainPolls)
+  int Ny, ncomp, ring, slot_bytes;
+  int wait_limit;  // polls before a wait gives up (the drain after it uses kDrainPolls)
   const int* skip;  // non-null and *skip != 0: return at once (ImmArgs::skip)
 };
 
@@ -386,6 +490,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 }
 __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_tx(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)),
@@ -419,19 +526,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   return false;
 }
 
-// Mode of item p on side q and whether its columns are solved.
-__device__ __forceinline__ bool item_mode(const SolveArgs& a, int p, int q, int* m) {
-  bool live = p < a.NP;
-  int mm = min(p, a.NP - 1);
-  if (q == 1) {
-    const int s = mm / a.NKX, ix = mm % a.NKX;
-    live = live && a.paired && s != 0;
-    if (live) mm = (a.NZ1 - s) * a.NKX + ix;
-  }
-  *m = mm;
-  return live;
-}
-
 // Row interchange of step ph (pivot offset d) on one window.
 template <int KL, int MODE>
 __device__ __forceinline__ double pivot_take(double (&w)[KL + 1], int ph, int d) {
@@ -460,11 +554,10 @@ __device__ __forceinline__ double pivot_take(double (&w)[KL + 1], int ph, int d)
   return bpj;
 }
 
-template <int KL, int NCP, int MW, int MODE, bool TAIL>
-__device__ __forceinline__ void tile_fwd_block(double2* const (&col)[NCP], int j0, int nsteps,
-                                               int Ny, bool live, double (&w)[2 * NCP][KL + 1],
-                                               const double2* Lp, const int (&dr)[KL + 1],
-                                               const double2* ent, int ES,
+template <int KL, int MODE, bool TAIL>
+__device__ __forceinline__ void tile_fwd_block(double2* col, int j0, int nsteps, int Ny,
+                                               double (&w)[2][KL + 1], const double2* Lp,
+                                               const int (&dr)[KL + 1], const double2* ent,
                                                unsigned long long pol) {
   constexpr int W = KL + 1;
 #pragma unroll
@@ -478,35 +571,26 @@ __device__ __forceinline__ void tile_fwd_block(double2* const (&col)[NCP], int j
         L[2 * i2] = t.x;
         L[2 * i2 + 1] = t.y;
       }
-      double bp[2 * NCP];
+      double bp[2];
 #pragma unroll
-      for (int c = 0; c < 2 * NCP; ++c) bp[c] = pivot_take<KL, MODE>(w[c], ph, dr[ph]);
-      if (live) {
+      for (int c = 0; c < 2; ++c) bp[c] = pivot_take<KL, MODE>(w[c], ph, dr[ph]);
+      st_l2(col + j * kLanes, make_double2(bp[0], bp[1]), pol);
 #pragma unroll
-        for (int cc = 0; cc < NCP; ++cc)
-          st_l2(col[cc] + j, make_double2(bp[2 * cc], bp[2 * cc + 1]), pol);
-      }
-#pragma unroll
-      for (int c = 0; c < 2 * NCP; ++c) {
+      for (int c = 0; c < 2; ++c) {
 #pragma unroll
         for (int i = 1; i <= KL; ++i) w[c][(i + ph) % W] -= L[i - 1] * bp[c];
       }
       // b[j+W] enters at offset KL (0 past the last row)
-      const bool in = j + W < Ny;
-#pragma unroll
-      for (int cc = 0; cc < NCP; ++cc) {
-        const double2 e = in ? ent[(cc * MW + ph) * ES] : make_double2(0.0, 0.0);
-        w[2 * cc][ph % W] = e.x;
-        w[2 * cc + 1][ph % W] = e.y;
-      }
+      const double2 e = j + W < Ny ? ent[ph * kLanes] : make_double2(0.0, 0.0);
+      w[0][ph % W] = e.x;
+      w[1][ph % W] = e.y;
     }
   }
 }
 
-template <int NU, int NCP, int MW, bool TAIL>
-__device__ __forceinline__ void tile_bwd_block(double2* const (&col)[NCP], int j0, bool live,
-                                               double (&w)[2 * NCP][NU + 1], const double2* Up,
-                                               const double2* ent, int ES,
+template <int NU, bool TAIL>
+__device__ __forceinline__ void tile_bwd_block(double2* col, int j0, double (&w)[2][NU + 1],
+                                               const double2* Up, const double2* ent,
                                                unsigned long long pol) {
   constexpr int WB = NU + 1, NUP = (NU + 2) & ~1;
 #pragma unroll
@@ -522,140 +606,134 @@ __device__ __forceinline__ void tile_bwd_block(double2* const (&col)[NCP], int j
         U[2 * i2 + 1] = t.y;
       }
       const int st = ((NU - ph) % WB + WB) % WB;
-      double bj[2 * NCP];
-#pragma unroll
-      for (int c = 0; c < 2 * NCP; ++c) bj[c] = w[c][st];
-      if (live) {
-#pragma unroll
-        for (int cc = 0; cc < NCP; ++cc)
-          st_l2(col[cc] + j, make_double2(bj[2 * cc] * U[0], bj[2 * cc + 1] * U[0]), pol);
-      }
+      const double bj[2] = {w[0][st], w[1][st]};
+      st_l2(col + j * kLanes, make_double2(bj[0] * U[0], bj[1] * U[0]), pol);
 #pragma unroll
       for (int i = 1; i <= NU; ++i) {
         const int si = ((NU - i - ph) % WB + WB) % WB;
 #pragma unroll
-        for (int c = 0; c < 2 * NCP; ++c) w[c][si] -= U[i] * bj[c];
+        for (int c = 0; c < 2; ++c) w[c][si] -= U[i] * bj[c];
       }
-      // b[j-WB] enters at offset 0 (0 below row 0)
-      const bool in = j - WB >= 0;
-#pragma unroll
-      for (int cc = 0; cc < NCP; ++cc) {
-        const double2 e = in ? ent[(cc * MW + ph) * ES] : make_double2(0.0, 0.0);
-        w[2 * cc][st] = e.x;
-        w[2 * cc + 1][st] = e.y;
-      }
+      // b[j-WB] enters at offset 0 (0 below row 0); rows in ascending order
+      const double2 e = j - WB >= 0 ? ent[(WB - 1 - ph) * kLanes] : make_double2(0.0, 0.0);
+      w[0][st] = e.x;
+      w[1][st] = e.y;
     }
   }
 }
 
+constexpr int kMaxRing = 4;
+
 template <int KL, int NU>
-__global__ void __launch_bounds__(96)
+__global__ void __launch_bounds__(128)
 imm_solve_kernel(SolveArgs a) {
   if (a.skip && *a.skip) return;  // before any barrier is set up
-  constexpr int NCP = 1;  // components per thread (one warp per component)
   constexpr int W = KL + 1, WB = NU + 1, NUP = (NU + 2) & ~1;
   constexpr int LB = W * KL * kTile * 8, PB = W * kTile, UB = WB * NUP * kTile * 8;
-  constexpr int MW = W > WB ? W : WB;  // rows per (component, lane) in a slot
+  constexpr int MW = W > WB ? W : WB;  // entering rows of a component in a slot
+  constexpr int RB = kLanes * 16;      // bytes of a tile row
   extern __shared__ __align__(128) unsigned char ring[];
-  __shared__ __align__(8) unsigned long long bars[3];
+  __shared__ __align__(8) unsigned long long full[kMaxRing], empty[kMaxRing], fwd_done;
   __shared__ int s_fail;
   const int tid = threadIdx.x, lane = tid & 31, cw = tid >> 5;  // warp = component
-  const int side = lane >> 4, it = lane & (kTile - 1);
-  const int tile = blockIdx.x;
-  const int Ny = a.Ny, R = a.ring, SB = a.slot_bytes, nthr = blockDim.x;
-  const int EB = MW * nthr * 16;  // entering rows of every thread, at the slot's end
+  const int it = lane & (kTile - 1);
+  const long long tile = blockIdx.x;
+  const int Ny = a.Ny, R = a.ring, SB = a.slot_bytes, nc = a.ncomp;
+  const int E0 = SB - nc * MW * RB;  // entering rows, at the slot's end
   const long long NyF = Ny + W, NyB = Ny + WB;
-  int m;
-  const bool live = item_mode(a, tile * kTile + it, side, &m);
-  const unsigned long long keep = l2_keep();
-  double2* col[NCP];
-#pragma unroll
-  for (int cc = 0; cc < NCP; ++cc) col[cc] = a.X + ((long long)(cw + cc) * a.NM + m) * Ny;
   const int nsteps = Ny - 1;
   const int nbf = (nsteps + W - 1) / W;  // forward blocks
   const int nbb = (Ny + WB - 1) / WB;    // back-substitution blocks
   const int nblk = nbf + nbb;
+  double2* X = a.X + tile * Ny * kLanes;
 
   if (tid == 0) {
-    for (int r = 0; r < R; ++r) mbar_init(&bars[r], 1);
+    for (int r = 0; r < R; ++r) {
+      mbar_init(&full[r], 1);
+      mbar_init(&empty[r], nc);
+    }
+    mbar_init(&fwd_done, nc);
     mbar_fence_init();
     s_fail = 0;
   }
   __syncthreads();
-  // Block g of the combined sequence into slot g % R: factors by lane 0
-  // (bulk, mbarrier), this lane's entering rows by every lane (cp.async
-  // group g).  Entering rows of component cc at ent[(cc * MW + ph) * 32 +
-  // lane]: forward row j0+W+ph, back substitution row j0-WB-ph.
-  int hi_issued = -1;
-  auto issue = [&](int g) {
-    if (g < nblk) {
-      hi_issued = g;
+  volatile int* fail = &s_fail;
+
+  if (cw == nc) {
+    if (lane != 0) return;
+    // Blocks 0 .. nblk-1 into slot g % R: forward blocks hold the factors and
+    // pivots of steps j0 .. j0+W-1 and rows j0+W .. j0+2W-1; back-substitution
+    // blocks U records j0-WB+1 .. j0 and rows j0-2WB+1 .. j0-WB, those that
+    // exist.
+    int g = 0;
+    bool ok = true;
+    for (; g < nblk; ++g) {
+      if (g >= R) ok = mbar_wait(&empty[g % R], (g / R - 1) & 1, a.wait_limit);
+      if (ok && g == nbf) ok = mbar_wait(&fwd_done, 0, a.wait_limit);
+      if (!ok || *fail) break;
       unsigned char* slot = ring + (g % R) * SB;
-      unsigned long long* bar = &bars[g % R];
-      double2* ent = reinterpret_cast<double2*>(slot + SB - EB) + tid;
-      if (g < nbf) {
-        const int j0 = g * W;
-        if (tid == 0) {
-          mbar_arrive_tx(bar, LB + PB);
-          bulk_g2s(slot, a.facL + (tile * NyF + j0) * KL * kTile, LB, bar);
-          bulk_g2s(slot + LB, a.dp + (tile * NyF + j0) * kTile, PB, bar);
-        }
-        if (live) {
-#pragma unroll
-          for (int ph = 0; ph < W; ++ph) {
-            const int e = j0 + W + ph;
-            if (e < Ny)
-              for (int cc = 0; cc < NCP; ++cc) cp_async16_l2(ent + (cc * MW + ph) * nthr, col[cc] + e, keep);
-          }
-        }
+      unsigned long long* bar = &full[g % R];
+      const bool fwd = g < nbf;
+      const int j0 = fwd ? g * W : Ny - 1 - (g - nbf) * WB;
+      const int first = fwd ? j0 + W : j0 - 2 * WB + 1;  // row of the slot's first entry
+      const int lo = max(first, 0), hi = min(fwd ? j0 + 2 * W : j0 - WB + 1, Ny);
+      const int rows = max(hi - lo, 0);
+      mbar_arrive_tx(bar, (fwd ? LB + PB : UB) + rows * RB * nc);
+      if (fwd) {
+        bulk_g2s(slot, a.facL + (tile * NyF + j0) * KL * kTile, LB, bar);
+        bulk_g2s(slot + LB, a.dp + (tile * NyF + j0) * kTile, PB, bar);
       } else {
-        const int j0 = Ny - 1 - (g - nbf) * WB;
-        if (tid == 0) {
-          mbar_arrive_tx(bar, UB);
-          bulk_g2s(slot, a.facU + (tile * NyB + j0 + 1) * NUP * kTile, UB, bar);
-        }
-        if (live) {
-#pragma unroll
-          for (int ph = 0; ph < WB; ++ph) {
-            const int e = j0 - WB - ph;
-            if (e >= 0)
-              for (int cc = 0; cc < NCP; ++cc) cp_async16_l2(ent + (cc * MW + ph) * nthr, col[cc] + e, keep);
-          }
-        }
+        bulk_g2s(slot, a.facU + (tile * NyB + j0 + 1) * NUP * kTile, UB, bar);
       }
+      if (rows > 0)
+        for (int c = 0; c < nc; ++c)
+          bulk_g2s(slot + E0 + (c * MW + lo - first) * RB, X + c * a.cs + (long long)lo * kLanes,
+                   rows * RB, bar);
     }
-    cp_async_commit();
-  };
-  auto wait_block = [&](int g) {
-    if (R == 3) cp_async_wait_2(); else cp_async_wait_1();  // this lane's rows of block g
-    if (!mbar_wait(&bars[g % R], (g / R) & 1, a.wait_limit)) s_fail = 1;
-    __syncthreads();
-  };
-  // The back substitution reads the forward results: its blocks are issued
-  // only after every forward result is stored.
-  for (int h = 0; h < R - 1; ++h) issue(h < nbf ? h : nblk);
+    if (!ok) {
+      *fail = 1;
+      atomicOr(a.status, 2);
+    }
+    // Leave no bulk copy in flight, whether the other warps take them or gave
+    // up: wait for the blocks issued last (a slot's earlier blocks were taken
+    // before it was filled again).
+    for (int h = max(g - R, 0); h < g; ++h) mbar_wait(&full[h % R], (h / R) & 1, kDrainPolls);
+    return;
+  }
+
+  const unsigned long long keep = l2_keep();
+  double2* col = X + cw * a.cs + lane;
   int g = 0;
   bool ok = true;
+  auto take = [&] {  // wait for block g
+    ok = mbar_wait(&full[g % R], (g / R) & 1, a.wait_limit) && !*fail;
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok && lane == 0) {
+      *fail = 1;
+      atomicOr(a.status, 2);
+    }
+    return ok;
+  };
+  auto give = [&] {  // block g's slot back
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[g % R]);
+  };
 
   // ---- forward elimination, steps j = 0 .. Ny-2 ----
   {
-    double w[2 * NCP][W];
+    double w[2][W];
 #pragma unroll
-    for (int cc = 0; cc < NCP; ++cc) {
-#pragma unroll
-      for (int o = 0; o < W; ++o) {
-        const double2 v = (o < Ny) ? ld_l2(col[cc] + o, keep) : make_double2(0.0, 0.0);
-        w[2 * cc][o] = v.x;
-        w[2 * cc + 1][o] = v.y;
-      }
+    for (int o = 0; o < W; ++o) {
+      const double2 v = (o < Ny) ? ld_l2(col + o * kLanes, keep) : make_double2(0.0, 0.0);
+      w[0][o] = v.x;
+      w[1][o] = v.y;
     }
     for (int k = 0; k < nbf; ++k, ++g) {
-      issue(g + R - 1 < nbf ? g + R - 1 : nblk);
-      wait_block(g);
+      if (!take()) break;
       const unsigned char* slot = ring + (g % R) * SB;
       const double2* Lp = reinterpret_cast<const double2*>(slot) + it;
       const unsigned char* Ps = slot + LB;
-      const double2* ent = reinterpret_cast<const double2*>(slot + SB - EB) + tid;
+      const double2* ent = reinterpret_cast<const double2*>(slot + E0 + cw * MW * RB) + lane;
       int dr[W];
       int dm = 0;
 #pragma unroll
@@ -666,73 +744,55 @@ imm_solve_kernel(SolveArgs a) {
       dm = __reduce_max_sync(0xffffffffu, dm);
       const int j0 = k * W;
       if (j0 + W > nsteps)
-        tile_fwd_block<KL, NCP, MW, 2, true>(col, j0, nsteps, Ny, live, w, Lp, dr, ent, nthr, keep);
+        tile_fwd_block<KL, 2, true>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else if (dm == 0)
-        tile_fwd_block<KL, NCP, MW, 0, false>(col, j0, nsteps, Ny, live, w, Lp, dr, ent, nthr, keep);
+        tile_fwd_block<KL, 0, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else if (dm == 1)
-        tile_fwd_block<KL, NCP, MW, 1, false>(col, j0, nsteps, Ny, live, w, Lp, dr, ent, nthr, keep);
+        tile_fwd_block<KL, 1, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else
-        tile_fwd_block<KL, NCP, MW, 2, false>(col, j0, nsteps, Ny, live, w, Lp, dr, ent, nthr, keep);
-      __syncthreads();  // the slot is refilled by the next issue
-      if (s_fail) {
-        ok = false;
-        break;
-      }
+        tile_fwd_block<KL, 2, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
+      give();
     }
     // b[Ny-1] sits at offset 0 after the last step: slot nsteps % W.
     const int last = nsteps % W;
+    double v0 = w[0][0], v1 = w[1][0];
 #pragma unroll
-    for (int cc = 0; cc < NCP; ++cc) {
-      double v0 = w[2 * cc][0], v1 = w[2 * cc + 1][0];
-#pragma unroll
-      for (int s = 1; s < W; ++s)
-        if (last == s) {
-          v0 = w[2 * cc][s];
-          v1 = w[2 * cc + 1][s];
-        }
-      if (live && ok) st_l2(col[cc] + Ny - 1, make_double2(v0, v1), keep);
+    for (int s = 1; s < W; ++s)
+      if (last == s) {
+        v0 = w[0][s];
+        v1 = w[1][s];
+      }
+    if (ok) {
+      st_l2(col + (Ny - 1) * kLanes, make_double2(v0, v1), keep);
+      // the forward results are read back by bulk copies (async proxy)
+      asm volatile("fence.proxy.async;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&fwd_done);
     }
   }
 
-  // ---- back substitution, rows j = Ny-1 .. 0 (this lane's own forward
-  // results, read back in program order) ----
+  // ---- back substitution, rows j = Ny-1 .. 0 ----
   if (ok) {
-    for (int h = nbf; h < nbf + R - 1; ++h) issue(h);
-    double w[2 * NCP][WB];
+    double w[2][WB];
 #pragma unroll
-    for (int cc = 0; cc < NCP; ++cc) {
-#pragma unroll
-      for (int o = 0; o < WB; ++o) {
-        const int idx = Ny - 1 - NU + o;
-        const double2 v = (idx >= 0) ? ld_l2(col[cc] + idx, keep) : make_double2(0.0, 0.0);
-        w[2 * cc][o] = v.x;
-        w[2 * cc + 1][o] = v.y;
-      }
+    for (int o = 0; o < WB; ++o) {
+      const int idx = Ny - 1 - NU + o;
+      const double2 v = (idx >= 0) ? ld_l2(col + idx * kLanes, keep) : make_double2(0.0, 0.0);
+      w[0][o] = v.x;
+      w[1][o] = v.y;
     }
     for (int k = 0; k < nbb; ++k, ++g) {
-      issue(g + R - 1);
-      wait_block(g);
+      if (!take()) break;
       const unsigned char* slot = ring + (g % R) * SB;
       const double2* Up = reinterpret_cast<const double2*>(slot) + it;
-      const double2* ent = reinterpret_cast<const double2*>(slot + SB - EB) + tid;
+      const double2* ent = reinterpret_cast<const double2*>(slot + E0 + cw * MW * RB) + lane;
       const int j0 = Ny - 1 - k * WB;
       if (j0 - WB + 1 < 0)
-        tile_bwd_block<NU, NCP, MW, true>(col, j0, live, w, Up, ent, nthr, keep);
+        tile_bwd_block<NU, true>(col, j0, w, Up, ent, keep);
       else
-        tile_bwd_block<NU, NCP, MW, false>(col, j0, live, w, Up, ent, nthr, keep);
-      __syncthreads();
-      if (s_fail) {
-        ok = false;
-        break;
-      }
+        tile_bwd_block<NU, false>(col, j0, w, Up, ent, keep);
+      give();
     }
-  }
-  cp_async_wait_all();
-  if (!ok && tid == 0) {
-    // Leave no bulk copy in flight: blocks g .. hi_issued were issued
-    // (block g is the one that timed out).
-    for (int h = g; h <= hi_issued; ++h) mbar_wait(&bars[h % R], (h / R) & 1, kDrainPolls);
-    atomicOr(a.status, 2);
   }
 }
 
@@ -740,26 +800,67 @@ imm_solve_kernel(SolveArgs a) {
 // Host side.
 // ---------------------------------------------------------------------------
 size_t imm_batch_stage_smem(int Ny) {
-  return sizeof(double2) * (size_t)(6 * Ny * kStageWarps);
+  return sizeof(double2) * (size_t)(stage_stride(Ny) * kStageWarps);
 }
 
-static size_t imm_batch_grad_smem(int Ny) {
-  return sizeof(double2) * (size_t)(Ny * kStageWarps);
+static size_t imm_batch_assemble_smem(int Ny) {
+  return sizeof(double2) * (size_t)(assemble_stride(Ny) * kStageWarps);
+}
+
+// Rows per lane of the stage kernel (odd): 32 lanes cover Ny rows.
+constexpr int kMaxNy = 512;  // four modes' rows fit in shared memory
+int imm_batch_rows(int Ny) {
+  return Ny <= 96 ? 3 : Ny <= 160 ? 5 : Ny <= 224 ? 7 : Ny <= 288 ? 9 : 17;
 }
 
 bool imm_batch_supported(int kl, int ny) {
   return (kl == 2 || kl == 4 || kl == 6 || kl == 8) && ny <= kMaxNy;
 }
 
+// Window-relative stencil weights of the stage kernel: lane l's window of
+// W = (p + 2) + YM - 1 rows starts at base[l], and w1x / w2x[(o W + i) 32 + l] is
+// the weight of window row i in D1 / D2 of row YM l + o (0 outside the stencil
+// and past the last row).
+void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const int* j02,
+                       const double* w2, std::vector<int>* base, std::vector<double>* w1x,
+                       std::vector<double>* w2x) {
+  const int YM = imm_batch_rows(Ny), S1 = p + 1, S2 = p + 2, W = S2 + YM - 1;
+  base->assign(32, 0);
+  w1x->assign((size_t)YM * W * 32, 0.0);
+  w2x->assign((size_t)YM * W * 32, 0.0);
+  for (int l = 0; l < 32; ++l) {
+    const int b = std::max(0, std::min(YM * l - S2 / 2, Ny - W));
+    (*base)[l] = b;
+    for (int o = 0; o < YM && YM * l + o < Ny; ++o) {
+      const int y = YM * l + o;
+      for (int m = 0; m < S1; ++m)
+        (*w1x)[(size_t)(o * W + j01[y] + m - b) * 32 + l] = w1[y * S1 + m];
+      for (int m = 0; m < S2; ++m)
+        (*w2x)[(size_t)(o * W + j02[y] + m - b) * 32 + l] = w2[y * S2 + m];
+    }
+  }
+}
+
+// Every stencil of a lane's rows lies in its window (true for stencils centred
+// in the interior and shifted to stay inside the walls).
+bool imm_batch_windows_ok(int Ny, int p, const int* j01, const int* j02) {
+  const int YM = imm_batch_rows(Ny), S1 = p + 1, S2 = p + 2, W = S2 + YM - 1;
+  for (int y = 0; y < Ny; ++y) {
+    const int b = std::max(0, std::min((y / YM) * YM - S2 / 2, Ny - W));
+    if (j01[y] < b || j02[y] < b || j01[y] + S1 > b + W || j02[y] + S2 > b + W) return false;
+  }
+  return true;
+}
+
 // Ring slot bytes of one substitution launch: the larger of a forward block
 // (factors, pivots) and a back-substitution block (U records), plus the
-// entering rows of every lane; and the ring depth that fits.
+// entering rows of every component; and the ring depth that fits.
 static int solve_slot_bytes(int kl, int nu, int ncomp) {
   const int W = kl + 1, WB = nu + 1, nup = (nu + 2) & ~1;
   const int MW = W > WB ? W : WB;
   const int f = W * kl * kTile * 8 + W * kTile;
   const int b = WB * nup * kTile * 8;
-  return (((f > b ? f : b) + 127) & ~127) + ncomp * MW * 32 * 16;
+  return (((f > b ? f : b) + 127) & ~127) + ncomp * MW * kLanes * 16;
 }
 
 static int solve_ring(int kl, int nu, int ncomp, int max_smem) {
@@ -774,21 +875,18 @@ bool imm_batch_fits(int kl, int nu, int max_smem) {
 }
 
 template <int KL>
-static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, int ncomp, int NM,
-                                int Ny, int NKX, int NZ1, const int* skip, cudaStream_t st) {
+static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, long long cs, int ncomp,
+                                int Ny, const int* skip, cudaStream_t st) {
   SolveArgs s{};
   s.skip = skip;
   s.facL = bt.facL[op];
   s.facU = bt.facU[op];
   s.dp = bt.dp[op];
   s.X = X;
+  s.cs = cs;
   s.status = bt.status;
-  s.NP = bt.NP;
-  s.NM = NM;
   s.Ny = Ny;
-  s.NKX = NKX;
-  s.NZ1 = NZ1;
-  s.paired = bt.paired;
+  s.ncomp = ncomp;
   s.ring = solve_ring(KL, bt.nu, ncomp, bt.max_smem);
   s.slot_bytes = solve_slot_bytes(KL, bt.nu, ncomp);
   s.wait_limit = bt.wait_limit;
@@ -796,31 +894,50 @@ static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, int ncom
   const size_t sm = (size_t)s.ring * s.slot_bytes;
   const int grid = (bt.NP + kTile - 1) / kTile;
   if (bt.nu == KL + 1)
-    imm_solve_kernel<KL, KL + 1><<<grid, 32 * ncomp, sm, st>>>(s);
+    imm_solve_kernel<KL, KL + 1><<<grid, 32 * (ncomp + 1), sm, st>>>(s);
   else
-    imm_solve_kernel<KL, 2 * KL><<<grid, 32 * ncomp, sm, st>>>(s);
+    imm_solve_kernel<KL, 2 * KL><<<grid, 32 * (ncomp + 1), sm, st>>>(s);
   return cudaGetLastError();
 }
 
-template <int K, int YM>
+template <int K>
 static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2* vel_n,
                            const double2* vel_j, const double2* nl_n, const double2* nl_j,
                            double2* vel_new, double2* corr_out, double* partials,
                            cudaStream_t st) {
   const int NM = a.NZ1 * a.NKX, Ny = a.Ny;
-  const int grid = (NM + kStageWarps - 1) / kStageWarps;
-  const size_t sm = imm_batch_stage_smem(Ny);
+  const int grid = (NM + kStageWarps - 1) / kStageWarps, threads = 32 * kStageWarps;
+  const int tiles = (bt.NP + kTile - 1) / kTile;
+  const long long cs = (long long)tiles * Ny * kLanes;
+  const size_t sm = imm_batch_stage_smem(Ny), sm6 = imm_batch_assemble_smem(Ny);
   cudaError_t e;
-  imm_stage013_kernel<K, YM><<<grid, 32 * kStageWarps, sm, st>>>(a, vel_n, nl_n, nl_j, bt.F, bt.R);
+#define DNSB_STAGE013(YM)                                                                   \
+  case YM:                                                                                  \
+    imm_stage013_kernel<K, YM><<<grid, threads, sm, st>>>(a, bt.paired, bt.w1x, bt.w2x,     \
+                                                          bt.base, vel_n, nl_n, nl_j, bt.F, \
+                                                          bt.R, cs);                        \
+    break;
+  switch (imm_batch_rows(Ny)) {
+    DNSB_STAGE013(3) DNSB_STAGE013(5) DNSB_STAGE013(7) DNSB_STAGE013(9) DNSB_STAGE013(17)
+  }
+#undef DNSB_STAGE013
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  e = solve_launch<K>(bt, 0, bt.F, 1, NM, Ny, a.NKX, a.NZ1, a.skip, st);
+  e = solve_launch<K>(bt, 0, bt.F, 0, 1, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
-  imm_grad_kernel<K, YM><<<grid, 32 * kStageWarps, imm_batch_grad_smem(Ny), st>>>(a, bt.F, bt.R);
+  const dim3 gg((Ny - 2 + kGradRows - 1) / kGradRows, tiles);
+  imm_grad_kernel<K><<<gg, kLanes * kGradRows, 0, st>>>(a, bt.paired, bt.NP, bt.F, bt.R, cs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  e = solve_launch<K>(bt, 1, bt.R, 3, NM, Ny, a.NKX, a.NZ1, a.skip, st);
+  e = solve_launch<K>(bt, 1, bt.R, cs, 3, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
-  imm_stage6_kernel<K, YM><<<grid, 32 * kStageWarps, 0, st>>>(a, bt.R, vel_j, vel_new, corr_out,
-                                                          partials);
+  if (Ny <= 96)
+    imm_stage6_kernel<K, 3><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
+                                                        corr_out, partials);
+  else if (Ny <= 160)
+    imm_stage6_kernel<K, 5><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
+                                                        corr_out, partials);
+  else
+    imm_stage6_kernel<K, 0><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
+                                                        corr_out, partials);
   return cudaGetLastError();
 }
 
@@ -829,30 +946,25 @@ cudaError_t launch_imm_batch(const ImmArgs& a, const ImmBatch& bt, const double2
                              const double2* vel_j, const double2* nl_n,
                              const double2* nl_j, double2* vel_new, double2* corr_out,
                              double* partials, cudaStream_t st) {
-  const bool regs = a.Ny <= 32 * kSYM;
   switch (a.kl) {
-#define DNSB_PIPE(K)                                                                          \
-  case K:                                                                                     \
-    return regs ? pipeline<K, kSYM>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out,       \
-                                    partials, st)                                             \
-                : pipeline<K, 0>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
-    DNSB_PIPE(2) DNSB_PIPE(4) DNSB_PIPE(6) DNSB_PIPE(8)
-#undef DNSB_PIPE
+    case 2: return pipeline<2>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
+    case 4: return pipeline<4>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
+    case 6: return pipeline<6>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
+    case 8: return pipeline<8>(a, bt, vel_n, vel_j, nl_n, nl_j, vel_new, corr_out, partials, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t set_imm_batch_attributes(int max_smem) {
   const void* fns[] = {
-#define DNSB_STAGE_FNS(K)                                                        \
-  (const void*)imm_stage013_kernel<K, kSYM>, (const void*)imm_stage013_kernel<K, 0>, \
-      (const void*)imm_grad_kernel<K, kSYM>, (const void*)imm_grad_kernel<K, 0>
-      DNSB_STAGE_FNS(2), DNSB_STAGE_FNS(4), DNSB_STAGE_FNS(6), DNSB_STAGE_FNS(8),
-#undef DNSB_STAGE_FNS
-#define DNSB_SOLVE_FNS(K) \
-  (const void*)imm_solve_kernel<K, K + 1>, (const void*)imm_solve_kernel<K, 2 * K>
-      DNSB_SOLVE_FNS(2), DNSB_SOLVE_FNS(4), DNSB_SOLVE_FNS(6), DNSB_SOLVE_FNS(8)};
-#undef DNSB_SOLVE_FNS
+#define DNSB_IMM_FNS(K)                                                              \
+  (const void*)imm_stage013_kernel<K, 3>, (const void*)imm_stage013_kernel<K, 5>,    \
+      (const void*)imm_stage013_kernel<K, 7>, (const void*)imm_stage013_kernel<K, 9>, \
+      (const void*)imm_stage013_kernel<K, 17>,                                       \
+      (const void*)imm_stage6_kernel<K, 0>, (const void*)imm_solve_kernel<K, K + 1>, \
+      (const void*)imm_solve_kernel<K, 2 * K>
+      DNSB_IMM_FNS(2), DNSB_IMM_FNS(4), DNSB_IMM_FNS(6), DNSB_IMM_FNS(8)};
+#undef DNSB_IMM_FNS
   cudaError_t e = cudaSuccess;
   for (const void* f : fns) {
     cudaError_t r = allow_dynamic_smem(f, max_smem);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <string>
+#include <vector>
 
 #include "common.cuh"
 
@@ -139,9 +140,9 @@ cudaError_t launch_ab_pair_check(const double* ab, const int* piv, int nz1,
 
 // Five-kernel IMM iteration (csrc/imm_batch.cu) over factors repacked at
 // bind time (record-major, item index fastest; 1/U_jj and U/U_jj pre-scaled;
-// pivots as validated offsets) and workspace F [NM][Ny], R [3][NM][Ny].
+// pivots as validated offsets) and workspace F [tiles][Ny][32], R [3][tiles][Ny][32].
 struct ImmBatch {
-  // per operator (0 = L_k, 1 = H_k), 32-item tiles (csrc/imm_batch.cu)
+  // per operator (0 = L_k, 1 = H_k), 16-item tiles (csrc/imm_batch.cu)
   const double* facL[2];
   const double* facU[2];
   const unsigned char* dp[2];
@@ -153,6 +154,10 @@ struct ImmBatch {
   int wait_limit;  // polls of a ring slot's mbarrier before the wait gives up
   double2* F;
   double2* R;
+  // window-relative D1 / D2 weights of the stage kernel (imm_batch_windows)
+  const double* w1x;
+  const double* w2x;
+  const int* base;
 };
 // Influence-matrix precompute (csrc/precompute.cu); every pointer is device
 // memory, D1 / D2 dense (ny, ny) row-major, outputs in the reference's
@@ -206,6 +211,10 @@ cudaError_t launch_mlp_adam(float* w, float* m, float* v, const float* grad, voi
                             cudaStream_t st);
 bool imm_batch_supported(int kl, int ny);
 size_t imm_batch_stage_smem(int Ny);
+bool imm_batch_windows_ok(int Ny, int p, const int* j01, const int* j02);
+void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const int* j02,
+                       const double* w2, std::vector<int>* base, std::vector<double>* w1x,
+                       std::vector<double>* w2x);
 int imm_nu(int kl, int row0);
 bool imm_batch_fits(int kl, int nu, int max_smem);
 cudaError_t launch_imm_repack(const double* ab, const int* piv, int Ny, int kl, int nu,
