@@ -1179,19 +1179,25 @@ extern "C" int dnsb_periodic_spec_to_phys(dnsb_periodic* p, const void* spec,
                                           double* phys, void* stream) {
   if (!p || !spec || !phys) return fail(DNSB_ERR_ARG, "null argument");
   cudaStream_t st = as_stream(stream);
-  YInvArgs yi{};
-  yi.u = (const double2*)spec;
-  yi.out = p->A;
-  yi.NY1 = p->NY1;
-  yi.NZ1 = p->NZ1;
-  yi.NKX = p->NKX;
-  yi.curl = 0;
-  yi.kx = p->kx;
-  yi.ky = p->ky;
-  yi.kz = p->kz;
-  yi.plan = p->py;
-  yi.tw = p->twy;
-  DNSB_LAUNCH(launch_yinv(yi, st));
+  if (two_stage_length(p->My)) {
+    ColPassArgs yc = periodic_ycurl(p, spec);
+    yc.curl = 0;
+    DNSB_LAUNCH(launch_col_pass(yc, 3, p->NZ1, st));
+  } else {
+    YInvArgs yi{};
+    yi.u = (const double2*)spec;
+    yi.out = p->A;
+    yi.NY1 = p->NY1;
+    yi.NZ1 = p->NZ1;
+    yi.NKX = p->NKX;
+    yi.curl = 0;
+    yi.kx = p->kx;
+    yi.ky = p->ky;
+    yi.kz = p->kz;
+    yi.plan = p->py;
+    yi.tw = p->twy;
+    DNSB_LAUNCH(launch_yinv(yi, st));
+  }
   DNSB_LAUNCH(launch_col_pass(periodic_zinv(p), 3, p->My, st));
   XPhysArgs xa{};
   xa.in = p->B;
@@ -1233,6 +1239,10 @@ extern "C" int dnsb_periodic_phys_to_spec(dnsb_periodic* p, const double* phys,
   xa.tw = p->twx;
   DNSB_LAUNCH(launch_x_fwd(xa, phys, p->B, st));
   DNSB_LAUNCH(launch_col_pass(periodic_zfwd(p), 3, p->My, st));
+  if (two_stage_length(p->My)) {
+    DNSB_LAUNCH(launch_col_pass(periodic_yfwd_col(p, spec), 3, p->NZ1, st));
+    return 0;
+  }
   YFwdArgs yf{};
   yf.in = p->A;
   yf.out = (double2*)spec;

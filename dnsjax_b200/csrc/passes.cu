@@ -687,6 +687,7 @@ x_phys_kernel(XPhysArgs a) {
 }
 
 cudaError_t launch_x_phys(const XPhysArgs& a, cudaStream_t st) {
+  if (two_stage_length(a.plan.L) && 3 * a.nkx == a.plan.L) return launch_x_phys2(a, st);
   dim3 grid((a.nrows + kXRows - 1) / kXRows);
   DNSB_DISPATCH(a.plan.L, x_phys_kernel, grid, x_phys_smem(a.plan.L), st, a);
   return cudaGetLastError();
@@ -760,6 +761,7 @@ size_t x_fwd_smem(int Mx) {
 
 cudaError_t launch_x_fwd(const XPhysArgs& a, const double* phys, double2* spec,
                          cudaStream_t st) {
+  if (two_stage_length(a.plan.L) && 3 * a.nkx == a.plan.L) return launch_x_fwd2(a, phys, spec, st);
   dim3 grid((a.nrows + kXRows - 1) / kXRows);
   DNSB_DISPATCH(a.plan.L, x_fwd_kernel, grid, x_fwd_smem(a.plan.L), st, a, phys, spec);
   return cudaGetLastError();
@@ -1297,8 +1299,9 @@ cudaError_t set_pass_attributes(int max_smem) {
              (const void*)col_pass2_kernel<LL, 1, double, false, false, true>});
   });
 #undef DNSB_STOCKHAM
-  const cudaError_t x = set_x_pass_attributes(max_smem);
-  return x != cudaSuccess ? x : e;
+  for (cudaError_t r : {set_x_pass_attributes(max_smem), set_x_transform_attributes(max_smem)})
+    if (r != cudaSuccess) e = r;
+  return e;
 }
 
 }  // namespace dnsb

@@ -219,6 +219,12 @@ cudaError_t launch_x_pass(const XPassArgs& a, cudaStream_t st);
 // nkx = plan.L / 3.
 cudaError_t launch_x_pass2(const XPassArgs& a, cudaStream_t st);
 cudaError_t set_x_pass_attributes(int max_smem);
+// The register-stage x passes of the plain transforms (csrc/x_transform.cu),
+// same lengths.
+cudaError_t launch_x_phys2(const XPhysArgs& a, cudaStream_t st);
+cudaError_t launch_x_fwd2(const XPhysArgs& a, const double* phys, double2* spec,
+                          cudaStream_t st);
+cudaError_t set_x_transform_attributes(int max_smem);
 
 // Work lists of the ensemble form (one launch per pass for every member;
 // FP64 two-stage passes, padded lengths 48, 72, 96, 192).
