@@ -351,7 +351,7 @@ static XPassArgs periodic_xpass(const dnsb_periodic* p) {
 }
 
 // y forward as a two-stage column pass with truncation, A[f][y][kz][kx] ->
-// rhs[comp][ky][kz][kx] (complex128); the projection follows in place.
+// spec[comp][ky][kz][kx] (complex128), without the projection.
 static ColPassArgs periodic_yfwd_col(const dnsb_periodic* p, void* rhs) {
   ColPassArgs yc{};
   yc.in = p->A;
@@ -369,6 +369,22 @@ static ColPassArgs periodic_yfwd_col(const dnsb_periodic* p, void* rhs) {
   yc.tw = p->twy;
   yc.occ4 = 1;  // measured faster at 4 CTAs per SM
   return yc;
+}
+
+// y forward with the projection, A[f][y][kz][kx] -> rhs[comp][ky][kz][kx].
+static YProjArgs periodic_yproj(const dnsb_periodic* p, void* rhs) {
+  YProjArgs yp{};
+  yp.in = p->A;
+  yp.out = (double2*)rhs;
+  yp.NY1 = p->NY1;
+  yp.NZ1 = p->NZ1;
+  yp.NKX = p->NKX;
+  yp.kx = p->kx;
+  yp.ky = p->ky;
+  yp.kz = p->kz;
+  yp.inv_lapl = p->inv_lapl;
+  yp.tw = p->twy;
+  return yp;
 }
 
 // The five passes of the periodic RHS; bit k of `mask` runs pass k (y
@@ -435,14 +451,11 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
   yf.fp32 = f32;
   yf.variant = p->var[4];
   if ((mask & 16u) && p->var[4] == 0 && two_stage_length(p->My)) {
-    // y forward as a two-stage column pass with truncation, A[f][y][kz][kx]
-    // -> rhs[comp][ky][kz][kx] (complex128), then the projection in place
-    ColPassArgs yc = periodic_yfwd_col(p, rhs);
-    yc.skip = p->skip;
-    yc.tw = yf.tw;
-    yc.fp32 = f32;
-    DNSB_LAUNCH(launch_col_pass(yc, 3, p->NZ1, st));
-    DNSB_LAUNCH(launch_periodic_project(p->point(), (double2*)rhs, st));
+    YProjArgs yp = periodic_yproj(p, rhs);
+    yp.tw = yf.tw;
+    yp.fp32 = f32;
+    yp.skip = p->skip;
+    DNSB_LAUNCH(launch_yfwd_project(yp, p->My, st));
   } else if (mask & 16u) {
     DNSB_LAUNCH(launch_yfwd(yf, st));
   }
@@ -707,8 +720,8 @@ static dnsb_step_graph* new_step_graph(size_t n) {
 
 // Corrector iterations a periodic step graph captures unrolled: the
 // context's setting, when every kernel of an iteration checks the skip flag
-// (the two-stage passes at the compiled sizes, the y forward as a column
-// pass plus the projection), at most max_iter; otherwise none.
+// (the register-stage passes at the compiled sizes), at most max_iter;
+// otherwise none.
 static int periodic_unroll(const dnsb_periodic* p, int max_iter) {
   if (p->graph_unroll <= 0 || !two_stage_length(p->My) || !two_stage_length(p->Mz) ||
       !two_stage_length(p->Mx) || 3 * p->NKX != p->Mx)
@@ -982,6 +995,34 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
     return st;
   };
+  auto y_stage = [&](auto out_of) -> EnsStage {
+    EnsStage st;
+    st.kind = 4;
+    std::vector<EnsYItem> items;
+    std::vector<int> base;
+    int total = 0;
+    for (int m : order) {
+      EnsYItem it{};
+      it.a = periodic_yproj(ctxs[m], out_of(m));
+      it.L = ctxs[m]->My;
+      it.member = m;
+      base.push_back(total);
+      total += ens_y_blocks(it.a, &it.gx);
+      items.push_back(it);
+    }
+    EnsYItem* di = nullptr;
+    int* db = nullptr;
+    if (!rc) rc = ens_upload(e, items, &di);
+    if (!rc) rc = ens_upload(e, base, &db);
+    st.items = di;
+    st.base = db;
+    st.n = n;
+    st.total = total;
+    st.smem = ens_y_smem(maxL);
+    st.grid = rc ? 0 : ens_pass_grid(4, st.smem, total, smax);
+    if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
+    return st;
+  };
   auto point_list = [&](auto fill) -> EnsPointItem* {
     std::vector<EnsPointItem> items;
     for (int m : order) {
@@ -998,7 +1039,6 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   // RHS work lists for (in, out) = (state, Ra), (P, Rb), (P, Ra)
   struct RhsLists {
     EnsStage yc, zi, x, zf, yf;
-    EnsPointItem* proj = nullptr;
   } rl[3];
   for (int c = 0; c < 3; ++c) {
     auto in_of = [&](int m) -> const void* { return c == 0 ? states[m] : (const void*)P[m]; };
@@ -1010,12 +1050,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     rl[c].x = x_stage();
     rl[c].zf = col_stage(2, [&](const dnsb_periodic* q, int) { return periodic_zfwd(q); }, 3,
                          [](const dnsb_periodic* q) { return q->My; });
-    rl[c].yf = col_stage(2, [&](const dnsb_periodic* q, int m) { return periodic_yfwd_col(q, out_of(m)); },
-                         3, [](const dnsb_periodic* q) { return q->NZ1; });
-    rl[c].proj = point_list([&](EnsPointItem& it, int m) {
-      it.in0 = (const double2*)out_of(m);
-      it.out = (double2*)out_of(m);
-    });
+    rl[c].yf = y_stage(out_of);
   }
   EnsPointItem* pred = point_list([&](EnsPointItem& it, int m) {
     it.in0 = (const double2*)states[m];
@@ -1055,8 +1090,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     if ((r = run_pass(L.zi, act, s)) != cudaSuccess) return r;
     if ((r = run_pass(L.x, act, s)) != cudaSuccess) return r;
     if ((r = run_pass(L.zf, act, s)) != cudaSuccess) return r;
-    if ((r = run_pass(L.yf, act, s)) != cudaSuccess) return r;
-    return launch_ens_point(L.proj, n, act, 2, 1, 0, pgrid, s);
+    return run_pass(L.yf, act, s);
   };
   auto correct = [&](int k, const int* act, cudaStream_t s) -> cudaError_t {
     cudaError_t r = launch_ens_point(corr[k], n, act, 1, 0, 0, pgrid, s);
@@ -1131,10 +1165,10 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     ensemble_free(e);
     return rc;
   }
-  // launches: prologue 2 RHS (6 each) + predict + correct + finalize +
-  // control, epilogue 1; an iteration 6 + 3
-  e->k_fixed = 2 * 6 + 4 + 1;
-  e->k_iter = 6 + 3;
+  // launches: prologue 2 RHS (5 each) + predict + correct + finalize +
+  // control, epilogue 1; an iteration 5 + 3
+  e->k_fixed = 2 * 5 + 4 + 1;
+  e->k_iter = 5 + 3;
   *out = e;
   return 0;
 }

@@ -599,6 +599,24 @@ __device__ __forceinline__ int pos_to_stored(int t, int nstored, int M) {
   return -1;
 }
 
+// u - grad(inv_lapl div u) of one mode (monochromatic.py:377-385, 516-565), each
+// rounding written out: the kernels that project give the same bits whatever
+// surrounds the call.
+__device__ __forceinline__ void project_mode(double2 (&u)[3], double kx, double ky, double kz,
+                                             double inv_lapl) {
+  const double k[3] = {kx, ky, kz};
+  // div u = i (sx + i sy); p = inv_lapl div u
+  const double sx = __fma_rn(kz, u[2].x, __fma_rn(ky, u[1].x, __dmul_rn(kx, u[0].x)));
+  const double sy = __fma_rn(kz, u[2].y, __fma_rn(ky, u[1].y, __dmul_rn(kx, u[0].y)));
+  const double px = __dmul_rn(sx, inv_lapl), py = __dmul_rn(sy, inv_lapl);
+  // - i k (i p) = k p
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    u[q].x = __fma_rn(k[q], px, u[q].x);
+    u[q].y = __fma_rn(k[q], py, u[q].y);
+  }
+}
+
 // Raise a kernel's dynamic shared-memory limit to what is left of max_smem
 // after its static shared memory.
 inline cudaError_t allow_dynamic_smem(const void* fn, int max_smem) {

@@ -134,27 +134,15 @@ col_pass_kernel(ColPassArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int col_columns(int L) { return L >= 288 ? 8 : 16; }
 template <int M>
-struct ColShape;
-#define DNSB_COL_SHAPE(M_, R1_, R2_, C_, ZB_)                                     \
-  template <>                                                                     \
-  struct ColShape<M_> {                                                           \
-    static constexpr int R1 = R1_, R2 = R2_, C = C_, NT = R2_ * C_, ZB = ZB_;     \
-    static_assert(R1 * R2 == M_ && C == col_columns(M_), "two radices");          \
-  };
-// ZB: CTAs per SM that the Couette z inverse's registers are held to
-DNSB_COL_SHAPE(36, 6, 6, 16, 5)
-DNSB_COL_SHAPE(48, 6, 8, 16, 4)
-DNSB_COL_SHAPE(54, 9, 6, 16, 5)
-DNSB_COL_SHAPE(72, 9, 8, 16, 4)
-DNSB_COL_SHAPE(96, 12, 8, 16, 4)
-DNSB_COL_SHAPE(108, 12, 9, 16, 3)
-DNSB_COL_SHAPE(144, 12, 12, 16, 3)
-DNSB_COL_SHAPE(162, 18, 9, 16, 3)
-DNSB_COL_SHAPE(192, 24, 8, 16, 4)
-DNSB_COL_SHAPE(216, 18, 12, 16, 2)
-DNSB_COL_SHAPE(288, 24, 12, 8, 4)
-DNSB_COL_SHAPE(384, 24, 16, 8, 4)
-#undef DNSB_COL_SHAPE
+struct ColShape {
+  static constexpr int R1 = ColRadix<M>::R1, R2 = ColRadix<M>::R2, C = col_columns(M);
+  static constexpr int NT = R2 * C;
+  // CTAs per SM that the Couette z inverse's registers are held to
+  static constexpr int ZB = M == 36 || M == 54               ? 5
+                            : M == 108 || M == 144 || M == 162 ? 3
+                            : M == 216                         ? 2
+                                                               : 4;
+};
 
 size_t col_pass2_smem(int M) {
   return sizeof(double2) * (size_t)(M * col_columns(M) + M);
@@ -569,7 +557,8 @@ static const void* ens_kernel(int kind) {
     case 0: return (const void*)ens_col_pass2_kernel<1, true>;
     case 1: return (const void*)ens_col_pass2_kernel<1, false>;
     case 2: return (const void*)ens_col_pass2_kernel<-1, false>;
-    default: return ens_x_kernel();
+    case 3: return ens_x_kernel();
+    default: return ens_y_kernel();
   }
 }
 
@@ -579,7 +568,7 @@ int ens_pass_grid(int kind, size_t smem, int total, int max_smem) {
   const void* f = ens_kernel(kind);
   if (allow_dynamic_smem(f, max_smem) != cudaSuccess) return 0;
   int per_sm = 0, dev = 0, nsm = 0;
-  const int threads = kind == 3 ? kEnsXThreads : kEnsColThreads;
+  const int threads = kind == 3 ? kEnsXThreads : kind == 4 ? kEnsYThreads : kEnsColThreads;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess)
     return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -604,6 +593,9 @@ cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n,
       ens_col_pass2_kernel<-1, false><<<grid, kEnsColThreads, smem, st>>>(
           static_cast<const EnsColItem*>(items), base, n, total, active);
       break;
+    case 4:
+      return launch_ens_y(static_cast<const EnsYItem*>(items), base, n, total, active, grid,
+                          smem, st);
     default:
       return launch_ens_x(static_cast<const EnsXItem*>(items), base, n, total, active, grid,
                           smem, st);
@@ -1299,7 +1291,8 @@ cudaError_t set_pass_attributes(int max_smem) {
              (const void*)col_pass2_kernel<LL, 1, double, false, false, true>});
   });
 #undef DNSB_STOCKHAM
-  for (cudaError_t r : {set_x_pass_attributes(max_smem), set_x_transform_attributes(max_smem)})
+  for (cudaError_t r : {set_x_pass_attributes(max_smem), set_x_transform_attributes(max_smem),
+                        set_yfwd_project_attributes(max_smem)})
     if (r != cudaSuccess) e = r;
   return e;
 }

@@ -49,6 +49,29 @@ inline void for_each_length(F&& f) {
   DNSB_LENGTHS(DNSB_LEN)
 #undef DNSB_LEN
 }
+// Two radices of a column transform, M = R1 R2.
+template <int M>
+struct ColRadix;
+#define DNSB_COL_RADIX(M_, R1_, R2_)                       \
+  template <>                                              \
+  struct ColRadix<M_> {                                    \
+    static constexpr int R1 = R1_, R2 = R2_;               \
+    static_assert(R1 * R2 == M_, "two radices");           \
+  };
+DNSB_COL_RADIX(36, 6, 6)
+DNSB_COL_RADIX(48, 6, 8)
+DNSB_COL_RADIX(54, 9, 6)
+DNSB_COL_RADIX(72, 9, 8)
+DNSB_COL_RADIX(96, 12, 8)
+DNSB_COL_RADIX(108, 12, 9)
+DNSB_COL_RADIX(144, 12, 12)
+DNSB_COL_RADIX(162, 18, 9)
+DNSB_COL_RADIX(192, 24, 8)
+DNSB_COL_RADIX(216, 18, 12)
+DNSB_COL_RADIX(288, 24, 12)
+DNSB_COL_RADIX(384, 24, 16)
+#undef DNSB_COL_RADIX
+
 // Shared memory a kernel may use without raising its limit (less a margin for
 // its static arrays).
 constexpr size_t kDefaultSmem = 47 * 1024;
@@ -176,6 +199,34 @@ struct YFwdArgs {
   int variant;  // 0 / 1: compile-time plan when compiled for L, 2: runtime plan
 };
 
+// Periodic last forward pass (y) with the projection, two-stage lengths
+// (csrc/y_project.cu): in [3][My][NZ1][NKX] -> spectral [3][NY1][NZ1][NKX].
+struct YProjArgs {
+  const double2* in;
+  double2* out;
+  int NY1, NZ1, NKX;
+  const double* kx;
+  const double* ky;
+  const double* kz;
+  const double* inv_lapl;  // [NY1][NZ1][NKX]
+  const double2* tw;       // float2 table when fp32
+  int fp32;                // FP32 input pass buffer and transform
+  const int* skip = nullptr;  // as ColPassArgs::skip
+};
+cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st);
+// Its work-list form for ensembles (see EnsColItem).
+struct EnsYItem {
+  YProjArgs a;
+  int L, gx, member;
+};
+constexpr int kEnsYThreads = 192;
+int ens_y_blocks(const YProjArgs& a, int* gx);
+size_t ens_y_smem(int maxL);
+const void* ens_y_kernel();
+cudaError_t launch_ens_y(const EnsYItem* items, const int* base, int n, int total,
+                         const int* active, int grid, size_t smem, cudaStream_t st);
+cudaError_t set_yfwd_project_attributes(int max_smem);
+
 // Couette first inverse pass (z), FD curl fused: spectral
 // [3][NZ1][NKX][Ny] -> 6 (or 3) fields [f][Mz][NKX][Ny].
 struct ZInvCurlArgs {
@@ -257,7 +308,7 @@ __device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int
 size_t ens_col_smem(int maxL);
 size_t ens_x_smem(int maxL, int maxNKX);
 // kind 0: inverse pass with the spectral curl, 1: inverse, 2: forward
-// (column passes); 3: the x pass.  base[k]: first virtual block of item k.
+// (column passes); 3: the x pass; 4: the y forward pass with the projection.  base[k]: first virtual block of item k.
 int ens_pass_grid(int kind, size_t smem, int total, int max_smem);
 cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n, int total,
                             const int* active, int grid, size_t smem, cudaStream_t st);

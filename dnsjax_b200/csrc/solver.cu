@@ -202,26 +202,19 @@ __device__ __forceinline__ void periodic_cv_body(const PeriodicPointArgs& a, con
                                                  int vb, int vgrid) {
   const int S = a.S;
   for (int s = vb * blockDim.x + threadIdx.x; s < S; s += vgrid * blockDim.x) {
-    double2 u0 = in[s], u1 = in[S + s], u2 = in[2 * S + s];
+    double2 u[3] = {in[s], in[S + s], in[2 * S + s]};
     if (divergence) {
       const int ix = s % a.NKX;
       const int iz = (s / a.NKX) % a.NZ1;
       const int iy = s / (a.NKX * a.NZ1);
-      const double kx = a.kx[ix], ky = a.ky[iy], kz = a.kz[iz];
-      const double2 div = cadd(cadd(cik(kx, u0), cik(ky, u1)), cik(kz, u2));
-      const double2 p = cscale(div, a.inv_lapl[s]);
-      // state + (-grad p)
-      const double2 g0 = cik(kx, p), g1 = cik(ky, p), g2 = cik(kz, p);
-      u0 = cadd(u0, make_double2(-g0.x, -g0.y));
-      u1 = cadd(u1, make_double2(-g1.x, -g1.y));
-      u2 = cadd(u2, make_double2(-g2.x, -g2.y));
+      project_mode(u, a.kx[ix], a.ky[iy], a.kz[iz], a.inv_lapl[s]);
     }
     if (s == 0 && zero_mean && a.kx0) {
-      u0 = u1 = u2 = make_double2(0.0, 0.0);
+      u[0] = u[1] = u[2] = make_double2(0.0, 0.0);
     }
-    out[s] = u0;
-    out[S + s] = u1;
-    out[2 * S + s] = u2;
+    out[s] = u[0];
+    out[S + s] = u[1];
+    out[2 * S + s] = u[2];
   }
 }
 
@@ -236,14 +229,6 @@ cudaError_t launch_periodic_correct_velocity(const PeriodicPointArgs& a,
                                              const double2* in, double2* out,
                                              int divergence, cudaStream_t st) {
   periodic_cv_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(a, in, out, divergence, 1);
-  return cudaGetLastError();
-}
-
-// The RHS projection NL - grad(inv_lapl div NL) (monochromatic.py:377-385),
-// in place, the mean mode kept.
-cudaError_t launch_periodic_project(const PeriodicPointArgs& a, double2* rhs,
-                                   cudaStream_t st) {
-  periodic_cv_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(a, rhs, rhs, 1, 0);
   return cudaGetLastError();
 }
 

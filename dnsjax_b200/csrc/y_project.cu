@@ -1,0 +1,180 @@
+// Periodic y forward transform with truncation and the pressure projection
+// NL - grad(inv_lapl div NL) (src/dnsjax/flows/monochromatic.py:366-386), in
+// register stages: a CTA takes 8 (kz, kx) columns of all three components, a
+// third of its threads each.  The transformed columns stay in shared memory
+// until every component of a mode is there.
+//
+// As two kernels, the transform wrote the RHS and the projection read and wrote
+// it again: 100 of 125 + 100 MB at 128^3, and one launch more, which is what
+// counts on small grids.  8 columns leave room for 2 CTAs per SM at every
+// length up to 288 (3 components x M x 8 columns), 16 would leave one.
+// Measured: 32^3 time step 183 -> 175 us, 24 x 36 x 48 predict_and_correct 85 ->
+// 81 us, 256^3 RHS 3.35 -> 3.28 ms, 128^3 as before (FP32 229 -> 225 us).
+#include "passes.cuh"
+
+namespace dnsb {
+
+namespace {
+
+// Radices (M = R1 R2) of the column pass; 8 columns, so NF threads per
+// component and R1 items per thread group of R2.
+template <int M>
+struct YShape {
+  static constexpr int C = 8;
+  static constexpr int R1 = ColRadix<M>::R1, R2 = ColRadix<M>::R2;
+  static constexpr int NF = R2 * C, NT = 3 * NF;
+  // registers: R1 <= 24 complex values a thread
+  static constexpr int MINB = NT <= 192 ? 2 : 1;
+};
+
+template <int ML, typename T>
+__device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, int iz) {
+  using CT = typename pass_types<T>::C;
+  using SH = YShape<ML>;
+  constexpr int M = ML, R1 = SH::R1, R2 = SH::R2, C = SH::C, NF = SH::NF, NT = SH::NT;
+  extern __shared__ double2 sm_[];
+  CT* sm = reinterpret_cast<CT*>(sm_);  // [component][t][C]
+  const CT* __restrict__ tw = reinterpret_cast<const CT*>(a.tw);
+  const int tid = threadIdx.x, f = tid / NF, t0 = tid % NF;
+  const int NY1 = a.NY1, NZ1 = a.NZ1, NKX = a.NKX;
+  const int i0 = bx * C;
+  const int ni = min(C, NKX - i0);
+  CT* X = sm + f * M * C;
+  const long long row = (long long)NZ1 * NKX;  // stride of y
+  {
+    const int c = t0 % C, j = t0 / C;
+    const CT* in = reinterpret_cast<const CT*>(a.in) + (long long)f * M * row +
+                   (long long)iz * NKX + i0 + c;
+    const unsigned long long drop = l2_drop();
+    CT v[R1];
+#pragma unroll
+    for (int i = 0; i < R1; ++i)
+      v[i] = c < ni ? CT(ld_l2(in + (j + R2 * i) * row, drop)) : cmake<CT>(0, 0);
+    dft_reg<R1, -1>(v);
+#pragma unroll
+    for (int i = 0; i < R1; ++i) X[(j * R1 + i) * C + c] = v[i];
+  }
+  __syncthreads();
+  for (int it = t0; it < R1 * C; it += NF) {
+    const int c = it % C, k = it / C;
+    CT z[R2];
+#pragma unroll
+    for (int i = 0; i < R2; ++i) z[i] = X[(k + R1 * i) * C + c];
+#pragma unroll
+    for (int i = 1; i < R2; ++i) z[i] = cmul(z[i], CT(tw[i * k]));
+    dft_reg<R2, -1>(z);
+    // position k + R1 i: where the item read
+#pragma unroll
+    for (int i = 0; i < R2; ++i) X[(k + R1 * i) * C + c] = z[i];
+  }
+  __syncthreads();
+  const double sc = 1.0 / M;
+  const double kz = a.kz[iz];
+  const long long cs = (long long)NY1 * row;
+  for (int idx = tid; idx < NY1 * C; idx += NT) {
+    const int c = idx % C, s = idx / C;
+    if (c >= ni) continue;
+    const int t = stored_to_pos(s, NY1, M) * C + c;
+    double2 u[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      // rounded before the projection, as where the transform stores it (the
+      // work-list ensemble's kernels give the same bits)
+      const double2 z = to_d(sm[q * M * C + t]);
+      u[q] = make_double2(__dmul_rn(z.x, sc), __dmul_rn(z.y, sc));
+    }
+    const long long off = s * row + (long long)iz * NKX + i0 + c;
+    project_mode(u, a.kx[i0 + c], a.ky[s], kz, a.inv_lapl[off]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) a.out[q * cs + off] = u[q];
+  }
+}
+
+template <int ML, typename T>
+__global__ void __launch_bounds__(YShape<ML>::NT, YShape<ML>::MINB)
+yfwd_project_kernel(YProjArgs a) {
+  if (a.skip && *a.skip) return;
+  yfwd_project_body<ML, T>(a, blockIdx.x, blockIdx.y);
+}
+
+// Work-list form for ensembles: as ens_x_pass2_kernel (csrc/x_pass.cu).
+static_assert(YShape<48>::NT == kEnsYThreads && YShape<72>::NT == kEnsYThreads &&
+                  YShape<96>::NT == kEnsYThreads && YShape<192>::NT == kEnsYThreads,
+              "one CTA shape for every member");
+__global__ void __launch_bounds__(kEnsYThreads)
+ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restrict__ base, int n,
+                        int total, const int* __restrict__ active) {
+  __shared__ int s_k;
+  for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
+    if (threadIdx.x == 0) s_k = ens_find(base, n, vb);
+    __syncthreads();
+    const int k = s_k;
+    const int m = items[k].member;
+    if (!active || active[m]) {
+      const YProjArgs a = items[k].a;
+      const int gx = items[k].gx, bx = (vb - base[k]) % gx, iz = (vb - base[k]) / gx;
+      switch (items[k].L) {
+        case 48: yfwd_project_body<48, double>(a, bx, iz); break;
+        case 72: yfwd_project_body<72, double>(a, bx, iz); break;
+        case 96: yfwd_project_body<96, double>(a, bx, iz); break;
+        default: yfwd_project_body<192, double>(a, bx, iz); break;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int ML>
+constexpr size_t yproj_smem() {
+  return sizeof(double2) * (size_t)(3 * ML * YShape<ML>::C);
+}
+
+}  // namespace
+
+cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st) {
+  if (a.fp32 && !fp32_length(L)) return cudaErrorInvalidValue;
+  return with_length(L, [&](auto len) {
+    constexpr int LL = decltype(len)::value;
+    using SH = YShape<LL>;
+    const dim3 grid((a.NKX + SH::C - 1) / SH::C, a.NZ1);
+    const size_t sm = a.fp32 ? yproj_smem<LL>() / 2 : yproj_smem<LL>();
+    if constexpr (fp32_length(LL)) {
+      if (a.fp32 == 2) yfwd_project_kernel<LL, fcomp><<<grid, SH::NT, sm, st>>>(a);
+      else if (a.fp32) yfwd_project_kernel<LL, float><<<grid, SH::NT, sm, st>>>(a);
+      if (a.fp32) return cudaGetLastError();
+    }
+    yfwd_project_kernel<LL, double><<<grid, SH::NT, sm, st>>>(a);
+    return cudaGetLastError();
+  });
+}
+
+int ens_y_blocks(const YProjArgs& a, int* gx) {
+  *gx = (a.NKX + YShape<192>::C - 1) / YShape<192>::C;
+  return *gx * a.NZ1;
+}
+
+size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192>::C); }
+
+const void* ens_y_kernel() { return (const void*)ens_yfwd_project_kernel; }
+
+cudaError_t launch_ens_y(const EnsYItem* items, const int* base, int n, int total,
+                         const int* active, int grid, size_t smem, cudaStream_t st) {
+  ens_yfwd_project_kernel<<<grid, kEnsYThreads, smem, st>>>(items, base, n, total, active);
+  return cudaGetLastError();
+}
+
+cudaError_t set_yfwd_project_attributes(int max_smem) {
+  cudaError_t e = cudaSuccess;
+  for_each_length([&](auto len) {
+    constexpr int LL = decltype(len)::value;
+    if (yproj_smem<LL>() <= kDefaultSmem) return;
+    const cudaError_t r =
+        allow_dynamic_smem((const void*)yfwd_project_kernel<LL, double>, max_smem);
+    if (r != cudaSuccess) e = r;
+    static_assert(!fp32_length(LL) || yproj_smem<LL>() / 2 <= kDefaultSmem,
+                  "the FP32 forms stay within the default");
+  });
+  return e;
+}
+
+}  // namespace dnsb
