@@ -129,6 +129,18 @@ struct dnsb_periodic {
   // flag that makes the iteration's kernels return at once
   const int* skip = nullptr;
 
+  bool graph = false;  // a step graph is being captured
+
+  // Dependent launches for the kernels of a call on small grids, where the gaps
+  // between kernels count (24 x 36 x 48 predict_and_correct 81 -> 70 us, 96 x 72 x
+  // 144 RHS 199 -> 190 us, 128^3 FP32 RHS 225 -> 218 us); on larger ones the early
+  // blocks of the next kernel cost more than the gap (128^3 FP64 RHS 332 -> 337
+  // us, 256^3 3.28 -> 3.39 ms).  Not inside step graphs, whose edges are as short
+  // without (32^3 step 173 us without, 176 with).
+  int dep() const {
+    return !graph && (long long)Mx * My * Mz <= (rhs_fp32 ? 192LL * 192 * 192 : 4000000LL);
+  }
+
   PeriodicPointArgs point() const {
     PeriodicPointArgs a;
     a.S = S;
@@ -145,6 +157,7 @@ struct dnsb_periodic {
     a.c = c;
     a.kx0 = slab.rank == 0 ? 1 : 0;
     a.skip = skip;
+    a.dep = dep();
     return a;
   }
 };
@@ -411,6 +424,7 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
     // [comp][ky][kz][kx] -> A[f][y][kz][kx]
     ColPassArgs yc = periodic_ycurl(p, state);
     yc.skip = p->skip;
+    yc.dep = p->dep();
     yc.tw = yi.tw;
     yc.fp32 = yc.out32 = f32;
     DNSB_LAUNCH(launch_col_pass(yc, 6, p->NZ1, st));
@@ -419,18 +433,21 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
   }
   ColPassArgs zi = periodic_zinv(p);
   zi.skip = p->skip;
+  zi.dep = p->dep();
   zi.fp32 = zi.out32 = f32;
   if (f32) zi.tw = reinterpret_cast<const double2*>(p->twz32);
   zi.variant = p->var[1];
   if (mask & 2u) DNSB_LAUNCH(launch_col_pass(zi, 6, p->My, st));
   XPassArgs xa = periodic_xpass(p);
   xa.skip = p->skip;
+  xa.dep = p->dep();
   xa.tw = f32 ? reinterpret_cast<const double2*>(p->twx32) : p->twx;
   xa.fp32 = f32;
   xa.variant = p->var[2];
   if (mask & 4u) DNSB_LAUNCH(launch_x_pass(xa, st));
   ColPassArgs zf = periodic_zfwd(p);
   zf.skip = p->skip;
+  zf.dep = p->dep();
   zf.fp32 = zf.out32 = f32;
   if (f32) zf.tw = reinterpret_cast<const double2*>(p->twz32);
   zf.variant = p->var[3];
@@ -455,6 +472,7 @@ static int periodic_rhs_impl(dnsb_periodic* p, const void* state, void* rhs, uns
     yp.tw = yf.tw;
     yp.fp32 = f32;
     yp.skip = p->skip;
+    yp.dep = p->dep();
     DNSB_LAUNCH(launch_yfwd_project(yp, p->My, st));
   } else if (mask & 16u) {
     DNSB_LAUNCH(launch_yfwd(yf, st));
@@ -706,6 +724,13 @@ static int build_step_graph(dnsb_step_graph* g, double tol, int max_iter,
   return rc;
 }
 
+// A context's `graph` flag, set while a step graph captures its calls.
+struct GraphScope {
+  bool& flag;
+  explicit GraphScope(bool& f) : flag(f) { flag = true; }
+  ~GraphScope() { flag = false; }
+};
+
 static dnsb_step_graph* new_step_graph(size_t n) {
   auto* g = new dnsb_step_graph();
   if (cudaMalloc(&g->P, n * sizeof(double2)) || cudaMalloc(&g->Ra, n * sizeof(double2)) ||
@@ -767,6 +792,7 @@ extern "C" int dnsb_periodic_step_graph_create(dnsb_periodic* p, void* state, do
   auto epilogue = [&](cudaStream_t s) {
     return dnsb_periodic_correct_velocity(p, g->P, state, divergence, s);
   };
+  const GraphScope scope(p->graph);
   const int rc = build_step_graph(g, tol, max_iter, prologue, body, epilogue,
                                  periodic_unroll(p, max_iter));
   if (rc) {
@@ -1333,6 +1359,15 @@ struct dnsb_couette {
   // flag that makes the iteration's kernels return at once
   const int* skip = nullptr;
 
+  bool graph = false;  // a step graph is being captured
+
+  // Dependent launches, as dnsb_periodic::dep (128 x 129 x 128 RHS 203 us without,
+  // 207 with; 64 x 65 x 64 predict_and_correct 221 -> 200 us).
+  int dep_rhs() const {
+    return !graph && (long long)Mx * Mz * Ny <= (rhs_fp32 ? 192LL * 192 * 129 : 4000000LL);
+  }
+  int dep_imm() const { return !graph && (long long)NM * Ny <= 1200000; }
+
   ImmArgs imm() const {
     ImmArgs a{};
     a.NZ1 = NZ1;
@@ -1366,6 +1401,7 @@ struct dnsb_couette {
     a.ab_row0 = ab_row0;
     a.pair_modes = pair_modes;
     a.kx0 = slab.rank == 0 ? 1 : 0;
+    a.dep = dep_imm();
     return a;
   }
 };
@@ -1665,6 +1701,7 @@ static int couette_rhs_impl(dnsb_couette* p, const void* state, void* rhs, unsig
   zi.fp32 = p->rhs_fp32;
   zi.variant = p->var[0];
   zi.skip = p->skip;
+  zi.dep = p->dep_rhs();
   if (mask & 1u) DNSB_LAUNCH(launch_zinv_curl(zi, p->span_max, st));
   XPassArgs xa{};
   xa.in = p->B;
@@ -1687,6 +1724,7 @@ static int couette_rhs_impl(dnsb_couette* p, const void* state, void* rhs, unsig
   xa.fp32 = p->rhs_fp32;
   xa.variant = p->var[1];
   xa.skip = p->skip;
+  xa.dep = p->dep_rhs();
   if (mask & 2u) DNSB_LAUNCH(launch_x_pass(xa, st));
   ColPassArgs zf{};
   zf.in = p->B;
@@ -1705,6 +1743,7 @@ static int couette_rhs_impl(dnsb_couette* p, const void* state, void* rhs, unsig
   zf.fp32 = p->rhs_fp32;
   zf.variant = p->var[2];
   zf.skip = p->skip;
+  zf.dep = p->dep_rhs();
   if (mask & 4u) DNSB_LAUNCH(launch_col_pass(zf, 3, p->NKX, st));
   return 0;
 }
@@ -1924,6 +1963,7 @@ extern "C" int dnsb_couette_step_graph_create(dnsb_couette* p, void* state, doub
       return fail(DNSB_ERR_CUDA, "state copy");
     return 0;
   };
+  const GraphScope scope(p->graph);
   const int rc = build_step_graph(g, tol, max_iter, prologue, body, epilogue,
                                  couette_unroll(p, max_iter));
   if (rc) {
@@ -2077,6 +2117,7 @@ extern "C" int dnsb_couette_mixed_graph_create(dnsb_couette* p, void* state, voi
     mixed_graph_free(g);
     return fail(DNSB_ERR_CUDA, "mixed step graph allocation failed");
   }
+  const GraphScope scope(p->graph);
   const int keep = p->rhs_fp32;
   // the RHS passes of one precision (the context's own setting is restored)
   auto rhs = [&](const void* in, void* o, int prec, cudaStream_t s) {

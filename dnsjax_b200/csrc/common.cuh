@@ -740,6 +740,30 @@ __device__ __forceinline__ void cp_async_wait_2() {
   asm volatile("cp.async.wait_group 2;\n" ::: "memory");
 }
 
+// Programmatic dependent launch: a kernel launched by launch_dep with dep != 0
+// may be set up while the kernel before it on the stream is finishing; it waits
+// here, first thing, for that kernel's results, and lets the next one be set up
+// in turn.  Without the launch attribute both are no-ops.
+__device__ __forceinline__ void grid_dep_sync() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <typename... KA, typename... A>
+inline cudaError_t launch_dep(int dep, void (*kernel)(KA...), dim3 grid, int threads,
+                              size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = dep ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, KA(args)...);
+}
+
 template <typename C>
 __device__ __forceinline__ void load_twiddles(C* s, const C* g, int L) {
   for (int i = threadIdx.x; i < L; i += blockDim.x) s[i] = g[i];

@@ -152,6 +152,7 @@ imm_stage013_kernel(ImmArgs a, int paired, const double* __restrict__ w1x,
                     const double2* __restrict__ vel_n, const double2* __restrict__ nl_n,
                     const double2* __restrict__ nl_j, double2* __restrict__ F,
                     double2* __restrict__ R, long long cs) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   constexpr int W = KL + 2 + YM - 1;
   extern __shared__ double2 sm[];
@@ -308,6 +309,7 @@ template <int KL>
 __global__ void __launch_bounds__(kLanes * kGradRows)
 imm_grad_kernel(ImmArgs a, int paired, int NP, const double2* __restrict__ P,
                 double2* __restrict__ R, long long cs) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   constexpr int S1 = KL + 1;
   const int lane = threadIdx.x & 31, side = lane / kTile, Ny = a.Ny;
@@ -350,6 +352,7 @@ __global__ void __launch_bounds__(32 * kStageWarps)
 imm_stage6_kernel(ImmArgs a, int paired, const double2* __restrict__ R, long long cs,
                   const double2* vel_j, double2* vel_new, double2* __restrict__ corr_out,
                   double* __restrict__ partials) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   constexpr int S1 = KL + 1, YR = YM > 0 ? YM : 1;
   extern __shared__ double2 sm[];
@@ -893,6 +896,9 @@ static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, long lon
   if (s.ring == 0) return cudaErrorInvalidValue;
   const size_t sm = (size_t)s.ring * s.slot_bytes;
   const int grid = (bt.NP + kTile - 1) / kTile;
+  // Never dependent on the kernel before: the one or two CTAs an SM has room for
+  // would gather on the SMs that finish first (96 x 71 x 108 corrector: 97 us
+  // so, 110 us with dependent substitutions).
   if (bt.nu == KL + 1)
     imm_solve_kernel<KL, KL + 1><<<grid, 32 * (ncomp + 1), sm, st>>>(s);
   else
@@ -913,9 +919,7 @@ static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2*
   cudaError_t e;
 #define DNSB_STAGE013(YM)                                                                   \
   case YM:                                                                                  \
-    imm_stage013_kernel<K, YM><<<grid, threads, sm, st>>>(a, bt.paired, bt.w1x, bt.w2x,     \
-                                                          bt.base, vel_n, nl_n, nl_j, bt.F, \
-                                                          bt.R, cs);                        \
+    launch_dep(a.dep, imm_stage013_kernel<K, YM>, grid, threads, sm, st, a, bt.paired, bt.w1x, bt.w2x, bt.base, vel_n, nl_n, nl_j, bt.F, bt.R, cs);                        \
     break;
   switch (imm_batch_rows(Ny)) {
     DNSB_STAGE013(3) DNSB_STAGE013(5) DNSB_STAGE013(7) DNSB_STAGE013(9) DNSB_STAGE013(17)
@@ -925,19 +929,16 @@ static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2*
   e = solve_launch<K>(bt, 0, bt.F, 0, 1, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
   const dim3 gg((Ny - 2 + kGradRows - 1) / kGradRows, tiles);
-  imm_grad_kernel<K><<<gg, kLanes * kGradRows, 0, st>>>(a, bt.paired, bt.NP, bt.F, bt.R, cs);
+  launch_dep(a.dep, imm_grad_kernel<K>, gg, kLanes * kGradRows, 0, st, a, bt.paired, bt.NP, bt.F, bt.R, cs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = solve_launch<K>(bt, 1, bt.R, cs, 3, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
   if (Ny <= 96)
-    imm_stage6_kernel<K, 3><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
-                                                        corr_out, partials);
+    launch_dep(a.dep, imm_stage6_kernel<K, 3>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
   else if (Ny <= 160)
-    imm_stage6_kernel<K, 5><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
-                                                        corr_out, partials);
+    launch_dep(a.dep, imm_stage6_kernel<K, 5>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
   else
-    imm_stage6_kernel<K, 0><<<grid, threads, sm6, st>>>(a, bt.paired, bt.R, cs, vel_j, vel_new,
-                                                        corr_out, partials);
+    launch_dep(a.dep, imm_stage6_kernel<K, 0>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
   return cudaGetLastError();
 }
 

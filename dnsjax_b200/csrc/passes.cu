@@ -279,6 +279,7 @@ template <int ML, int SIGN, typename T = double, bool OUT32 = false, bool CURL =
           bool SLAB = false>
 __global__ void __launch_bounds__(ColShape<ML>::NT)
 col_pass2_kernel(ColPassArgs a) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   col_pass2_body<ML, SIGN, T, OUT32, CURL, SLAB>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -290,6 +291,7 @@ col_pass2_kernel(ColPassArgs a) {
 template <int ML, int SIGN, bool CURL>
 __global__ void __launch_bounds__(ColShape<ML>::NT, 512 / ColShape<ML>::NT)
 col_pass2_occ4_kernel(ColPassArgs a) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   col_pass2_body<ML, SIGN, double, false, CURL, false>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -309,37 +311,37 @@ cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
       constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;
       if constexpr (fp32_length(LL)) {
         if (slab)
-          col_pass2_kernel<LL, 1, double, false, false, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, double, false, false, true>, g2, NT, sm2, st, a);
         else if (a.curl && a.fp32 == 2)
-          col_pass2_kernel<LL, 1, fcomp, true, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, fcomp, true, true>, g2, NT, sm2, st, a);
         else if (a.fp32 == 2 && a.inverse)
-          col_pass2_kernel<LL, 1, fcomp, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, fcomp, true>, g2, NT, sm2, st, a);
         else if (a.fp32 == 2 && a.out32)
-          col_pass2_kernel<LL, -1, fcomp, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, -1, fcomp, true>, g2, NT, sm2, st, a);
         else if (a.fp32 == 2)
-          col_pass2_kernel<LL, -1, fcomp><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, -1, fcomp>, g2, NT, sm2, st, a);
         else if (a.curl && a.fp32)
-          col_pass2_kernel<LL, 1, float, true, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, float, true, true>, g2, NT, sm2, st, a);
         else if (a.fp32 && a.inverse)
-          col_pass2_kernel<LL, 1, float, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, float, true>, g2, NT, sm2, st, a);
         else if (a.fp32 && a.out32)
-          col_pass2_kernel<LL, -1, float, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, -1, float, true>, g2, NT, sm2, st, a);
         else if (a.fp32)
-          col_pass2_kernel<LL, -1, float><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, -1, float>, g2, NT, sm2, st, a);
         else if (!a.occ4 && a.curl)
-          col_pass2_kernel<LL, 1, double, false, true><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, double, false, true>, g2, NT, sm2, st, a);
         else if (!a.occ4 && a.inverse)
-          col_pass2_kernel<LL, 1><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1>, g2, NT, sm2, st, a);
         else if (!a.occ4)
-          col_pass2_kernel<LL, -1><<<g2, NT, sm2, st>>>(a);
+          launch_dep(a.dep, col_pass2_kernel<LL, -1>, g2, NT, sm2, st, a);
         if (slab || a.fp32 || !a.occ4) return cudaGetLastError();
       }
       if (a.curl)
-        col_pass2_occ4_kernel<LL, 1, true><<<g2, NT, sm2, st>>>(a);
+        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, true>, g2, NT, sm2, st, a);
       else if (a.inverse)
-        col_pass2_occ4_kernel<LL, 1, false><<<g2, NT, sm2, st>>>(a);
+        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, false>, g2, NT, sm2, st, a);
       else
-        col_pass2_occ4_kernel<LL, -1, false><<<g2, NT, sm2, st>>>(a);
+        launch_dep(a.dep, col_pass2_occ4_kernel<LL, -1, false>, g2, NT, sm2, st, a);
       return cudaGetLastError();
     });
   }
@@ -1139,6 +1141,7 @@ template <int ML, typename T = double, bool SLAB = false>
 __global__ void __launch_bounds__(ColShape<ML>::NT,
                                   std::is_same<T, float>::value ? 6 : ColShape<ML>::ZB)
 zinv_curl2_kernel(ZInvCurlArgs a) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   using CT = typename pass_types<T>::C;
   using RT = typename pass_types<T>::R;
@@ -1241,12 +1244,12 @@ cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,
     return with_length(L, [&](auto len) {
       constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;
       if constexpr (fp32_length(LL)) {
-        if (slab) zinv_curl2_kernel<LL, double, true><<<grid, NT, sm, st>>>(a);
-        else if (a.fp32 == 2) zinv_curl2_kernel<LL, fcomp><<<grid, NT, sm, st>>>(a);
-        else if (a.fp32) zinv_curl2_kernel<LL, float><<<grid, NT, sm, st>>>(a);
+        if (slab) launch_dep(a.dep, zinv_curl2_kernel<LL, double, true>, grid, NT, sm, st, a);
+        else if (a.fp32 == 2) launch_dep(a.dep, zinv_curl2_kernel<LL, fcomp>, grid, NT, sm, st, a);
+        else if (a.fp32) launch_dep(a.dep, zinv_curl2_kernel<LL, float>, grid, NT, sm, st, a);
         if (slab || a.fp32) return cudaGetLastError();
       }
-      zinv_curl2_kernel<LL><<<grid, NT, sm, st>>>(a);
+      launch_dep(a.dep, zinv_curl2_kernel<LL>, grid, NT, sm, st, a);
       return cudaGetLastError();
     });
   }

@@ -121,6 +121,7 @@ struct ColPassArgs {
   // Unrolled step-graph iterations: when non-null and *skip != 0 (the
   // corrector loop ended earlier in the step), the kernel returns at once.
   const int* skip = nullptr;
+  int dep = 0;  // launch_dep
 };
 
 // x pass.  Rows are (outer, inner) pairs; row r = outer * inner_n + inner
@@ -150,6 +151,7 @@ struct XPassArgs {
   // Unrolled step-graph iterations: when non-null and *skip != 0 (the
   // corrector loop ended earlier in the step), the kernel returns at once.
   const int* skip = nullptr;
+  int dep = 0;  // launch_dep
 };
 
 // x pass to physical space only (3 fields -> real [c] at row offsets
@@ -212,6 +214,7 @@ struct YProjArgs {
   const double2* tw;       // float2 table when fp32
   int fp32;                // FP32 input pass buffer and transform
   const int* skip = nullptr;  // as ColPassArgs::skip
+  int dep = 0;                // launch_dep
 };
 cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st);
 // Its work-list form for ensembles (see EnsColItem).
@@ -251,6 +254,7 @@ struct ZInvCurlArgs {
   // Unrolled step-graph iterations: when non-null and *skip != 0 (the
   // corrector loop ended earlier in the step), the kernel returns at once.
   const int* skip = nullptr;
+  int dep = 0;  // launch_dep
 };
 
 constexpr int kZTile = 8;  // y values per CTA in the Couette z passes

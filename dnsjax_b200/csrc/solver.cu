@@ -88,13 +88,14 @@ __global__ void periodic_predict_kernel(PeriodicPointArgs a,
                                         const double2* __restrict__ state,
                                         const double2* __restrict__ rhs,
                                         double2* __restrict__ out) {
+  grid_dep_sync();
   periodic_predict_body(a, state, rhs, out, blockIdx.x, gridDim.x);
 }
 
 cudaError_t launch_periodic_predict(const PeriodicPointArgs& a,
                                     const double2* state, const double2* rhs,
                                     double2* out, cudaStream_t st) {
-  periodic_predict_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(a, state, rhs, out);
+  launch_dep(a.dep, periodic_predict_kernel, kRedBlocks, kRedThreads, 0, st, a, state, rhs, out);
   return cudaGetLastError();
 }
 
@@ -128,6 +129,7 @@ __global__ void periodic_correct_kernel(PeriodicPointArgs a,
                                         const double2* __restrict__ next,
                                         double2* pred_out, double2* corr_out,
                                         double* __restrict__ partials) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   periodic_correct_body(a, pred, prev, next, pred_out, corr_out, partials, blockIdx.x,
                         gridDim.x);
@@ -139,8 +141,7 @@ cudaError_t launch_periodic_correct(const PeriodicPointArgs& a,
                                     const double2* rhs_next, double2* pred_out,
                                     double2* corr_out, double* partials,
                                     cudaStream_t st) {
-  periodic_correct_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(
-      a, pred, rhs_prev, rhs_next, pred_out, corr_out, partials);
+  launch_dep(a.dep, periodic_correct_kernel, kRedBlocks, kRedThreads, 0, st,  a, pred, rhs_prev, rhs_next, pred_out, corr_out, partials);
   return cudaGetLastError();
 }
 

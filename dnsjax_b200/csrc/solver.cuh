@@ -34,6 +34,7 @@ struct PeriodicPointArgs {
   // correct and projection kernels return at once (the work-list forms
   // ignore it).
   const int* skip = nullptr;
+  int dep = 0;  // launch_dep
 };
 
 // One member's pointwise call in an ensemble work list: predict (op 0:
@@ -108,6 +109,7 @@ struct ImmArgs {
   // Unrolled step-graph iterations (the batched pipeline): when non-null and
   // *skip != 0, every kernel of the call returns at once.
   const int* skip = nullptr;
+  int dep = 0;  // launch_dep
 };
 
 constexpr int kImmWarps = 4;  // modes per CTA (one warp each)

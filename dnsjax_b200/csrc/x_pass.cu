@@ -400,6 +400,7 @@ template <int ML, typename T = double, bool SLAB = false>
 __global__ void __launch_bounds__(XShape<ML>::NT,
                                   std::is_same<T, float>::value ? 8 : XShape<ML>::MINB)
 x_pass2_kernel(XPassArgs a) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   x_pass2_body<ML, T, SLAB>(a, blockIdx.x);
 }
@@ -447,12 +448,12 @@ cudaError_t launch_x_pass2(const XPassArgs& a, cudaStream_t st) {
     const dim3 grid((a.nrows + R - 1) / R);
     const size_t sm = a.fp32 ? XLayout<LL>::bytes / 2 : XLayout<LL>::bytes;
     if constexpr (fp32_length(LL)) {
-      if (slab) x_pass2_kernel<LL, double, true><<<grid, NT, sm, st>>>(a);
-      else if (a.fp32 == 2) x_pass2_kernel<LL, fcomp><<<grid, NT, sm, st>>>(a);
-      else if (a.fp32) x_pass2_kernel<LL, float><<<grid, NT, sm, st>>>(a);
+      if (slab) launch_dep(a.dep, x_pass2_kernel<LL, double, true>, grid, NT, sm, st, a);
+      else if (a.fp32 == 2) launch_dep(a.dep, x_pass2_kernel<LL, fcomp>, grid, NT, sm, st, a);
+      else if (a.fp32) launch_dep(a.dep, x_pass2_kernel<LL, float>, grid, NT, sm, st, a);
       if (slab || a.fp32) return cudaGetLastError();
     }
-    x_pass2_kernel<LL><<<grid, NT, sm, st>>>(a);
+    launch_dep(a.dep, x_pass2_kernel<LL>, grid, NT, sm, st, a);
     return cudaGetLastError();
   });
 }

@@ -93,6 +93,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
 template <int ML, typename T>
 __global__ void __launch_bounds__(YShape<ML>::NT, YShape<ML>::MINB)
 yfwd_project_kernel(YProjArgs a) {
+  grid_dep_sync();
   if (a.skip && *a.skip) return;
   yfwd_project_body<ML, T>(a, blockIdx.x, blockIdx.y);
 }
@@ -139,11 +140,11 @@ cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st) {
     const dim3 grid((a.NKX + SH::C - 1) / SH::C, a.NZ1);
     const size_t sm = a.fp32 ? yproj_smem<LL>() / 2 : yproj_smem<LL>();
     if constexpr (fp32_length(LL)) {
-      if (a.fp32 == 2) yfwd_project_kernel<LL, fcomp><<<grid, SH::NT, sm, st>>>(a);
-      else if (a.fp32) yfwd_project_kernel<LL, float><<<grid, SH::NT, sm, st>>>(a);
+      if (a.fp32 == 2) launch_dep(a.dep, yfwd_project_kernel<LL, fcomp>, grid, SH::NT, sm, st, a);
+      else if (a.fp32) launch_dep(a.dep, yfwd_project_kernel<LL, float>, grid, SH::NT, sm, st, a);
       if (a.fp32) return cudaGetLastError();
     }
-    yfwd_project_kernel<LL, double><<<grid, SH::NT, sm, st>>>(a);
+    launch_dep(a.dep, yfwd_project_kernel<LL, double>, grid, SH::NT, sm, st, a);
     return cudaGetLastError();
   });
 }
