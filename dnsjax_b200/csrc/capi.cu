@@ -990,7 +990,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     st.n = n;
     st.total = total;
     st.smem = ens_col_smem(maxL);
-    st.grid = rc ? 0 : ens_pass_grid(kind, st.smem, total, smax);
+    st.grid = rc ? 0 : ens_pass_grid(kind, maxL == 192, st.smem, total, smax);
     if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
     return st;
   };
@@ -1017,7 +1017,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     st.n = n;
     st.total = total;
     st.smem = ens_x_smem(maxL, maxNKX);
-    st.grid = rc ? 0 : ens_pass_grid(3, st.smem, total, smax);
+    st.grid = rc ? 0 : ens_pass_grid(3, maxL == 192, st.smem, total, smax);
     if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
     return st;
   };
@@ -1045,7 +1045,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     st.n = n;
     st.total = total;
     st.smem = ens_y_smem(maxL);
-    st.grid = rc ? 0 : ens_pass_grid(4, st.smem, total, smax);
+    st.grid = rc ? 0 : ens_pass_grid(4, maxL == 192, st.smem, total, smax);
     if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
     return st;
   };
@@ -1107,7 +1107,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   const int pgrid = std::min(n * kRedBlocks, 4 * nsm);
 
   auto run_pass = [&](const EnsStage& st, const int* act, cudaStream_t s) {
-    return launch_ens_pass(st.kind, st.items, st.base, st.n, st.total, act, st.grid, st.smem, s);
+    return launch_ens_pass(st.kind, maxL == 192, st.items, st.base, st.n, st.total, act, st.grid, st.smem, s);
   };
   auto rhs = [&](int c, const int* act, cudaStream_t s) -> cudaError_t {
     cudaError_t r;

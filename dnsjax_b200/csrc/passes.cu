@@ -124,9 +124,12 @@ col_pass_kernel(ColPassArgs a) {
 // on store); one shared buffer in between.  A CTA takes C columns with one
 // thread per stage-1 item.
 //
-// Shapes: R1 >= R2 as balanced as the register file allows (R1 <= 24 complex
-// values a thread), 16 columns (256-byte runs), 8 where 16 would leave two
-// CTAs per SM (M = 288, 384).  Against the Stockham stages with one radix <= 8
+// Shapes: one thread per stage-1 item, 16 columns (256-byte runs), 8 where 16
+// would leave two CTAs per SM (M = 288, 384).  What bounds the pass is latency at
+// the occupancy its registers allow (DRAM 32-56%, FP64 19-28% busy at M = 192),
+// so M = 192 is 12 x 16 with 24 warps per SM, not 24 x 8 with 16: 128^3 periodic
+// RHS 359 -> 344 us, Couette 128 RHS 213 -> 203 us (16 x 12: 360, 210).
+// Against the Stockham stages with one radix <= 8
 // exchange each that the lengths beyond 48, 72, 96 and 192 ran before, one
 // shared-memory round trip replaces three to five: the four column passes of a
 // 256^3 periodic RHS (M = 384) took 5.3 ms, now 2.0 ms (all the passes of a
@@ -137,11 +140,14 @@ template <int M>
 struct ColShape {
   static constexpr int R1 = ColRadix<M>::R1, R2 = ColRadix<M>::R2, C = col_columns(M);
   static constexpr int NT = R2 * C;
-  // CTAs per SM that the Couette z inverse's registers are held to
-  static constexpr int ZB = M == 36 || M == 54               ? 5
-                            : M == 108 || M == 144 || M == 162 ? 3
-                            : M == 216                         ? 2
-                                                               : 4;
+  // CTAs per SM that the registers are held to: 24 warps where at most 16 complex
+  // values a thread fit 80 registers, else 16
+  static constexpr int MINB = (R1 <= 16 && R2 <= 16 ? 768 : 512) / NT;
+  // the same for the Couette z inverse, whose curl takes more
+  static constexpr int ZB = M == 36 || M == 54                             ? 5
+                            : M == 108 || M == 144 || M == 162 || M == 192 ? 3
+                            : M == 216                                     ? 2
+                                                                           : 4;
 };
 
 size_t col_pass2_smem(int M) {
@@ -153,8 +159,9 @@ size_t col_pass2_smem(int M) {
 // OUT32 (FP32 only) an FP32 pass buffer.  CURL (inverse): `in` is the FP64
 // spectral state and field f of the 6 is u, v, w (f < 3) or the spectral
 // curl i (k x u) (triply_periodic.py:122-132), formed in FP64 at the load.
+// WIDE: the CTA has more threads than the shape's NT (the work-list kernels).
 template <int ML, int SIGN, typename T = double, bool OUT32 = false, bool CURL = false,
-          bool SLAB = false>
+          bool SLAB = false, bool WIDE = false>
 __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int by, int bz) {
   using CT = typename pass_types<T>::C;
   using RT = typename pass_types<T>::R;
@@ -175,7 +182,7 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
   const unsigned long long drop = l2_drop();
   load_twiddles(tw, reinterpret_cast<const CT*>(a.tw), M);
   __syncthreads();
-  {
+  if (!WIDE || tid < NT) {
     const int c = tid % C, j = tid / C;
     CT v[R1];
 #pragma unroll
@@ -233,7 +240,7 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
   }
   __syncthreads();
   const double sc = 1.0 / M;
-  for (int it = tid; it < R1 * C; it += NT) {
+  for (int it = tid; it < R1 * C && (!WIDE || tid < NT); it += NT) {
     const int c = it % C, k = it / C;
     CT z[R2];
 #pragma unroll
@@ -284,12 +291,11 @@ col_pass2_kernel(ColPassArgs a) {
   col_pass2_body<ML, SIGN, T, OUT32, CURL, SLAB>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// The FP64 pass held to 512 threads' worth of 128 registers per SM, so 4 CTAs
-// of 128 threads fit instead of 3 (ColPassArgs::occ4: the periodic flows'
-// column passes, measured faster so; the Couette z forward at 192 measured
-// slower, the lengths compiled for FP64 alone take it always).
+// The FP64 pass with its registers held to ColShape::MINB CTAs per SM
+// (ColPassArgs::occ4: the periodic flows' column passes; the lengths compiled for
+// FP64 alone take it always).
 template <int ML, int SIGN, bool CURL>
-__global__ void __launch_bounds__(ColShape<ML>::NT, 512 / ColShape<ML>::NT)
+__global__ void __launch_bounds__(ColShape<ML>::NT, ColShape<ML>::MINB)
 col_pass2_occ4_kernel(ColPassArgs a) {
   grid_dep_sync();
   if (a.skip && *a.skip) return;
@@ -511,14 +517,16 @@ cudaError_t launch_x_pass(const XPassArgs& a, cudaStream_t st) {
 // runs the member's body on its block, so each member computes exactly what
 // its own launch computes.  Members whose `active` flag is 0 are skipped.
 // ---------------------------------------------------------------------------
-// the fp32_length lengths all run 128 threads on 16 columns
-constexpr int kEnsColThreads = ColShape<192>::NT;
-static_assert(ColShape<48>::NT == kEnsColThreads && ColShape<72>::NT == kEnsColThreads &&
-                  ColShape<96>::NT == kEnsColThreads,
-              "one CTA shape for every member");
+// CTAs of the widest member's shape: 256 threads where a member is 192 long,
+// else 128.
+constexpr int ens_col_threads(bool wide) { return wide ? ColShape<192>::NT : ColShape<96>::NT; }
+static_assert(ColShape<48>::NT == ens_col_threads(false) &&
+                  ColShape<72>::NT == ens_col_threads(false) &&
+                  ens_col_threads(true) >= ens_col_threads(false),
+              "a CTA shape for every member");
 
-template <int SIGN, bool CURL>
-__global__ void __launch_bounds__(kEnsColThreads)
+template <int SIGN, bool CURL, bool WIDE>
+__global__ void __launch_bounds__(ens_col_threads(WIDE))
 ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict__ base, int n,
                      int total, const int* __restrict__ active) {
   __shared__ int s_k;
@@ -532,10 +540,12 @@ ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict
       const int local = vb - base[k], gx = items[k].gx, gy = items[k].gy;
       const int bx = local % gx, by = (local / gx) % gy, bz = local / (gx * gy);
       switch (a.plan.L) {
-        case 48: col_pass2_body<48, SIGN, double, false, CURL>(a, bx, by, bz); break;
-        case 72: col_pass2_body<72, SIGN, double, false, CURL>(a, bx, by, bz); break;
-        case 96: col_pass2_body<96, SIGN, double, false, CURL>(a, bx, by, bz); break;
-        default: col_pass2_body<192, SIGN, double, false, CURL>(a, bx, by, bz); break;
+        case 48: col_pass2_body<48, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
+        case 72: col_pass2_body<72, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
+        case 96: col_pass2_body<96, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
+        default:
+          if constexpr (WIDE) col_pass2_body<192, SIGN, double, false, CURL>(a, bx, by, bz);
+          break;
       }
     }
     __syncthreads();  // shared memory and s_k are reused by the next block
@@ -553,24 +563,35 @@ int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy) 
 
 size_t ens_col_smem(int maxL) { return col_pass2_smem(maxL); }
 
-// kind 0: inverse with the curl, 1: inverse, 2: forward (col_pass2); 3: x pass.
-static const void* ens_kernel(int kind) {
+// kind 0: inverse with the curl, 1: inverse, 2: forward (col_pass2); 3: x pass;
+// 4: y forward with the projection.  wide: a member is 192 long.
+static const void* ens_kernel(int kind, bool wide) {
   switch (kind) {
-    case 0: return (const void*)ens_col_pass2_kernel<1, true>;
-    case 1: return (const void*)ens_col_pass2_kernel<1, false>;
-    case 2: return (const void*)ens_col_pass2_kernel<-1, false>;
+    case 0:
+      return wide ? (const void*)ens_col_pass2_kernel<1, true, true>
+                  : (const void*)ens_col_pass2_kernel<1, true, false>;
+    case 1:
+      return wide ? (const void*)ens_col_pass2_kernel<1, false, true>
+                  : (const void*)ens_col_pass2_kernel<1, false, false>;
+    case 2:
+      return wide ? (const void*)ens_col_pass2_kernel<-1, false, true>
+                  : (const void*)ens_col_pass2_kernel<-1, false, false>;
     case 3: return ens_x_kernel();
     default: return ens_y_kernel();
   }
 }
 
+static int ens_threads(int kind, bool wide) {
+  return kind == 3 ? kEnsXThreads : kind == 4 ? kEnsYThreads : ens_col_threads(wide);
+}
+
 // Persistent grid of a work-list pass kernel: resident CTAs per SM x SMs,
 // at most `total`; also raises the kernel's dynamic shared-memory limit.
-int ens_pass_grid(int kind, size_t smem, int total, int max_smem) {
-  const void* f = ens_kernel(kind);
+int ens_pass_grid(int kind, bool wide, size_t smem, int total, int max_smem) {
+  const void* f = ens_kernel(kind, wide);
   if (allow_dynamic_smem(f, max_smem) != cudaSuccess) return 0;
   int per_sm = 0, dev = 0, nsm = 0;
-  const int threads = kind == 3 ? kEnsXThreads : kind == 4 ? kEnsYThreads : kEnsColThreads;
+  const int threads = ens_threads(kind, wide);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess)
     return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -580,29 +601,13 @@ int ens_pass_grid(int kind, size_t smem, int total, int max_smem) {
   return g < total ? g : total;
 }
 
-cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n, int total,
-                            const int* active, int grid, size_t smem, cudaStream_t st) {
-  switch (kind) {
-    case 0:
-      ens_col_pass2_kernel<1, true><<<grid, kEnsColThreads, smem, st>>>(
-          static_cast<const EnsColItem*>(items), base, n, total, active);
-      break;
-    case 1:
-      ens_col_pass2_kernel<1, false><<<grid, kEnsColThreads, smem, st>>>(
-          static_cast<const EnsColItem*>(items), base, n, total, active);
-      break;
-    case 2:
-      ens_col_pass2_kernel<-1, false><<<grid, kEnsColThreads, smem, st>>>(
-          static_cast<const EnsColItem*>(items), base, n, total, active);
-      break;
-    case 4:
-      return launch_ens_y(static_cast<const EnsYItem*>(items), base, n, total, active, grid,
+cudaError_t launch_ens_pass(int kind, bool wide, const void* items, const int* base, int n,
+                            int total, const int* active, int grid, size_t smem,
+                            cudaStream_t st) {
+  // every kernel's parameters are (items, base, n, total, active)
+  void* args[] = {&items, &base, &n, &total, &active};
+  return cudaLaunchKernel(ens_kernel(kind, wide), dim3(grid), dim3(ens_threads(kind, wide)), args,
                           smem, st);
-    default:
-      return launch_ens_x(static_cast<const EnsXItem*>(items), base, n, total, active, grid,
-                          smem, st);
-  }
-  return cudaGetLastError();
 }
 
 // x pass to physical values only (spec_to_phys of 3 fields).
@@ -1139,7 +1144,8 @@ __device__ __forceinline__ void zinv2_fill(const ZInvCurlArgs& a, CT* X,
 // read, and the curl's fill computed, in FP64.
 template <int ML, typename T = double, bool SLAB = false>
 __global__ void __launch_bounds__(ColShape<ML>::NT,
-                                  std::is_same<T, float>::value ? 6 : ColShape<ML>::ZB)
+                                  std::is_same<T, float>::value ? 768 / ColShape<ML>::NT
+                                                              : ColShape<ML>::ZB)
 zinv_curl2_kernel(ZInvCurlArgs a) {
   grid_dep_sync();
   if (a.skip && *a.skip) return;

@@ -66,7 +66,7 @@ DNSB_COL_RADIX(96, 12, 8)
 DNSB_COL_RADIX(108, 12, 9)
 DNSB_COL_RADIX(144, 12, 12)
 DNSB_COL_RADIX(162, 18, 9)
-DNSB_COL_RADIX(192, 24, 8)
+DNSB_COL_RADIX(192, 12, 16)
 DNSB_COL_RADIX(216, 18, 12)
 DNSB_COL_RADIX(288, 24, 12)
 DNSB_COL_RADIX(384, 24, 16)
@@ -226,8 +226,6 @@ constexpr int kEnsYThreads = 192;
 int ens_y_blocks(const YProjArgs& a, int* gx);
 size_t ens_y_smem(int maxL);
 const void* ens_y_kernel();
-cudaError_t launch_ens_y(const EnsYItem* items, const int* base, int n, int total,
-                         const int* active, int grid, size_t smem, cudaStream_t st);
 cudaError_t set_yfwd_project_attributes(int max_smem);
 
 // Couette first inverse pass (z), FD curl fused: spectral
@@ -297,8 +295,6 @@ int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy);
 int ens_x_blocks(const XPassArgs& a);
 constexpr int kEnsXThreads = 96;
 const void* ens_x_kernel();
-cudaError_t launch_ens_x(const EnsXItem* items, const int* base, int n, int total,
-                         const int* active, int grid, size_t smem, cudaStream_t st);
 // Item of virtual block vb: the last k with base[k] <= vb.
 __device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int vb) {
   int lo = 0, hi = n - 1;
@@ -312,10 +308,12 @@ __device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int
 size_t ens_col_smem(int maxL);
 size_t ens_x_smem(int maxL, int maxNKX);
 // kind 0: inverse pass with the spectral curl, 1: inverse, 2: forward
-// (column passes); 3: the x pass; 4: the y forward pass with the projection.  base[k]: first virtual block of item k.
-int ens_pass_grid(int kind, size_t smem, int total, int max_smem);
-cudaError_t launch_ens_pass(int kind, const void* items, const int* base, int n, int total,
-                            const int* active, int grid, size_t smem, cudaStream_t st);
+// (column passes); 3: the x pass; 4: the y forward pass with the projection.
+// wide: a member's padded length is 192.  base[k]: first virtual block of item k.
+int ens_pass_grid(int kind, bool wide, size_t smem, int total, int max_smem);
+cudaError_t launch_ens_pass(int kind, bool wide, const void* items, const int* base, int n,
+                            int total, const int* active, int grid, size_t smem,
+                            cudaStream_t st);
 cudaError_t launch_x_phys(const XPhysArgs& a, cudaStream_t st);
 // Forward x pass from physical rows (uses XPhysArgs with in_fs = spectral
 // field stride, out_fs = physical field stride).

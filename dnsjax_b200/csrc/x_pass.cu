@@ -486,10 +486,4 @@ size_t ens_x_smem(int maxL, int maxNKX) {
 
 const void* ens_x_kernel() { return (const void*)ens_x_pass2_kernel; }
 
-cudaError_t launch_ens_x(const EnsXItem* items, const int* base, int n, int total,
-                         const int* active, int grid, size_t smem, cudaStream_t st) {
-  ens_x_pass2_kernel<<<grid, kEnsXThreads, smem, st>>>(items, base, n, total, active);
-  return cudaGetLastError();
-}
-
 }  // namespace dnsb

@@ -21,7 +21,8 @@ namespace {
 template <int M>
 struct YShape {
   static constexpr int C = 8;
-  static constexpr int R1 = ColRadix<M>::R1, R2 = ColRadix<M>::R2;
+  // 192: 24 x 8, so that three components of 8 columns are 192 threads
+  static constexpr int R1 = M == 192 ? 24 : ColRadix<M>::R1, R2 = M / R1;
   static constexpr int NF = R2 * C, NT = 3 * NF;
   // registers: R1 <= 24 complex values a thread
   static constexpr int MINB = NT <= 192 ? 2 : 1;
@@ -157,12 +158,6 @@ int ens_y_blocks(const YProjArgs& a, int* gx) {
 size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192>::C); }
 
 const void* ens_y_kernel() { return (const void*)ens_yfwd_project_kernel; }
-
-cudaError_t launch_ens_y(const EnsYItem* items, const int* base, int n, int total,
-                         const int* active, int grid, size_t smem, cudaStream_t st) {
-  ens_yfwd_project_kernel<<<grid, kEnsYThreads, smem, st>>>(items, base, n, total, active);
-  return cudaGetLastError();
-}
 
 cudaError_t set_yfwd_project_attributes(int max_smem) {
   cudaError_t e = cudaSuccess;
