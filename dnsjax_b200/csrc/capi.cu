@@ -337,6 +337,9 @@ static ColPassArgs periodic_ycurl(const dnsb_periodic* p, const void* state) {
   yc.ky = p->ky;
   yc.kz = p->kz;
   yc.occ4 = 1;  // measured faster at 4 CTAs per SM
+  // beyond a few waves of blocks (128^3 RHS 359 -> 347 us, 256^3 3285 -> 3193; a
+  // 32^3 step took 174 -> 177 us so)
+  yc.fields_fast = (long long)p->NKX * p->NZ1 >= 4096;
   return yc;
 }
 

@@ -299,7 +299,10 @@ __global__ void __launch_bounds__(ColShape<ML>::NT, ColShape<ML>::MINB)
 col_pass2_occ4_kernel(ColPassArgs a) {
   grid_dep_sync();
   if (a.skip && *a.skip) return;
-  col_pass2_body<ML, SIGN, double, false, CURL, false>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+  if (CURL && a.fields_fast)
+    col_pass2_body<ML, SIGN, double, false, CURL, false>(a, blockIdx.y, blockIdx.z, blockIdx.x);
+  else
+    col_pass2_body<ML, SIGN, double, false, CURL, false>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
@@ -342,9 +345,10 @@ cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
           launch_dep(a.dep, col_pass2_kernel<LL, -1>, g2, NT, sm2, st, a);
         if (slab || a.fp32 || !a.occ4) return cudaGetLastError();
       }
-      if (a.curl)
-        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, true>, g2, NT, sm2, st, a);
-      else if (a.inverse)
+      if (a.curl) {
+        const dim3 gf = a.fields_fast ? dim3(g2.z, g2.x, g2.y) : g2;
+        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, true>, gf, NT, sm2, st, a);
+      } else if (a.inverse)
         launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, false>, g2, NT, sm2, st, a);
       else
         launch_dep(a.dep, col_pass2_occ4_kernel<LL, -1, false>, g2, NT, sm2, st, a);

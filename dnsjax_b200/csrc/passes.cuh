@@ -113,6 +113,9 @@ struct ColPassArgs {
   const double* kx;
   const double* ky;
   const double* kz;
+  // curl, occ4: the blocks of a column tile's six fields next to one another, so
+  // that the components that several fields read come from L2
+  int fields_fast;
   int occ4;  // FP64 two-stage pass held to 4 CTAs per SM (always beyond fp32_length)
   // Slab store (inverse, FP64 two-stage pass): position t goes to
   // slab.buf[t / blk] + f*fs + o*out_os + (t % blk)*ts + off + i, instead of
