@@ -1165,7 +1165,7 @@ zinv_curl2_kernel(ZInvCurlArgs a) {
   const int tid = threadIdx.x;
   const int NZ1 = a.NZ1, NKX = a.NKX, Ny = a.Ny;
   const long long ncol = (long long)NKX * Ny;
-  const long long q0 = (long long)blockIdx.x * C;
+  const long long q0 = (long long)(a.fields_fast ? blockIdx.y : blockIdx.x) * C;
   const int nq = (int)min((long long)C, ncol - q0);
   const long long cs = (long long)NZ1 * ncol;
   for (int i = tid; i < M; i += NT) cp_async_elem(tw + i, gtw + i);
@@ -1179,13 +1179,12 @@ zinv_curl2_kernel(ZInvCurlArgs a) {
   const double2* U = a.u + (long long)ix * Ny;
   const double2* V = U + cs;
   const double2* Wc = U + 2 * cs;
-  const int nf = a.curl ? 6 : 3;
   const long long fs = (long long)M * ncol;
   // Half of the pass buffer's lines stay in L2 for the x pass that reads
   // them next (all of them would not fit beside the rest).
   const unsigned long long keep = l2_keep_half();
-  // the fields of this CTA: blockIdx.y, blockIdx.y + gridDim.y, ...
-  for (int f = blockIdx.y; f < nf; f += gridDim.y) {
+  const int f = a.fields_fast ? blockIdx.x : blockIdx.y;  // one field per CTA
+  {
     switch (f) {
       case 0: zinv2_fill<M, 0>(a, X, U, V, Wc, ncol, y, kx, live); break;
       case 1: zinv2_fill<M, 1>(a, X, U, V, Wc, ncol, y, kx, live); break;
@@ -1235,7 +1234,6 @@ zinv_curl2_kernel(ZInvCurlArgs a) {
         }
       }
     }
-    __syncthreads();  // X is refilled by the next field
   }
 }
 
@@ -1248,8 +1246,8 @@ cudaError_t launch_zinv_curl(const ZInvCurlArgs& a, int span_max,
     if (a.fp32 && !fp32_length(L)) return cudaErrorInvalidValue;
     const long long ncol = (long long)a.NKX * a.Ny;
     const int C = col_columns(L);
-    // one field per CTA along y
-    const dim3 grid((unsigned)((ncol + C - 1) / C), a.curl ? 6 : 3);
+    const unsigned tiles = (unsigned)((ncol + C - 1) / C), nf = a.curl ? 6 : 3;
+    const dim3 grid = a.fields_fast ? dim3(nf, tiles) : dim3(tiles, nf);
     const size_t sm = a.fp32 ? zinv_curl2_smem(L) / 2 : zinv_curl2_smem(L);
     return with_length(L, [&](auto len) {
       constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;

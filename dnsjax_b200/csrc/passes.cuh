@@ -238,6 +238,7 @@ struct ZInvCurlArgs {
   double2* out;
   int NZ1, NKX, Ny;
   int curl;
+  int fields_fast;     // two-stage pass: as ColPassArgs::fields_fast (any field count)
   int s1;              // D1 stencil width (p + 1)
   const int* d1_j0;    // [Ny]
   const double* d1_w;  // [Ny][s1]
