@@ -290,7 +290,7 @@ static ColPassArgs periodic_zinv(const dnsb_periodic* p) {
   a.inverse = 1;
   a.plan = p->pz;
   a.tw = p->twz;
-  a.occ4 = 1;  // measured faster at 4 CTAs per SM
+  a.occ4 = 1;
   return a;
 }
 
@@ -310,7 +310,7 @@ static ColPassArgs periodic_zfwd(const dnsb_periodic* p) {
   a.inverse = 0;
   a.plan = p->pz;
   a.tw = p->twz;
-  a.occ4 = 1;  // measured faster at 4 CTAs per SM
+  a.occ4 = 1;
   return a;
 }
 
@@ -336,7 +336,7 @@ static ColPassArgs periodic_ycurl(const dnsb_periodic* p, const void* state) {
   yc.kx = p->kx;
   yc.ky = p->ky;
   yc.kz = p->kz;
-  yc.occ4 = 1;  // measured faster at 4 CTAs per SM
+  yc.occ4 = 1;
   // beyond a few waves of blocks (128^3 RHS 359 -> 347 us, 256^3 3285 -> 3193; a
   // 32^3 step took 174 -> 177 us so)
   yc.fields_fast = (long long)p->NKX * p->NZ1 >= 4096;
@@ -383,7 +383,7 @@ static ColPassArgs periodic_yfwd_col(const dnsb_periodic* p, void* rhs) {
   yc.inverse = 0;
   yc.plan = p->py;
   yc.tw = p->twy;
-  yc.occ4 = 1;  // measured faster at 4 CTAs per SM
+  yc.occ4 = 1;
   return yc;
 }
 

@@ -21,7 +21,10 @@
 // block of substitution steps are one bulk copy and every result row one
 // coalesced store.  (As [mode][y], which the kernels ran on before, each lane's
 // 16 bytes were a sector of their own, read and written twice per solve: the
-// L_k / H_k launches took 38 / 68 us at 128 x 129 x 128.)  The stage kernels
+// L_k / H_k launches took 38 / 68 us at 128 x 129 x 128, now 30 / 36.  What is
+// left is the dependent chain of a step, about 220 cycles, on a warp that has its
+// scheduler to itself; real and imaginary columns on a warp each made the whole
+// corrector slower, 201 -> 214 us.)  The stage kernels
 // transpose through shared memory, four modes (64 bytes of a row) at a time.
 //
 // The LU factors are repacked once, when the operators are bound, into
@@ -45,10 +48,9 @@ constexpr int kStageWarps = 4;  // modes per CTA in the stage kernels
 
 // L2 residency of the workspaces F and R (K Ny and 3 K Ny complex, 67 MB at
 // 128x129x128, each touched about three times per call): their writes carry an
-// evict_last policy, and their last reads (F in the gradient kernel, R in stage
-// 6) evict_first, so the streamed inputs do not push them out of the 126 MB L2
-// between the kernels of one call (l2_keep / l2_drop and the hinted accesses
-// are in common.cuh).
+// evict_last policy, and the last read of R (stage 6) evict_first, so the
+// streamed inputs do not push them out of the 126 MB L2 between the kernels of
+// one call (l2_keep / l2_drop and the hinted accesses are in common.cuh).
 
 // Tile and lane of mode m: item p on side 0, or the mirror of item p on side 1.
 struct ModeSlot {
@@ -134,7 +136,10 @@ cudaError_t launch_imm_repack(const double* ab, const int* piv, int Ny, int kl, 
 // ([o][W][32 lanes], zero outside the stencil), so rows whose stencils are
 // shifted at the walls run the same code.  YM is odd, so lanes YM rows apart
 // read without bank conflicts.  All rows live in place in 7 Ny complex values a
-// mode (3 CTAs per SM at 129 rows): Q_u, Q_v, Q_w over N, f over d.
+// mode (3 CTAs per SM at 129 rows): Q_u, Q_v, Q_w over N, f over d.  Bound by
+// latency and the weights' L1 reads: 71 us cold at 128 x 129 x 128 for 33 us of
+// memory time (72 with one read per tap and row-major workspaces; 80 with the
+// window in registers, 55 against 43 at 96 x 193 x 72).
 // ---------------------------------------------------------------------------
 // Values per mode in shared memory: 7 Ny, rounded so that the four modes of a
 // row fall on other banks when the CTA writes it out.

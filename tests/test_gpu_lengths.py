@@ -104,3 +104,32 @@ def test_unrolled_step_graph_lengths(system):
         g.launch()
         assert g.status() == (c, e)
         assert bool((s_graph == s_host).all())
+
+
+def test_worklist_ensemble_with_192():
+    """Work-list ensembles with members that are 192 long on one axis beside
+    shorter ones (the wider CTAs of the column kernels): each member's step
+    graph's states bit for bit."""
+    import torch
+
+    from dnsjax_b200 import initial
+    from dnsjax_b200.ensemble import Ensemble
+    from dnsjax_b200.flows.monochromatic import TriplyPeriodicFlow
+    from dnsjax_b200.parameters import Parameters
+
+    flows, fields = [], []
+    for s, g in enumerate([(32, 128, 48), (64, 48, 128), (128, 32, 32), (48, 64, 64)]):
+        p = Parameters(phys=dict(system="kolmogorov", re=50.0), geo=dict(lx=2 * pi, lz=2 * pi),
+                       res=dict(nx=g[0], ny=g[1], nz=g[2]),
+                       step=dict(dt=0.01, corrector_tolerance=1e-10))
+        flows.append(TriplyPeriodicFlow(p, ly=2 * pi))
+        fields.append(initial.periodic_field(*g, 2 * pi, 2 * pi, 2 * pi, s,
+                                             initial.kolmogorov_spectrum_cfg0, 1e-2))
+    a = Ensemble(flows, [dev(u) for u in fields], worklist=True)
+    b = Ensemble(flows, [dev(u) for u in fields], graphs=True)
+    for _ in range(2):
+        assert a.step().corrector_iterations == b.step().corrector_iterations
+    for x, y in zip(a.states, b.states):
+        assert torch.equal(x, y)
+    a.close()
+    b.close()
