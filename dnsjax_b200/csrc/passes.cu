@@ -581,12 +581,12 @@ static const void* ens_kernel(int kind, bool wide) {
       return wide ? (const void*)ens_col_pass2_kernel<-1, false, true>
                   : (const void*)ens_col_pass2_kernel<-1, false, false>;
     case 3: return ens_x_kernel();
-    default: return ens_y_kernel();
+    default: return ens_y_kernel(wide);
   }
 }
 
 static int ens_threads(int kind, bool wide) {
-  return kind == 3 ? kEnsXThreads : kind == 4 ? kEnsYThreads : ens_col_threads(wide);
+  return kind == 3 ? kEnsXThreads : kind == 4 ? ens_y_threads(wide) : ens_col_threads(wide);
 }
 
 // Persistent grid of a work-list pass kernel: resident CTAs per SM x SMs,

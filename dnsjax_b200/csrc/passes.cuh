@@ -116,7 +116,7 @@ struct ColPassArgs {
   // curl, occ4: the blocks of a column tile's six fields next to one another, so
   // that the components that several fields read come from L2
   int fields_fast;
-  int occ4;  // FP64 two-stage pass held to 4 CTAs per SM (always beyond fp32_length)
+  int occ4;  // FP64 two-stage pass with its registers held (always beyond fp32_length)
   // Slab store (inverse, FP64 two-stage pass): position t goes to
   // slab.buf[t / blk] + f*fs + o*out_os + (t % blk)*ts + off + i, instead of
   // out + f*out_fs + o*out_os + t*out_ts + i.
@@ -225,10 +225,10 @@ struct EnsYItem {
   YProjArgs a;
   int L, gx, member;
 };
-constexpr int kEnsYThreads = 192;
 int ens_y_blocks(const YProjArgs& a, int* gx);
 size_t ens_y_smem(int maxL);
-const void* ens_y_kernel();
+int ens_y_threads(bool wide);
+const void* ens_y_kernel(bool wide);
 cudaError_t set_yfwd_project_attributes(int max_smem);
 
 // Couette first inverse pass (z), FD curl fused: spectral

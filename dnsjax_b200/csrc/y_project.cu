@@ -18,20 +18,25 @@ namespace {
 
 // Radices (M = R1 R2) of the column pass; 8 columns, so NF threads per
 // component and R1 items per thread group of R2.
-template <int M>
+template <int M, typename T>
 struct YShape {
-  static constexpr int C = 8;
-  // 192: 24 x 8, so that three components of 8 columns are 192 threads
-  static constexpr int R1 = M == 192 ? 24 : ColRadix<M>::R1, R2 = M / R1;
+  static constexpr int C = 8;  // of every length and type
+  static constexpr bool F32 = !std::is_same_v<T, double>;
+  // FP32 at 192: 24 x 8 in 192 threads (128^3 RHS 213.8 us; 12 x 16: 215.6)
+  static constexpr int R1 = F32 && M == 192 ? 24 : ColRadix<M>::R1, R2 = M / R1;
   static constexpr int NF = R2 * C, NT = 3 * NF;
-  // registers: R1 <= 24 complex values a thread
-  static constexpr int MINB = NT <= 192 ? 2 : 1;
+  // registers: 24 warps per SM where at most 16 FP64 values a thread fit 80 of
+  // them and the CTA is not small anyway (192 points against 12 warps of 24 x 8:
+  // 128^3 RHS 328.1 -> 320.2 us; 108 points: 96 x 72 x 144 RHS 179.5 -> 176.8 us;
+  // at 72 points 90 registers are better, 48 x 48 x 96 RHS 55.4 us against 56.1)
+  static constexpr int MINB = NT <= 192 ? 2 : !F32 && R1 <= 16 ? 768 / NT : 1;
 };
 
-template <int ML, typename T>
+// WIDE: the CTA has more threads than the shape's NT (the work-list kernel).
+template <int ML, typename T, bool WIDE = false>
 __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, int iz) {
   using CT = typename pass_types<T>::C;
-  using SH = YShape<ML>;
+  using SH = YShape<ML, T>;
   constexpr int M = ML, R1 = SH::R1, R2 = SH::R2, C = SH::C, NF = SH::NF, NT = SH::NT;
   extern __shared__ double2 sm_[];
   CT* sm = reinterpret_cast<CT*>(sm_);  // [component][t][C]
@@ -42,7 +47,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
   const int ni = min(C, NKX - i0);
   CT* X = sm + f * M * C;
   const long long row = (long long)NZ1 * NKX;  // stride of y
-  {
+  if (!WIDE || tid < NT) {
     const int c = t0 % C, j = t0 / C;
     const CT* in = reinterpret_cast<const CT*>(a.in) + (long long)f * M * row +
                    (long long)iz * NKX + i0 + c;
@@ -56,7 +61,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
     for (int i = 0; i < R1; ++i) X[(j * R1 + i) * C + c] = v[i];
   }
   __syncthreads();
-  for (int it = t0; it < R1 * C; it += NF) {
+  for (int it = t0; it < R1 * C && (!WIDE || tid < NT); it += NF) {
     const int c = it % C, k = it / C;
     CT z[R2];
 #pragma unroll
@@ -72,7 +77,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
   const double sc = 1.0 / M;
   const double kz = a.kz[iz];
   const long long cs = (long long)NY1 * row;
-  for (int idx = tid; idx < NY1 * C; idx += NT) {
+  for (int idx = tid; idx < NY1 * C && (!WIDE || tid < NT); idx += NT) {
     const int c = idx % C, s = idx / C;
     if (c >= ni) continue;
     const int t = stored_to_pos(s, NY1, M) * C + c;
@@ -92,7 +97,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
 }
 
 template <int ML, typename T>
-__global__ void __launch_bounds__(YShape<ML>::NT, YShape<ML>::MINB)
+__global__ void __launch_bounds__(YShape<ML, T>::NT, YShape<ML, T>::MINB)
 yfwd_project_kernel(YProjArgs a) {
   grid_dep_sync();
   if (a.skip && *a.skip) return;
@@ -100,10 +105,14 @@ yfwd_project_kernel(YProjArgs a) {
 }
 
 // Work-list form for ensembles: as ens_x_pass2_kernel (csrc/x_pass.cu).
-static_assert(YShape<48>::NT == kEnsYThreads && YShape<72>::NT == kEnsYThreads &&
-                  YShape<96>::NT == kEnsYThreads && YShape<192>::NT == kEnsYThreads,
-              "one CTA shape for every member");
-__global__ void __launch_bounds__(kEnsYThreads)
+constexpr int ens_y_shape(bool wide) {
+  return wide ? YShape<192, double>::NT : YShape<96, double>::NT;
+}
+static_assert(YShape<48, double>::NT == ens_y_shape(false) &&
+                  YShape<72, double>::NT == ens_y_shape(false),
+              "a CTA shape for every member");
+template <bool WIDE>
+__global__ void __launch_bounds__(ens_y_shape(WIDE))
 ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restrict__ base, int n,
                         int total, const int* __restrict__ active) {
   __shared__ int s_k;
@@ -116,10 +125,12 @@ ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restric
       const YProjArgs a = items[k].a;
       const int gx = items[k].gx, bx = (vb - base[k]) % gx, iz = (vb - base[k]) / gx;
       switch (items[k].L) {
-        case 48: yfwd_project_body<48, double>(a, bx, iz); break;
-        case 72: yfwd_project_body<72, double>(a, bx, iz); break;
-        case 96: yfwd_project_body<96, double>(a, bx, iz); break;
-        default: yfwd_project_body<192, double>(a, bx, iz); break;
+        case 48: yfwd_project_body<48, double, WIDE>(a, bx, iz); break;
+        case 72: yfwd_project_body<72, double, WIDE>(a, bx, iz); break;
+        case 96: yfwd_project_body<96, double, WIDE>(a, bx, iz); break;
+        default:
+          if constexpr (WIDE) yfwd_project_body<192, double>(a, bx, iz);
+          break;
       }
     }
     __syncthreads();
@@ -128,7 +139,7 @@ ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restric
 
 template <int ML>
 constexpr size_t yproj_smem() {
-  return sizeof(double2) * (size_t)(3 * ML * YShape<ML>::C);
+  return sizeof(double2) * (size_t)(3 * ML * YShape<ML, double>::C);
 }
 
 }  // namespace
@@ -137,27 +148,32 @@ cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st) {
   if (a.fp32 && !fp32_length(L)) return cudaErrorInvalidValue;
   return with_length(L, [&](auto len) {
     constexpr int LL = decltype(len)::value;
-    using SH = YShape<LL>;
-    const dim3 grid((a.NKX + SH::C - 1) / SH::C, a.NZ1);
+    const dim3 grid((a.NKX + YShape<LL, double>::C - 1) / YShape<LL, double>::C, a.NZ1);
     const size_t sm = a.fp32 ? yproj_smem<LL>() / 2 : yproj_smem<LL>();
     if constexpr (fp32_length(LL)) {
-      if (a.fp32 == 2) launch_dep(a.dep, yfwd_project_kernel<LL, fcomp>, grid, SH::NT, sm, st, a);
-      else if (a.fp32) launch_dep(a.dep, yfwd_project_kernel<LL, float>, grid, SH::NT, sm, st, a);
+      constexpr int NT = YShape<LL, float>::NT;
+      if (a.fp32 == 2) launch_dep(a.dep, yfwd_project_kernel<LL, fcomp>, grid, NT, sm, st, a);
+      else if (a.fp32) launch_dep(a.dep, yfwd_project_kernel<LL, float>, grid, NT, sm, st, a);
       if (a.fp32) return cudaGetLastError();
     }
-    launch_dep(a.dep, yfwd_project_kernel<LL, double>, grid, SH::NT, sm, st, a);
+    launch_dep(a.dep, yfwd_project_kernel<LL, double>, grid, YShape<LL, double>::NT, sm, st, a);
     return cudaGetLastError();
   });
 }
 
 int ens_y_blocks(const YProjArgs& a, int* gx) {
-  *gx = (a.NKX + YShape<192>::C - 1) / YShape<192>::C;
+  *gx = (a.NKX + YShape<192, double>::C - 1) / YShape<192, double>::C;
   return *gx * a.NZ1;
 }
 
-size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192>::C); }
+size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192, double>::C); }
 
-const void* ens_y_kernel() { return (const void*)ens_yfwd_project_kernel; }
+int ens_y_threads(bool wide) { return ens_y_shape(wide); }
+
+const void* ens_y_kernel(bool wide) {
+  return wide ? (const void*)ens_yfwd_project_kernel<true>
+              : (const void*)ens_yfwd_project_kernel<false>;
+}
 
 cudaError_t set_yfwd_project_attributes(int max_smem) {
   cudaError_t e = cudaSuccess;
