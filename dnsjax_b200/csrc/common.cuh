@@ -683,6 +683,18 @@ __device__ __forceinline__ void st_l2(float2* g, float2 v, unsigned long long po
                "f"(v.y), "l"(pol)
                : "memory");
 }
+__device__ __forceinline__ void st_l2(double* g, double v, unsigned long long pol) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;\n" ::"l"(g), "d"(v), "l"(pol)
+               : "memory");
+}
+__device__ __forceinline__ double ld_l2(const double* g, unsigned long long pol) {
+  double v;
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;\n"
+               : "=d"(v)
+               : "l"(g), "l"(pol)
+               : "memory");
+  return v;
+}
 __device__ __forceinline__ double2 ld_l2(const double2* g, unsigned long long pol) {
   double2 v;
   asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;\n"

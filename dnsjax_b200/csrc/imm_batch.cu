@@ -24,7 +24,8 @@
 // L_k / H_k launches took 38 / 68 us at 128 x 129 x 128, now 30 / 36.  What is
 // left is the dependent chain of a step, about 220 cycles, on a warp that has its
 // scheduler to itself; real and imaginary columns on a warp each made the whole
-// corrector slower, 201 -> 214 us.)  The stage kernels
+// corrector slower, 201 -> 214 us, as the lanes' 8-byte stores were 16 apart; with
+// a warp per side, lane = (item, re or im), they are contiguous.)  The stage kernels
 // transpose through shared memory, four modes (64 bytes of a row) at a time.
 //
 // The LU factors are repacked once, when the operators are bound, into
@@ -44,6 +45,11 @@ namespace {
 
 constexpr int kTile = 16;       // items per substitution CTA (two sides per item)
 constexpr int kLanes = 2 * kTile;  // lanes of a tile row (two sides)
+constexpr int kRowDoubles = 2 * kLanes;
+// Substitution lanes of one real column: bandwidths and tiles (see solve_launch).
+template <int KL>
+constexpr int kSplitCols = KL >= 6 ? 1 : 2;
+constexpr int kSplitTiles = 148;
 constexpr int kStageWarps = 4;  // modes per CTA in the stage kernels
 
 // L2 residency of the workspaces F and R (K Ny and 3 K Ny complex, 67 MB at
@@ -457,7 +463,8 @@ imm_stage6_kernel(ImmArgs a, int paired, const double2* __restrict__ R, long lon
 // component (1 for L_k: p_P; 3 for H_k) and one copying warp; lane = (side,
 // item) (lanes 0-15 the items' own modes, 16-31 their mirrors), and each thread
 // solves both real columns (re, im) of its mode's component as two recurrences
-// sharing every factor load; the warps share the tile's factor stream.  Lane 0
+// sharing every factor load, or, on few tiles of wide bands, one of them (COLS
+// below); the warps share the tile's factor stream.  Lane 0
 // of the copying warp streams each block of steps -- its factors and pivots and,
 // per component, the right-hand-side rows that enter the windows during the
 // block, each one contiguous bulk copy -- into a ring of shared-memory slots
@@ -562,12 +569,32 @@ __device__ __forceinline__ double pivot_take(double (&w)[KL + 1], int ph, int d)
   return bpj;
 }
 
-template <int KL, int MODE, bool TAIL>
-__device__ __forceinline__ void tile_fwd_block(double2* col, int j0, int nsteps, int Ny,
-                                               double (&w)[2][KL + 1], const double2* Lp,
-                                               const int (&dr)[KL + 1], const double2* ent,
+// A lane's element of a tile row, re and im or one of them, as COLS doubles.
+__device__ __forceinline__ void put(double* g, const double (&v)[2], unsigned long long pol) {
+  st_l2(reinterpret_cast<double2*>(g), make_double2(v[0], v[1]), pol);
+}
+__device__ __forceinline__ void put(double* g, const double (&v)[1], unsigned long long pol) {
+  st_l2(g, v[0], pol);
+}
+template <int N>
+__device__ __forceinline__ void get(double (&w)[2][N], int i, const double2 v) {
+  w[0][i] = v.x;
+  w[1][i] = v.y;
+}
+template <int N>
+__device__ __forceinline__ void get(double (&w)[1][N], int i, double v) {
+  w[0][i] = v;
+}
+template <int COLS>
+using lane_elem = std::conditional_t<COLS == 2, double2, double>;
+
+template <int KL, int MODE, bool TAIL, int COLS>
+__device__ __forceinline__ void tile_fwd_block(double* col, int j0, int nsteps, int Ny,
+                                               double (&w)[COLS][KL + 1], const double2* Lp,
+                                               const int (&dr)[KL + 1], const double* ent,
                                                unsigned long long pol) {
   constexpr int W = KL + 1;
+  using E = lane_elem<COLS>;
 #pragma unroll
   for (int ph = 0; ph < W; ++ph) {
     const int j = j0 + ph;
@@ -579,27 +606,26 @@ __device__ __forceinline__ void tile_fwd_block(double2* col, int j0, int nsteps,
         L[2 * i2] = t.x;
         L[2 * i2 + 1] = t.y;
       }
-      double bp[2];
+      double bp[COLS];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) bp[c] = pivot_take<KL, MODE>(w[c], ph, dr[ph]);
-      st_l2(col + j * kLanes, make_double2(bp[0], bp[1]), pol);
+      for (int c = 0; c < COLS; ++c) bp[c] = pivot_take<KL, MODE>(w[c], ph, dr[ph]);
+      put(col + j * kRowDoubles, bp, pol);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < COLS; ++c) {
 #pragma unroll
         for (int i = 1; i <= KL; ++i) w[c][(i + ph) % W] -= L[i - 1] * bp[c];
       }
       // b[j+W] enters at offset KL (0 past the last row)
-      const double2 e = j + W < Ny ? ent[ph * kLanes] : make_double2(0.0, 0.0);
-      w[0][ph % W] = e.x;
-      w[1][ph % W] = e.y;
+      get(w, ph % W, j + W < Ny ? *reinterpret_cast<const E*>(ent + ph * kRowDoubles) : E{});
     }
   }
 }
 
-template <int NU, bool TAIL>
-__device__ __forceinline__ void tile_bwd_block(double2* col, int j0, double (&w)[2][NU + 1],
-                                               const double2* Up, const double2* ent,
+template <int NU, bool TAIL, int COLS>
+__device__ __forceinline__ void tile_bwd_block(double* col, int j0, double (&w)[COLS][NU + 1],
+                                               const double2* Up, const double* ent,
                                                unsigned long long pol) {
+  using E = lane_elem<COLS>;
   constexpr int WB = NU + 1, NUP = (NU + 2) & ~1;
 #pragma unroll
   for (int ph = 0; ph < WB; ++ph) {
@@ -614,26 +640,32 @@ __device__ __forceinline__ void tile_bwd_block(double2* col, int j0, double (&w)
         U[2 * i2 + 1] = t.y;
       }
       const int st = ((NU - ph) % WB + WB) % WB;
-      const double bj[2] = {w[0][st], w[1][st]};
-      st_l2(col + j * kLanes, make_double2(bj[0] * U[0], bj[1] * U[0]), pol);
+      double bj[COLS], x[COLS];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        bj[c] = w[c][st];
+        x[c] = bj[c] * U[0];
+      }
+      put(col + j * kRowDoubles, x, pol);
 #pragma unroll
       for (int i = 1; i <= NU; ++i) {
         const int si = ((NU - i - ph) % WB + WB) % WB;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) w[c][si] -= U[i] * bj[c];
+        for (int c = 0; c < COLS; ++c) w[c][si] -= U[i] * bj[c];
       }
       // b[j-WB] enters at offset 0 (0 below row 0); rows in ascending order
-      const double2 e = j - WB >= 0 ? ent[(WB - 1 - ph) * kLanes] : make_double2(0.0, 0.0);
-      w[0][st] = e.x;
-      w[1][st] = e.y;
+      get(w, st,
+          j - WB >= 0 ? *reinterpret_cast<const E*>(ent + (WB - 1 - ph) * kRowDoubles) : E{});
     }
   }
 }
 
 constexpr int kMaxRing = 4;
 
-template <int KL, int NU>
-__global__ void __launch_bounds__(128)
+// COLS: real columns of a lane, 2 (one warp per component, lane = (side, item)) or
+// 1 (two warps per component, one for each side, lane = (item, re or im)).
+template <int KL, int NU, int COLS>
+__global__ void __launch_bounds__(COLS == 2 ? 128 : 224)
 imm_solve_kernel(SolveArgs a) {
   if (a.skip && *a.skip) return;  // before any barrier is set up
   constexpr int W = KL + 1, WB = NU + 1, NUP = (NU + 2) & ~1;
@@ -643,8 +675,10 @@ imm_solve_kernel(SolveArgs a) {
   extern __shared__ __align__(128) unsigned char ring[];
   __shared__ __align__(8) unsigned long long full[kMaxRing], empty[kMaxRing], fwd_done;
   __shared__ int s_fail;
-  const int tid = threadIdx.x, lane = tid & 31, cw = tid >> 5;  // warp = component
-  const int it = lane & (kTile - 1);
+  constexpr int WPC = 3 - COLS;  // warps per component
+  using E = lane_elem<COLS>;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cw = warp / WPC;
+  const int it = COLS == 2 ? lane & (kTile - 1) : lane >> 1;
   const long long tile = blockIdx.x;
   const int Ny = a.Ny, R = a.ring, SB = a.slot_bytes, nc = a.ncomp;
   const int E0 = SB - nc * MW * RB;  // entering rows, at the slot's end
@@ -658,16 +692,16 @@ imm_solve_kernel(SolveArgs a) {
   if (tid == 0) {
     for (int r = 0; r < R; ++r) {
       mbar_init(&full[r], 1);
-      mbar_init(&empty[r], nc);
+      mbar_init(&empty[r], WPC * nc);
     }
-    mbar_init(&fwd_done, nc);
+    mbar_init(&fwd_done, WPC * nc);
     mbar_fence_init();
     s_fail = 0;
   }
   __syncthreads();
   volatile int* fail = &s_fail;
 
-  if (cw == nc) {
+  if (warp == WPC * nc) {
     if (lane != 0) return;
     // Blocks 0 .. nblk-1 into slot g % R: forward blocks hold the factors and
     // pivots of steps j0 .. j0+W-1 and rows j0+W .. j0+2W-1; back-substitution
@@ -710,7 +744,8 @@ imm_solve_kernel(SolveArgs a) {
   }
 
   const unsigned long long keep = l2_keep();
-  double2* col = X + cw * a.cs + lane;
+  const int at = (warp % WPC) * kLanes + lane * COLS;  // the lane's double in a tile row
+  double* col = reinterpret_cast<double*>(X + cw * a.cs) + at;
   int g = 0;
   bool ok = true;
   auto take = [&] {  // wait for block g
@@ -729,19 +764,16 @@ imm_solve_kernel(SolveArgs a) {
 
   // ---- forward elimination, steps j = 0 .. Ny-2 ----
   {
-    double w[2][W];
+    double w[COLS][W];
 #pragma unroll
-    for (int o = 0; o < W; ++o) {
-      const double2 v = (o < Ny) ? ld_l2(col + o * kLanes, keep) : make_double2(0.0, 0.0);
-      w[0][o] = v.x;
-      w[1][o] = v.y;
-    }
+    for (int o = 0; o < W; ++o)
+      get(w, o, o < Ny ? ld_l2(reinterpret_cast<const E*>(col + o * kRowDoubles), keep) : E{});
     for (int k = 0; k < nbf; ++k, ++g) {
       if (!take()) break;
       const unsigned char* slot = ring + (g % R) * SB;
       const double2* Lp = reinterpret_cast<const double2*>(slot) + it;
       const unsigned char* Ps = slot + LB;
-      const double2* ent = reinterpret_cast<const double2*>(slot + E0 + cw * MW * RB) + lane;
+      const double* ent = reinterpret_cast<const double*>(slot + E0 + cw * MW * RB) + at;
       int dr[W];
       int dm = 0;
 #pragma unroll
@@ -752,26 +784,27 @@ imm_solve_kernel(SolveArgs a) {
       dm = __reduce_max_sync(0xffffffffu, dm);
       const int j0 = k * W;
       if (j0 + W > nsteps)
-        tile_fwd_block<KL, 2, true>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
+        tile_fwd_block<KL, 2, true, COLS>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else if (dm == 0)
-        tile_fwd_block<KL, 0, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
+        tile_fwd_block<KL, 0, false, COLS>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else if (dm == 1)
-        tile_fwd_block<KL, 1, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
+        tile_fwd_block<KL, 1, false, COLS>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       else
-        tile_fwd_block<KL, 2, false>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
+        tile_fwd_block<KL, 2, false, COLS>(col, j0, nsteps, Ny, w, Lp, dr, ent, keep);
       give();
     }
     // b[Ny-1] sits at offset 0 after the last step: slot nsteps % W.
     const int last = nsteps % W;
-    double v0 = w[0][0], v1 = w[1][0];
+    double v[COLS];
 #pragma unroll
-    for (int s = 1; s < W; ++s)
-      if (last == s) {
-        v0 = w[0][s];
-        v1 = w[1][s];
-      }
+    for (int c = 0; c < COLS; ++c) {
+      v[c] = w[c][0];
+#pragma unroll
+      for (int t = 1; t < W; ++t)
+        if (last == t) v[c] = w[c][t];
+    }
     if (ok) {
-      st_l2(col + (Ny - 1) * kLanes, make_double2(v0, v1), keep);
+      put(col + (Ny - 1) * kRowDoubles, v, keep);
       // the forward results are read back by bulk copies (async proxy)
       asm volatile("fence.proxy.async;\n" ::: "memory");
       __syncwarp();
@@ -781,24 +814,22 @@ imm_solve_kernel(SolveArgs a) {
 
   // ---- back substitution, rows j = Ny-1 .. 0 ----
   if (ok) {
-    double w[2][WB];
+    double w[COLS][WB];
 #pragma unroll
     for (int o = 0; o < WB; ++o) {
       const int idx = Ny - 1 - NU + o;
-      const double2 v = (idx >= 0) ? ld_l2(col + idx * kLanes, keep) : make_double2(0.0, 0.0);
-      w[0][o] = v.x;
-      w[1][o] = v.y;
+      get(w, o, idx >= 0 ? ld_l2(reinterpret_cast<const E*>(col + idx * kRowDoubles), keep) : E{});
     }
     for (int k = 0; k < nbb; ++k, ++g) {
       if (!take()) break;
       const unsigned char* slot = ring + (g % R) * SB;
       const double2* Up = reinterpret_cast<const double2*>(slot) + it;
-      const double2* ent = reinterpret_cast<const double2*>(slot + E0 + cw * MW * RB) + lane;
+      const double* ent = reinterpret_cast<const double*>(slot + E0 + cw * MW * RB) + at;
       const int j0 = Ny - 1 - k * WB;
       if (j0 - WB + 1 < 0)
-        tile_bwd_block<NU, true>(col, j0, w, Up, ent, keep);
+        tile_bwd_block<NU, true, COLS>(col, j0, w, Up, ent, keep);
       else
-        tile_bwd_block<NU, false>(col, j0, w, Up, ent, keep);
+        tile_bwd_block<NU, false, COLS>(col, j0, w, Up, ent, keep);
       give();
     }
   }
@@ -904,10 +935,19 @@ static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, long lon
   // Never dependent on the kernel before: the one or two CTAs an SM has room for
   // would gather on the SMs that finish first (96 x 71 x 108 corrector: 97 us
   // so, 110 us with dependent substitutions).
-  if (bt.nu == KL + 1)
-    imm_solve_kernel<KL, KL + 1><<<grid, 32 * (ncomp + 1), sm, st>>>(s);
-  else
-    imm_solve_kernel<KL, 2 * KL><<<grid, 32 * (ncomp + 1), sm, st>>>(s);
+  // Real and imaginary columns on lanes of their own shorten a step's chain but
+  // run twice the warps: faster for the wide bands while every CTA has an SM to
+  // itself (corrector, kl = 6: 48 x 49 x 48 49.5 -> 45.4 us, 64 x 65 x 64 62.5 ->
+  // 59.8, 96 x 97 x 96 113.1 -> 109.3; kl = 8, 64 x 65 x 64: 70.0 -> 63.1).  On more
+  // tiles it loses (128 x 129 x 128 193.7 -> 195.1 us), as it does at kl = 4 (32 x
+  // 53 x 36 predict_and_correct 131.4 -> 133.7 us).
+  constexpr int SC = kSplitCols<KL>;
+  const bool split = SC == 1 && grid <= kSplitTiles;
+  const int threads = 32 * ((split ? 2 : 1) * ncomp + 1);
+  auto* kernel = bt.nu == KL + 1
+                     ? (split ? imm_solve_kernel<KL, KL + 1, SC> : imm_solve_kernel<KL, KL + 1, 2>)
+                     : (split ? imm_solve_kernel<KL, 2 * KL, SC> : imm_solve_kernel<KL, 2 * KL, 2>);
+  kernel<<<grid, threads, sm, st>>>(s);
   return cudaGetLastError();
 }
 
@@ -967,8 +1007,10 @@ cudaError_t set_imm_batch_attributes(int max_smem) {
   (const void*)imm_stage013_kernel<K, 3>, (const void*)imm_stage013_kernel<K, 5>,    \
       (const void*)imm_stage013_kernel<K, 7>, (const void*)imm_stage013_kernel<K, 9>, \
       (const void*)imm_stage013_kernel<K, 17>,                                       \
-      (const void*)imm_stage6_kernel<K, 0>, (const void*)imm_solve_kernel<K, K + 1>, \
-      (const void*)imm_solve_kernel<K, 2 * K>
+      (const void*)imm_stage6_kernel<K, 0>, (const void*)imm_solve_kernel<K, K + 1, 2>, \
+      (const void*)imm_solve_kernel<K, 2 * K, 2>,                       \
+      (const void*)imm_solve_kernel<K, K + 1, kSplitCols<K>>,                     \
+      (const void*)imm_solve_kernel<K, 2 * K, kSplitCols<K>>
       DNSB_IMM_FNS(2), DNSB_IMM_FNS(4), DNSB_IMM_FNS(6), DNSB_IMM_FNS(8)};
 #undef DNSB_IMM_FNS
   cudaError_t e = cudaSuccess;
