@@ -1565,11 +1565,23 @@ extern "C" size_t dnsb_couette_workspace_bytes(const dnsb_couette* p) {
   return p ? p->ws_bytes : 0;
 }
 
+// Frees the five-kernel IMM's repacked factors and workspaces.
+static void batch_free(dnsb_couette* p) {
+  void* ptrs[] = {p->fac, p->dp, p->Fw, p->Rw};
+  for (void* q : ptrs)
+    if (q) cudaFree(q);
+  p->fac = nullptr;
+  p->dp = nullptr;
+  p->Fw = p->Rw = nullptr;
+  p->batch_ready = false;
+}
+
 // Repack both operators' factors for the five-kernel IMM (items = modes
 // (s, kx), s <= (nz-1)/2, when mirror modes share factors; 16-item tiles)
 // and allocate its stage workspace; kept until the next bind or destroy.
 // Returns 0 with batch_ready false when the ring of the substitution
-// kernel does not fit in shared memory (the single-kernel IMM runs then).
+// kernel does not fit in shared memory or the factors and workspaces do not fit
+// in device memory (a single-kernel IMM, which needs neither, runs then).
 static int bind_batch(dnsb_couette* p) {
   const int kl = p->p, nu = imm_nu(kl, p->ab_row0);
   const int smax = max_smem_optin();
@@ -1580,20 +1592,19 @@ static int bind_batch(dnsb_couette* p) {
   const size_t nL = (size_t)ntiles * (p->Ny + kl + 1) * kl * tile;
   const size_t nU = (size_t)ntiles * (p->Ny + nu + 1) * ((nu + 2) & ~1) * tile;
   const size_t nP = (size_t)ntiles * (p->Ny + kl + 1) * tile;
-  void* ptrs[] = {p->fac, p->dp, p->Fw, p->Rw};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
-  p->fac = nullptr;
-  p->dp = nullptr;
-  p->Fw = p->Rw = nullptr;
   const size_t fac_bytes = 2 * (nL + nU) * sizeof(double);
-  cudaError_t e1 = cudaMalloc(&p->fac, fac_bytes);
-  cudaError_t e2 = cudaMalloc(&p->dp, 2 * nP);
   // [tile][y][32 lanes], zero in the lanes of no mode
   const size_t wbytes = (size_t)ntiles * p->Ny * 2 * tile * sizeof(double2);
-  cudaError_t e3 = cudaMalloc(&p->Fw, wbytes);
-  cudaError_t e4 = cudaMalloc(&p->Rw, 3 * wbytes);
-  if (e1 || e2 || e3 || e4) return fail(DNSB_ERR_CUDA, "IMM workspace allocation failed");
+  cudaError_t e = cudaMalloc(&p->fac, fac_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&p->dp, 2 * nP);
+  if (e == cudaSuccess) e = cudaMalloc(&p->Fw, wbytes);
+  if (e == cudaSuccess) e = cudaMalloc(&p->Rw, 3 * wbytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // not left for a later launch check
+    batch_free(p);
+    return 0;
+  }
+  if (e != cudaSuccess) return fail(DNSB_ERR_CUDA, "IMM workspace allocation failed");
   if (cudaMemset(p->fac, 0, fac_bytes) != cudaSuccess ||
       cudaMemset(p->dp, 0, 2 * nP) != cudaSuccess ||
       cudaMemset(p->Fw, 0, wbytes) != cudaSuccess ||
@@ -1674,7 +1685,7 @@ extern "C" int dnsb_couette_bind_imm(dnsb_couette* p, const dnsb_imm_ops* ops) {
   p->pair_modes = (allow && h_diff == 0) ? 1 : 0;
   p->ab_row0 = h_row;
   p->bound = true;
-  p->batch_ready = false;
+  batch_free(p);  // of an earlier bind
   if (p->w1x) {
     rc = bind_batch(p);
     if (rc) return rc;

@@ -11,6 +11,8 @@ non-finite field) and read back as a status or an exception.
   of zero polls every wait gives up at once; the call sets the status bit,
   drains its copies and returns, the context stays usable, and after the
   status is cleared and the limit restored the next call matches the oracle.
+* Operators bound where device memory does not hold the batched IMM's factors
+  and workspaces: the single-kernel form, which needs none, runs.
 * A non-finite initial field ends the run after its first step, as the
   reference's loop does (``__main__.py:125-129``: it steps while
   last_error < corrector_tolerance), through the host loop and the step
@@ -123,6 +125,50 @@ def test_imm_ring_wait_gives_up_and_recovers():
                        imm=imm)
     want = orc.predict(u0, orc.get_rhs(u0))
     assert rel_l2(got, want) < 1e-12
+
+
+def test_bind_without_memory_for_the_batched_imm(monkeypatch):
+    import torch
+
+    from dnsjax_b200 import _lib, initial
+
+    g = (96, 193, 72)  # 55 MB of repacked factors, 43 MB of workspaces
+    u = torch.as_tensor(initial.couette_field(*g, 2 * pi, pi, 4, 1, 8.0, 1e-3), device="cuda")
+
+    def predict(flow):
+        before = _lib.launch_count()
+        out = flow.predict(u, r)
+        return out, _lib.launch_count() - before
+
+    full = _couette(*g)
+    r = full.get_rhs(u)
+    assert predict(full)[1] == 5
+    full.set_variants([0, 0, 0, 2])  # the single-kernel form
+    want, n = predict(full)
+    assert n == 1
+    make, ballast = _lib.ImmOps, []
+
+    def ops_without_memory(*args):  # between the context's creation and the bind
+        torch.cuda.empty_cache()
+        ballast.append(torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8,
+                                   device="cuda"))
+        return make(*args)
+
+    monkeypatch.setattr(_lib, "ImmOps", ops_without_memory)
+    flow = _couette(*g, imm=full.imm)
+    monkeypatch.undo()
+    assert ballast
+    ballast.clear()
+    torch.cuda.empty_cache()
+    got, n = predict(flow)
+    assert n == 1 and torch.equal(got, want)
+    flow.check_status()
+    # a later bind, with the memory there, is batched again
+    ops = _lib.ImmOps(*[_lib.ptr(flow.imm[k]) for k in (
+        "Lk_ab", "Lk_piv", "Hk_ab", "Hk_piv", "v1", "v2", "q1", "q2", "M_inv")])
+    _lib.check(flow._L.dnsb_couette_bind_imm(flow._ctx, _lib.C.byref(ops)))
+    got, n = predict(flow)
+    assert n == 5 and rel_l2(got.cpu(), want.cpu()) < 1e-11
 
 
 @pytest.mark.parametrize("system", ["plane-couette", "kolmogorov"])
