@@ -12,7 +12,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "libdnsb.so"
 SOURCES = ["passes.cu", "x_pass.cu", "x_transform.cu", "y_project.cu", "solver.cu", "imm.cu",
-           "imm_batch.cu", "noalloc.cu", "precompute.cu", "learned.cu", "mlp_tc.cu", "capi.cu"]
+           "imm_batch.cu", "imm_solve_plain.cu", "noalloc.cu", "precompute.cu", "learned.cu",
+           "mlp_tc.cu", "capi.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -1542,7 +1542,7 @@ extern "C" int dnsb_couette_create(const dnsb_couette_desc* d,
     cudaError_t e = set_pass_attributes(smax);
     if (e == cudaSuccess) e = set_solver_attributes(smax);
     if (e == cudaSuccess) e = set_imm_v2_attributes(smax);
-    if (e == cudaSuccess) e = set_imm_batch_attributes(smax);
+    if (e == cudaSuccess) e = set_imm_batch_attributes(smax, p->Ny);
     if (e != cudaSuccess)
       rc = fail(DNSB_ERR_CUDA, std::string("cudaFuncSetAttribute: ") +
                                    cudaGetErrorString(e));
@@ -1618,8 +1618,8 @@ static int bind_batch(dnsb_couette* p) {
     double* fU = fL + nL;
     unsigned char* d = p->dp + k * nP;
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (launch_imm_repack(abs_[k], pivs[k], p->Ny, kl, nu, p->ab_row0, NP, ntiles, fL, fU, d,
-                          p->status, 0) != cudaSuccess)
+    if (launch_imm_repack(abs_[k], pivs[k], p->Ny, kl, nu, p->ab_row0, NP,
+                          imm_batch_scaled(p->Ny), fL, fU, d, p->status, 0) != cudaSuccess)
       return fail(DNSB_ERR_CUDA, "IMM repack launch failed");
     b.facL[k] = fL;
     b.facU[k] = fU;

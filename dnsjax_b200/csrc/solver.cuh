@@ -139,7 +139,7 @@ cudaError_t launch_ab_pair_check(const double* ab, const int* piv, int nz1,
                                  cudaStream_t st);
 
 // Five-kernel IMM iteration (csrc/imm_batch.cu) over factors repacked at
-// bind time (record-major, item index fastest; 1/U_jj and U/U_jj pre-scaled;
+// bind time (record-major, item index fastest; 1/U_jj, and U over U_jj or plain;
 // pivots as validated offsets) and workspace F [tiles][Ny][32], R [3][tiles][Ny][32].
 struct ImmBatch {
   // per operator (0 = L_k, 1 = H_k), 16-item tiles (csrc/imm_batch.cu)
@@ -217,14 +217,15 @@ void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const in
                        std::vector<double>* w2x);
 int imm_nu(int kl, int row0);
 bool imm_batch_fits(int kl, int nu, int max_smem);
+bool imm_batch_scaled(int Ny);  // facU holds U over U_jj
 cudaError_t launch_imm_repack(const double* ab, const int* piv, int Ny, int kl, int nu,
-                              int row0, int NP, int ntiles, double* facL, double* facU,
+                              int row0, int NP, int scaled, double* facL, double* facU,
                               unsigned char* dp, int* status, cudaStream_t st);
 cudaError_t launch_imm_batch(const ImmArgs& a, const ImmBatch& bt, const double2* vel_n,
                              const double2* vel_j, const double2* nl_n,
                              const double2* nl_j, double2* vel_new, double2* corr_out,
                              double* partials, cudaStream_t st);
-cudaError_t set_imm_batch_attributes(int max_smem);
+cudaError_t set_imm_batch_attributes(int max_smem, int Ny);
 
 // Simpson-weighted k_metric |v|^2 per block (Couette norm).
 cudaError_t launch_couette_norm2(const ImmArgs& a, const double2* v,
