@@ -981,7 +981,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
       it.a = make(ctxs[m], m);
       it.member = m;
       base.push_back(total);
-      total += ens_col_blocks(it.a, nO(ctxs[m]), nfields, &it.gx, &it.gy);
+      total += ens_col_blocks(&it, nO(ctxs[m]), nfields, maxL == 192);
       items.push_back(it);
     }
     EnsColItem* di = nullptr;
@@ -1036,7 +1036,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
       it.L = ctxs[m]->My;
       it.member = m;
       base.push_back(total);
-      total += ens_y_blocks(it.a, &it.gx);
+      total += ens_y_blocks(&it, maxL == 192);
       items.push_back(it);
     }
     EnsYItem* di = nullptr;

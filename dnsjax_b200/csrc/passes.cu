@@ -159,18 +159,21 @@ size_t col_pass2_smem(int M) {
 // OUT32 (FP32 only) an FP32 pass buffer.  CURL (inverse): `in` is the FP64
 // spectral state and field f of the 6 is u, v, w (f < 3) or the spectral
 // curl i (k x u) (triply_periodic.py:122-132), formed in FP64 at the load.
-// WIDE: the CTA has more threads than the shape's NT (the work-list kernels).
+// H = 2 (the work-list kernels): the CTA has twice the shape's NT threads, and each
+// half of it runs a block, (bx, by, bz) its own; idle: no block is left for the half.
 template <int ML, int SIGN, typename T = double, bool OUT32 = false, bool CURL = false,
-          bool SLAB = false, bool WIDE = false>
-__device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int by, int bz) {
+          bool SLAB = false, int H = 1>
+__device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int by, int bz,
+                                               bool idle = false) {
   using CT = typename pass_types<T>::C;
   using RT = typename pass_types<T>::R;
   constexpr int M = ML, R1 = ColShape<ML>::R1, R2 = ColShape<ML>::R2, C = ColShape<ML>::C;
   constexpr int NT = ColShape<ML>::NT;
   extern __shared__ double2 sm_[];
-  CT* X = reinterpret_cast<CT*>(sm_);  // [t][C]
+  const int half = H == 2 ? threadIdx.x / NT : 0;
+  CT* X = reinterpret_cast<CT*>(sm_) + half * (M * C + M);  // [t][C]
   CT* tw = X + M * C;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x - half * NT;
   const int i0 = bx * C;
   const long long o = by;
   const long long f = bz;
@@ -178,11 +181,15 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
   // FP64 output, or (OUT32, FP32 arithmetic) an FP32 pass buffer
   double2* out = a.out + f * a.out_fs + o * a.out_os + i0;
   CT* out_c = reinterpret_cast<CT*>(a.out) + f * a.out_fs + o * a.out_os + i0;
-  const int ni = min(C, a.nI - i0);
+  const int ni = H == 2 && idle ? 0 : min(C, a.nI - i0);
   const unsigned long long drop = l2_drop();
-  load_twiddles(tw, reinterpret_cast<const CT*>(a.tw), M);
+  if constexpr (H == 2) {
+    for (int i = tid; i < M; i += NT) tw[i] = reinterpret_cast<const CT*>(a.tw)[i];
+  } else {
+    load_twiddles(tw, reinterpret_cast<const CT*>(a.tw), M);
+  }
   __syncthreads();
-  if (!WIDE || tid < NT) {
+  {
     const int c = tid % C, j = tid / C;
     CT v[R1];
 #pragma unroll
@@ -240,7 +247,7 @@ __device__ __forceinline__ void col_pass2_body(const ColPassArgs& a, int bx, int
   }
   __syncthreads();
   const double sc = 1.0 / M;
-  for (int it = tid; it < R1 * C && (!WIDE || tid < NT); it += NT) {
+  for (int it = tid; it < R1 * C; it += NT) {
     const int c = it % C, k = it / C;
     CT z[R2];
 #pragma unroll
@@ -521,16 +528,33 @@ cudaError_t launch_x_pass(const XPassArgs& a, cudaStream_t st) {
 // runs the member's body on its block, so each member computes exactly what
 // its own launch computes.  Members whose `active` flag is 0 are skipped.
 // ---------------------------------------------------------------------------
-// CTAs of the widest member's shape: 256 threads where a member is 192 long,
-// else 128.
-constexpr int ens_col_threads(bool wide) { return wide ? ColShape<192>::NT : ColShape<96>::NT; }
+// CTAs of the widest member's shape: 256 threads where a member is 192 long, else
+// 128.  Members of the shorter shape run two of their blocks in a wide CTA: with one
+// and half of its threads idle, a step of 24 members of 48 to 192 points took 9.15
+// ms, 7.67 so (128 threads for all, 24 x 8 at 192: 8.98); four of 128^3: 9.49 and
+// 9.32 ms.
+__host__ __device__ constexpr int ens_col_threads(bool wide) {
+  return wide ? ColShape<192>::NT : ColShape<96>::NT;
+}
 static_assert(ColShape<48>::NT == ens_col_threads(false) &&
                   ColShape<72>::NT == ens_col_threads(false) &&
-                  ens_col_threads(true) >= ens_col_threads(false),
+                  ens_col_threads(true) == 2 * ens_col_threads(false),
               "a CTA shape for every member");
 
+// A member's block in this half of the CTA.
+template <int ML, int SIGN, bool CURL, bool WIDE>
+__device__ __forceinline__ void ens_col_block(const EnsColItem& it, const ColPassArgs& a,
+                                              int local) {
+  constexpr int H = WIDE && ColShape<ML>::NT < ens_col_threads(true) ? 2 : 1;
+  const int b = H == 2 ? 2 * local + threadIdx.x / ColShape<ML>::NT : local;
+  const int blk = min(b, it.blocks - 1), gx = it.gx, gy = it.gy;
+  col_pass2_body<ML, SIGN, double, false, CURL, false, H>(a, blk % gx, (blk / gx) % gy,
+                                                          blk / (gx * gy), b != blk);
+}
+
+// Wide: 16 warps per SM (the curl pass without the bound takes 246 registers).
 template <int SIGN, bool CURL, bool WIDE>
-__global__ void __launch_bounds__(ens_col_threads(WIDE))
+__global__ void __launch_bounds__(ens_col_threads(WIDE), WIDE ? 2 : 0)
 ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict__ base, int n,
                      int total, const int* __restrict__ active) {
   __shared__ int s_k;
@@ -541,14 +565,13 @@ ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict
     const int m = items[k].member;
     if (!active || active[m]) {
       const ColPassArgs a = items[k].a;
-      const int local = vb - base[k], gx = items[k].gx, gy = items[k].gy;
-      const int bx = local % gx, by = (local / gx) % gy, bz = local / (gx * gy);
+      const int local = vb - base[k];
       switch (a.plan.L) {
-        case 48: col_pass2_body<48, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
-        case 72: col_pass2_body<72, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
-        case 96: col_pass2_body<96, SIGN, double, false, CURL, false, WIDE>(a, bx, by, bz); break;
+        case 48: ens_col_block<48, SIGN, CURL, WIDE>(items[k], a, local); break;
+        case 72: ens_col_block<72, SIGN, CURL, WIDE>(items[k], a, local); break;
+        case 96: ens_col_block<96, SIGN, CURL, WIDE>(items[k], a, local); break;
         default:
-          if constexpr (WIDE) col_pass2_body<192, SIGN, double, false, CURL>(a, bx, by, bz);
+          if constexpr (WIDE) ens_col_block<192, SIGN, CURL, WIDE>(items[k], a, local);
           break;
       }
     }
@@ -558,11 +581,12 @@ ens_col_pass2_kernel(const EnsColItem* __restrict__ items, const int* __restrict
 
 bool ens_pass_supported(int L) { return fp32_length(L); }
 
-int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy) {
-  const int C = col_columns(a.plan.L);
-  *gx = (a.nI + C - 1) / C;
-  *gy = nO;
-  return *gx * nO * nfields;
+int ens_col_blocks(EnsColItem* it, int nO, int nfields, bool wide) {
+  const int L = it->a.plan.L, C = col_columns(L);
+  it->gx = (it->a.nI + C - 1) / C;
+  it->gy = nO;
+  it->blocks = it->gx * nO * nfields;
+  return wide && L != 192 ? (it->blocks + 1) / 2 : it->blocks;
 }
 
 size_t ens_col_smem(int maxL) { return col_pass2_smem(maxL); }

@@ -223,9 +223,9 @@ cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st);
 // Its work-list form for ensembles (see EnsColItem).
 struct EnsYItem {
   YProjArgs a;
-  int L, gx, member;
+  int L, gx, blocks, member;
 };
-int ens_y_blocks(const YProjArgs& a, int* gx);
+int ens_y_blocks(EnsYItem* it, bool wide);
 size_t ens_y_smem(int maxL);
 int ens_y_threads(bool wide);
 const void* ens_y_kernel(bool wide);
@@ -288,6 +288,7 @@ cudaError_t set_x_transform_attributes(int max_smem);
 struct EnsColItem {
   ColPassArgs a;
   int gx, gy;  // the member's grid (gx, gy, nfields), flattened bx fastest
+  int blocks;  // gx gy nfields
   int member;
 };
 struct EnsXItem {
@@ -295,7 +296,8 @@ struct EnsXItem {
   int member;
 };
 bool ens_pass_supported(int L);
-int ens_col_blocks(const ColPassArgs& a, int nO, int nfields, int* gx, int* gy);
+// Fill an item's grid; CTAs that its blocks take (wide: see ens_pass_grid).
+int ens_col_blocks(EnsColItem* it, int nO, int nfields, bool wide);
 int ens_x_blocks(const XPassArgs& a);
 constexpr int kEnsXThreads = 96;
 const void* ens_x_kernel();

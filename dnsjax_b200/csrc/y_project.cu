@@ -32,22 +32,25 @@ struct YShape {
   static constexpr int MINB = NT <= 192 ? 2 : !F32 && R1 <= 16 ? 768 / NT : 1;
 };
 
-// WIDE: the CTA has more threads than the shape's NT (the work-list kernel).
-template <int ML, typename T, bool WIDE = false>
-__device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, int iz) {
+// H = 2: two blocks in a CTA of twice the shape's NT threads, as col_pass2_body
+// (csrc/passes.cu).
+template <int ML, typename T, int H = 1>
+__device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, int iz,
+                                                  bool idle = false) {
   using CT = typename pass_types<T>::C;
   using SH = YShape<ML, T>;
   constexpr int M = ML, R1 = SH::R1, R2 = SH::R2, C = SH::C, NF = SH::NF, NT = SH::NT;
   extern __shared__ double2 sm_[];
-  CT* sm = reinterpret_cast<CT*>(sm_);  // [component][t][C]
+  const int half = H == 2 ? threadIdx.x / NT : 0;
+  CT* sm = reinterpret_cast<CT*>(sm_) + half * 3 * M * C;  // [component][t][C]
   const CT* __restrict__ tw = reinterpret_cast<const CT*>(a.tw);
-  const int tid = threadIdx.x, f = tid / NF, t0 = tid % NF;
+  const int tid = threadIdx.x - half * NT, f = tid / NF, t0 = tid % NF;
   const int NY1 = a.NY1, NZ1 = a.NZ1, NKX = a.NKX;
   const int i0 = bx * C;
-  const int ni = min(C, NKX - i0);
+  const int ni = H == 2 && idle ? 0 : min(C, NKX - i0);
   CT* X = sm + f * M * C;
   const long long row = (long long)NZ1 * NKX;  // stride of y
-  if (!WIDE || tid < NT) {
+  {
     const int c = t0 % C, j = t0 / C;
     const CT* in = reinterpret_cast<const CT*>(a.in) + (long long)f * M * row +
                    (long long)iz * NKX + i0 + c;
@@ -61,7 +64,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
     for (int i = 0; i < R1; ++i) X[(j * R1 + i) * C + c] = v[i];
   }
   __syncthreads();
-  for (int it = t0; it < R1 * C && (!WIDE || tid < NT); it += NF) {
+  for (int it = t0; it < R1 * C; it += NF) {
     const int c = it % C, k = it / C;
     CT z[R2];
 #pragma unroll
@@ -77,7 +80,7 @@ __device__ __forceinline__ void yfwd_project_body(const YProjArgs& a, int bx, in
   const double sc = 1.0 / M;
   const double kz = a.kz[iz];
   const long long cs = (long long)NY1 * row;
-  for (int idx = tid; idx < NY1 * C && (!WIDE || tid < NT); idx += NT) {
+  for (int idx = tid; idx < NY1 * C; idx += NT) {
     const int c = idx % C, s = idx / C;
     if (c >= ni) continue;
     const int t = stored_to_pos(s, NY1, M) * C + c;
@@ -104,15 +107,26 @@ yfwd_project_kernel(YProjArgs a) {
   yfwd_project_body<ML, T>(a, blockIdx.x, blockIdx.y);
 }
 
-// Work-list form for ensembles: as ens_x_pass2_kernel (csrc/x_pass.cu).
-constexpr int ens_y_shape(bool wide) {
+// Work-list form for ensembles: as ens_x_pass2_kernel (csrc/x_pass.cu), two blocks of
+// a shorter member in a wide CTA as ens_col_pass2_kernel (csrc/passes.cu).  Wide: 24
+// warps per SM as the plain kernel at 192 (308 bytes of spills; with 12 warps a step
+// of four 128^3 members took 9.55 ms, 9.32 so).
+__host__ __device__ constexpr int ens_y_shape(bool wide) {
   return wide ? YShape<192, double>::NT : YShape<96, double>::NT;
 }
 static_assert(YShape<48, double>::NT == ens_y_shape(false) &&
-                  YShape<72, double>::NT == ens_y_shape(false),
+                  YShape<72, double>::NT == ens_y_shape(false) &&
+                  ens_y_shape(true) == 2 * ens_y_shape(false),
               "a CTA shape for every member");
+template <int ML, bool WIDE>
+__device__ __forceinline__ void ens_y_block(const EnsYItem& it, const YProjArgs& a, int local) {
+  constexpr int NT = YShape<ML, double>::NT, H = WIDE && NT < ens_y_shape(true) ? 2 : 1;
+  const int b = H == 2 ? 2 * local + threadIdx.x / NT : local;
+  const int blk = min(b, it.blocks - 1);
+  yfwd_project_body<ML, double, H>(a, blk % it.gx, blk / it.gx, b != blk);
+}
 template <bool WIDE>
-__global__ void __launch_bounds__(ens_y_shape(WIDE))
+__global__ void __launch_bounds__(ens_y_shape(WIDE), WIDE ? 2 : 0)
 ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restrict__ base, int n,
                         int total, const int* __restrict__ active) {
   __shared__ int s_k;
@@ -123,13 +137,13 @@ ens_yfwd_project_kernel(const EnsYItem* __restrict__ items, const int* __restric
     const int m = items[k].member;
     if (!active || active[m]) {
       const YProjArgs a = items[k].a;
-      const int gx = items[k].gx, bx = (vb - base[k]) % gx, iz = (vb - base[k]) / gx;
+      const int local = vb - base[k];
       switch (items[k].L) {
-        case 48: yfwd_project_body<48, double, WIDE>(a, bx, iz); break;
-        case 72: yfwd_project_body<72, double, WIDE>(a, bx, iz); break;
-        case 96: yfwd_project_body<96, double, WIDE>(a, bx, iz); break;
+        case 48: ens_y_block<48, WIDE>(items[k], a, local); break;
+        case 72: ens_y_block<72, WIDE>(items[k], a, local); break;
+        case 96: ens_y_block<96, WIDE>(items[k], a, local); break;
         default:
-          if constexpr (WIDE) yfwd_project_body<192, double>(a, bx, iz);
+          if constexpr (WIDE) ens_y_block<192, WIDE>(items[k], a, local);
           break;
       }
     }
@@ -161,9 +175,10 @@ cudaError_t launch_yfwd_project(const YProjArgs& a, int L, cudaStream_t st) {
   });
 }
 
-int ens_y_blocks(const YProjArgs& a, int* gx) {
-  *gx = (a.NKX + YShape<192, double>::C - 1) / YShape<192, double>::C;
-  return *gx * a.NZ1;
+int ens_y_blocks(EnsYItem* it, bool wide) {
+  it->gx = (it->a.NKX + YShape<192, double>::C - 1) / YShape<192, double>::C;
+  it->blocks = it->gx * it->a.NZ1;
+  return wide && it->L != 192 ? (it->blocks + 1) / 2 : it->blocks;
 }
 
 size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192, double>::C); }
