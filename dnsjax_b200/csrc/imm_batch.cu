@@ -475,8 +475,13 @@ bool imm_batch_supported(int kl, int ny) {
   return (kl == 2 || kl == 4 || kl == 6 || kl == 8) && ny <= kMaxNy;
 }
 
-// Window-relative stencil weights of the stage kernel: lane l's window of
-// W = (p + 2) + YM - 1 rows starts at base[l], and w1x / w2x[(o W + i) 32 + l] is
+// First row of lane l's window of W = (p + 2) + YM - 1 rows.
+static int window_base(int Ny, int p, const int* j01, const int* j02, int l) {
+  const int YM = imm_batch_rows(Ny), W = p + 2 + YM - 1, y = std::min(YM * l, Ny - 1);
+  return std::max(0, std::min(std::min(j01[y], j02[y]), Ny - W));
+}
+
+// Window-relative stencil weights of the stage kernel: base[l] = window_base, and w1x / w2x[(o W + i) 32 + l] is
 // the weight of window row i in D1 / D2 of row YM l + o (0 outside the stencil
 // and past the last row).
 void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const int* j02,
@@ -487,7 +492,7 @@ void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const in
   w1x->assign((size_t)YM * W * 32, 0.0);
   w2x->assign((size_t)YM * W * 32, 0.0);
   for (int l = 0; l < 32; ++l) {
-    const int b = std::max(0, std::min(YM * l - S2 / 2, Ny - W));
+    const int b = window_base(Ny, p, j01, j02, l);
     (*base)[l] = b;
     for (int o = 0; o < YM && YM * l + o < Ny; ++o) {
       const int y = YM * l + o;
@@ -499,12 +504,13 @@ void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const in
   }
 }
 
-// Every stencil of a lane's rows lies in its window (true for stencils centred
-// in the interior and shifted to stay inside the walls).
+// Every stencil of a lane's rows lies in its window: true where D1's start a row
+// after D2's or with them, as they do centred in the interior (D2's even width
+// either way) and shifted to stay inside the walls.
 bool imm_batch_windows_ok(int Ny, int p, const int* j01, const int* j02) {
   const int YM = imm_batch_rows(Ny), S1 = p + 1, S2 = p + 2, W = S2 + YM - 1;
   for (int y = 0; y < Ny; ++y) {
-    const int b = std::max(0, std::min((y / YM) * YM - S2 / 2, Ny - W));
+    const int b = window_base(Ny, p, j01, j02, y / YM);
     if (j01[y] < b || j02[y] < b || j01[y] + S1 > b + W || j02[y] + S2 > b + W) return false;
   }
   return true;

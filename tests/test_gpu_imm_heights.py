@@ -51,6 +51,37 @@ def test_imm_heights(nx, ny, nz, fd):
     flow.check_status()
 
 
+@pytest.mark.parametrize("ny,fd", [(65, 4), (129, 6), (161, 2)])
+def test_other_stencils(monkeypatch, ny, fd):
+    """D2's even stencils centred half a row the other way: any stencils whose
+    rows contain the point are accepted, and these run batched too."""
+    import torch
+
+    import dnsjax_b200.fd
+    from dnsjax_b200 import _lib, initial
+    from dnsjax_b200.flows.plane_couette import PlaneCouetteFlow
+    from dnsjax_b200.parameters import Parameters
+    from oracle.config import Config
+    from oracle.couette import CouetteSetup
+
+    monkeypatch.setattr(dnsjax_b200.fd, "stencil_start",
+                        lambda i, n, width: max(0, min(i - (width - 1) // 2, n - width)))
+    p = Parameters(phys=dict(system="plane-couette", re=400.0), geo=dict(lx=2 * pi, lz=pi),
+                   res=dict(nx=8, ny=ny, nz=8, fd_order=fd), step=dict(dt=0.01))
+    flow = PlaneCouetteFlow(p)
+    imm = {k: v.cpu().numpy() for k, v in flow.imm.items()}
+    orc = CouetteSetup(Config(system="plane-couette", nx=8, ny=ny, nz=8, lx=2 * pi, lz=pi,
+                              re=400.0, dt=0.01, fd_order=fd),
+                       imm=dict(imm, D1=flow.D1, D2=flow.D2))
+    f = [initial.couette_field(8, ny, 8, 2 * pi, pi, fd, s, 8.0, 1e-2) for s in (1, 2, 3, 4)]
+    new, _ = orc.correct(*f)
+    before = _lib.launch_count()
+    got, _ = flow.correct(*[torch.as_tensor(np.ascontiguousarray(a), device="cuda") for a in f])
+    assert _lib.launch_count() - before == 5
+    assert rel_l2(got.cpu(), new) < 1e-12 * max(1.0, (ny / 129.0) ** 4)
+    flow.check_status()
+
+
 def _fma(a, b, c):
     """a b + c rounded once (an 80-bit product and sum, then 64 bits)."""
     return (np.longdouble(a) * np.longdouble(b) + np.longdouble(c)).astype(np.float64)
