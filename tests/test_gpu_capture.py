@@ -1,6 +1,8 @@
-"""Calls whose kernels are launched dependent on one another (small grids) and
-plainly (large ones), captured in a CUDA graph by the caller: replays equal
-the eager calls bit for bit, alone and back to back."""
+"""Calls whose kernels are launched dependent on one another (small grids),
+plainly (large ones) and, plane Couette between the two, plainly in the RHS alone,
+captured in a CUDA graph by the caller: replays equal the eager calls bit for bit,
+alone and back to back.  On the small grids the eager calls also equal those of a
+step graph, whose kernels are all launched plainly."""
 
 from math import pi
 
@@ -10,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("system,n", [("kolmogorov", 32), ("kolmogorov", 192),
-                                      ("plane-couette", 32), ("plane-couette", 96)])
+                                      ("plane-couette", 32), ("plane-couette", 96),
+                                      ("plane-couette", 128), ("plane-couette", 144)])
 def test_captured_calls(system, n):
     import torch
 
@@ -34,6 +37,14 @@ def test_captured_calls(system, n):
         r2 = flow.get_rhs(v)
         return r, r2, flow.correct_fused(u, v, r, r2, err)
 
+    if n == 32:
+        pac, _ = flow.make_stepper()
+        state = u.clone()
+        step = flow.make_step_graph(state, tol=1e30, max_iter=60)  # the first correction
+        step.launch()
+        assert step.status()[0] == 0
+        assert torch.equal(state, flow.correct_velocity(pac(u)[0])[0])
+        step.close()
     want = [t.clone() for t in calls()]
     e = err.clone()
     torch.cuda.synchronize()

@@ -15,9 +15,14 @@ from conftest import rel_l2
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("fd", [2, 4, 6, 8])
-@pytest.mark.parametrize("nx,ny,nz", [(16, 11, 16), (12, 65, 24), (16, 159, 8), (8, 161, 16),
-                                      (16, 193, 12), (8, 257, 8), (4, 301, 8)])
+GRIDS = [(16, 11, 16), (12, 65, 24), (16, 159, 8), (8, 161, 16), (16, 193, 12), (8, 257, 8),
+         (4, 301, 8)]
+
+
+# 96 x 21 x 128: 192 tiles, beyond the 148 up to which the substitutions of orders 6
+# and 8 take one column per lane
+@pytest.mark.parametrize("nx,ny,nz,fd", [(*g, fd) for fd in (2, 4, 6, 8) for g in GRIDS]
+                         + [(96, 21, 128, 6), (96, 21, 128, 8)])
 def test_imm_heights(nx, ny, nz, fd):
     import torch
 

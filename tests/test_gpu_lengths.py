@@ -1,7 +1,9 @@
 """Every padded length of the two-stage passes on each axis, against the
-oracle: the RHS and the transforms, both flow families.  The other axes stay
-at 16 modes (padded 24, Stockham stages), so one length is tested at a time;
-nx/2 = n/2 columns leave the last column tile partly filled."""
+oracle: the RHS and the transforms, both flow families.  First one length at a
+time, the other axes at 16 modes (padded 24, Stockham stages; one column tile of
+the periodic flows' y and z passes); then grids of these lengths alone, with
+several column tiles of which the last is partly filled, and both block orders of
+the curl passes."""
 
 from math import pi
 
@@ -22,9 +24,20 @@ def dev(a):
     return torch.as_tensor(np.ascontiguousarray(a), device="cuda")
 
 
-@pytest.mark.parametrize("axis", [0, 1, 2])
-@pytest.mark.parametrize("n", MODES)
-def test_periodic_lengths(n, axis):
+# grid of each flow family: several column tiles, a partly filled last one
+PERIODIC_GRIDS = [
+    (36, 24, 72), (36, 72, 24), (72, 96, 144), (108, 36, 108),
+    (128, 24, 72),   # a tile's fields next to one another: (nx / 2)(nz - 1) >= 4096
+    (72, 192, 128),  # the same with the 8-column tiles of 288 points
+]
+COUETTE_GRIDS = [
+    (36, 33, 72), (108, 21, 96), (72, 19, 256),
+    (144, 65, 144),  # a tile's fields next to one another: (nx / 2) ny >= 4096
+    (96, 97, 192),   # the same with 8-column tiles
+]
+
+
+def check_periodic(g, seed):
     from dnsjax_b200 import initial
     from dnsjax_b200.flows.monochromatic import TriplyPeriodicFlow
     from dnsjax_b200.parameters import Parameters
@@ -32,15 +45,13 @@ def test_periodic_lengths(n, axis):
     from oracle.fft import spec_to_phys
     from oracle.periodic import PeriodicSetup
 
-    g = [16, 16, 16]
-    g[axis] = n
     p = Parameters(phys=dict(system="waleffe", re=60.0),
                    geo=dict(lx=2 * pi, lz=2 * pi, tilt_degree=30.0),
                    res=dict(nx=g[0], ny=g[1], nz=g[2]), step=dict(dt=0.01))
     cfg = Config(system="waleffe", nx=g[0], ny=g[1], nz=g[2], lx=2 * pi, lz=2 * pi, ly=2 * pi,
                  re=60.0, dt=0.01, tilt_degree=30.0)
     flow, orc = TriplyPeriodicFlow(p, ly=2 * pi), PeriodicSetup(cfg)
-    u0 = initial.periodic_field(*g, 2 * pi, 2 * pi, 2 * pi, n + axis,
+    u0 = initial.periodic_field(*g, 2 * pi, 2 * pi, 2 * pi, seed,
                                 initial.kolmogorov_spectrum_k53, 0.1)
     assert rel_l2(flow.get_rhs(dev(u0)).cpu(), orc.get_rhs(u0)) < 1e-12
     phys = spec_to_phys(u0, cfg)
@@ -48,9 +59,20 @@ def test_periodic_lengths(n, axis):
     assert rel_l2(flow.phys_to_spec(dev(phys)).cpu(), u0) < 1e-13
 
 
-@pytest.mark.parametrize("axis", [0, 2])
+@pytest.mark.parametrize("axis", [0, 1, 2])
 @pytest.mark.parametrize("n", MODES)
-def test_couette_lengths(n, axis):
+def test_periodic_lengths(n, axis):
+    g = [16, 16, 16]
+    g[axis] = n
+    check_periodic(g, n + axis)
+
+
+@pytest.mark.parametrize("g", PERIODIC_GRIDS)
+def test_periodic_grids(g):
+    check_periodic(g, 5)
+
+
+def check_couette(g, seed):
     from dnsjax_b200 import initial
     from dnsjax_b200.flows.plane_couette import PlaneCouetteFlow
     from dnsjax_b200.parameters import Parameters
@@ -58,8 +80,6 @@ def test_couette_lengths(n, axis):
     from oracle.couette import CouetteSetup
     from oracle.fft import spec_to_phys_2d
 
-    g = [16, 19, 16]
-    g[axis] = n
     p = Parameters(phys=dict(system="plane-couette", re=400.0), geo=dict(lx=2 * pi, lz=pi),
                    res=dict(nx=g[0], ny=g[1], nz=g[2], fd_order=4), step=dict(dt=0.01))
     cfg = Config(system="plane-couette", nx=g[0], ny=g[1], nz=g[2], lx=2 * pi, lz=pi,
@@ -67,11 +87,24 @@ def test_couette_lengths(n, axis):
     flow = PlaneCouetteFlow(p)
     imm = {k: v.cpu().numpy() for k, v in flow.imm.items()}
     orc = CouetteSetup(cfg, imm=dict(imm, D1=flow.D1, D2=flow.D2))
-    u0 = initial.couette_field(*g, 2 * pi, pi, 4, n + axis, 8.0, 1e-2)
+    u0 = initial.couette_field(*g, 2 * pi, pi, 4, seed, 8.0, 1e-2)
     assert rel_l2(flow.get_rhs(dev(u0)).cpu(), orc.get_rhs(u0)) < 1e-12
     phys = spec_to_phys_2d(u0, cfg)
     assert rel_l2(flow.spec_to_phys(dev(u0)).cpu(), phys) < 1e-13
     assert rel_l2(flow.phys_to_spec(dev(phys)).cpu(), u0) < 1e-13
+
+
+@pytest.mark.parametrize("axis", [0, 2])
+@pytest.mark.parametrize("n", MODES)
+def test_couette_lengths(n, axis):
+    g = [16, 19, 16]
+    g[axis] = n
+    check_couette(g, n + axis)
+
+
+@pytest.mark.parametrize("g", COUETTE_GRIDS)
+def test_couette_grids(g):
+    check_couette(g, 5)
 
 
 @pytest.mark.parametrize("system", ["kolmogorov", "plane-couette"])
