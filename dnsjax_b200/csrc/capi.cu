@@ -82,6 +82,13 @@ int max_smem_optin() {
   return v;
 }
 
+int multiprocessors() {
+  int dev = 0, v = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+  return v;
+}
+
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace
@@ -290,7 +297,6 @@ static ColPassArgs periodic_zinv(const dnsb_periodic* p) {
   a.inverse = 1;
   a.plan = p->pz;
   a.tw = p->twz;
-  a.occ4 = 1;
   return a;
 }
 
@@ -310,7 +316,7 @@ static ColPassArgs periodic_zfwd(const dnsb_periodic* p) {
   a.inverse = 0;
   a.plan = p->pz;
   a.tw = p->twz;
-  a.occ4 = 1;
+  a.held = 1;
   return a;
 }
 
@@ -336,7 +342,6 @@ static ColPassArgs periodic_ycurl(const dnsb_periodic* p, const void* state) {
   yc.kx = p->kx;
   yc.ky = p->ky;
   yc.kz = p->kz;
-  yc.occ4 = 1;
   // beyond a few waves of blocks (128^3 RHS 359 -> 347 us, 256^3 3285 -> 3193; a
   // 32^3 step took 174 -> 177 us so)
   yc.fields_fast = (long long)p->NKX * p->NZ1 >= 4096;
@@ -383,7 +388,7 @@ static ColPassArgs periodic_yfwd_col(const dnsb_periodic* p, void* rhs) {
   yc.inverse = 0;
   yc.plan = p->py;
   yc.tw = p->twy;
-  yc.occ4 = 1;
+  yc.held = 1;
   return yc;
 }
 
@@ -494,7 +499,8 @@ extern "C" int dnsb_periodic_set_rhs_precision(dnsb_periodic* p, int fp32) {
   if (!p) return fail(DNSB_ERR_ARG, "null argument");
   if (fp32 && p->slab.nranks) return fail(DNSB_ERR_ARG, "slab contexts run the FP64 passes");
   if (fp32) {
-      if (!fp32_length(p->My) || !fp32_length(p->Mz) || !fp32_length(p->Mx) || 3 * p->NKX != p->Mx)
+    if (!fp32_length(p->My) || !fp32_length(p->Mz) || !fp32_length(p->Mx) ||
+        3 * p->NKX != p->Mx)
       return fail(DNSB_ERR_ARG,
                   "FP32 RHS passes need padded sizes in {48, 72, 96, 192} with nx_p = 3 nx / 2");
   }
@@ -964,11 +970,8 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return ctxs[a]->S > ctxs[b]->S; });
   const int smax = max_smem_optin();
-  int maxL = 0, maxNKX = 0;
-  for (int m = 0; m < n; ++m) {
-    maxL = std::max({maxL, ctxs[m]->My, ctxs[m]->Mz, ctxs[m]->Mx});
-    maxNKX = std::max(maxNKX, ctxs[m]->NKX);
-  }
+  int maxL = 0;
+  for (int m = 0; m < n; ++m) maxL = std::max({maxL, ctxs[m]->My, ctxs[m]->Mz, ctxs[m]->Mx});
   // kind 0..3: col (curl), col (inverse), col (forward), x pass
   auto col_stage = [&](int kind, auto make, int nfields, auto nO) -> EnsStage {
     EnsStage st;
@@ -1019,7 +1022,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     st.base = db;
     st.n = n;
     st.total = total;
-    st.smem = ens_x_smem(maxL, maxNKX);
+    st.smem = ens_x_smem(maxL);
     st.grid = rc ? 0 : ens_pass_grid(3, maxL == 192, st.smem, total, smax);
     if (!rc && st.grid <= 0) rc = fail(DNSB_ERR_CUDA, "ensemble pass occupancy");
     return st;
@@ -1072,7 +1075,8 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   for (int c = 0; c < 3; ++c) {
     auto in_of = [&](int m) -> const void* { return c == 0 ? states[m] : (const void*)P[m]; };
     auto out_of = [&](int m) -> void* { return c == 1 ? (void*)Rb[m] : (void*)Ra[m]; };
-    rl[c].yc = col_stage(0, [&](const dnsb_periodic* q, int m) { return periodic_ycurl(q, in_of(m)); },
+    rl[c].yc = col_stage(0,
+                         [&](const dnsb_periodic* q, int m) { return periodic_ycurl(q, in_of(m)); },
                          6, [](const dnsb_periodic* q) { return q->NZ1; });
     rl[c].zi = col_stage(1, [&](const dnsb_periodic* q, int) { return periodic_zinv(q); }, 6,
                          [](const dnsb_periodic* q) { return q->My; });
@@ -1110,7 +1114,8 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   const int pgrid = std::min(n * kRedBlocks, 4 * nsm);
 
   auto run_pass = [&](const EnsStage& st, const int* act, cudaStream_t s) {
-    return launch_ens_pass(st.kind, maxL == 192, st.items, st.base, st.n, st.total, act, st.grid, st.smem, s);
+    return launch_ens_pass(st.kind, maxL == 192, st.items, st.base, st.n, st.total, act, st.grid,
+                           st.smem, s);
   };
   auto rhs = [&](int c, const int* act, cudaStream_t s) -> cudaError_t {
     cudaError_t r;
@@ -1122,7 +1127,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     return run_pass(L.yf, act, s);
   };
   auto correct = [&](int k, const int* act, cudaStream_t s) -> cudaError_t {
-    cudaError_t r = launch_ens_point(corr[k], n, act, 1, 0, 0, pgrid, s);
+    cudaError_t r = launch_ens_point(corr[k], n, act, 1, 0, pgrid, s);
     if (r == cudaSuccess) r = launch_ens_finalize(corr[k], n, act, err, s);
     return r;
   };
@@ -1149,7 +1154,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
   ck(cudaGraphConditionalHandleCreate(&h, graph, 0, 0), "conditional handle");
   // prologue: every member
   ck(rhs(0, nullptr, s), "rhs");
-  ck(launch_ens_point(pred, n, nullptr, 0, 0, 0, pgrid, s), "predict");
+  ck(launch_ens_point(pred, n, nullptr, 0, 0, pgrid, s), "predict");
   ck(rhs(1, nullptr, s), "rhs");
   ck(correct(0, nullptr, s), "correct");
   ens_ctl_kernel<<<1, 1024, 0, s>>>(h, 0, 0, n, err, d_tol, d_max, e->iters, active,
@@ -1182,7 +1187,7 @@ extern "C" int dnsb_ensemble_create(dnsb_periodic* const* ctxs, void* const* sta
     cudaGraph_t bout = nullptr;
     ck(cudaStreamEndCapture(sb, &bout), "end body capture");
   }
-  ck(launch_ens_point(cv, n, nullptr, 2, divergence, 1, pgrid, s), "correct_velocity");
+  ck(launch_ens_point(cv, n, nullptr, 2, divergence, pgrid, s), "correct_velocity");
   cudaGraph_t done = nullptr;
   ck(cudaStreamEndCapture(s, &done), "end capture");  // always end the capture
   if (!rc) ck(cudaGraphInstantiate(&e->exec, done, 0), "instantiate");
@@ -1410,9 +1415,10 @@ struct dnsb_couette {
 };
 
 static void couette_free(dnsb_couette* p) {
-  void* ptrs[] = {p->twz, p->twx, p->twz32, p->twx32, p->kx, p->kz, p->d1w, p->d2w, p->d1wT, p->d2wT, p->d1j0,
-                  p->d2j0, p->U, p->cU, p->nU, p->simpson, p->B, p->partials,
-                  p->status, p->fac, p->dp, p->Fw, p->Rw, p->w1x, p->w2x, p->wbase, p->slab.Bx};
+  void* ptrs[] = {p->twz,  p->twx,  p->twz32, p->twx32,    p->kx,     p->kz,  p->d1w,
+                  p->d2w,  p->d1wT, p->d2wT,  p->d1j0,     p->d2j0,   p->U,   p->cU,
+                  p->nU,   p->simpson, p->B,  p->partials, p->status, p->fac, p->dp,
+                  p->Fw,   p->Rw,   p->w1x,   p->w2x,      p->wbase,  p->slab.Bx};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   delete p;
@@ -1630,6 +1636,7 @@ static int bind_batch(dnsb_couette* p) {
   b.nu = nu;
   b.paired = p->pair_modes;
   b.max_smem = smax;
+  b.sms = multiprocessors();
   b.status = p->status;
   b.wait_limit = p->wait_limit;
   b.F = p->Fw;

@@ -481,9 +481,9 @@ static int window_base(int Ny, int p, const int* j01, const int* j02, int l) {
   return std::max(0, std::min(std::min(j01[y], j02[y]), Ny - W));
 }
 
-// Window-relative stencil weights of the stage kernel: base[l] = window_base, and w1x / w2x[(o W + i) 32 + l] is
-// the weight of window row i in D1 / D2 of row YM l + o (0 outside the stencil
-// and past the last row).
+// Window-relative stencil weights of the stage kernel: base[l] = window_base, and
+// w1x / w2x[(o W + i) 32 + l] is the weight of window row i in D1 / D2 of row YM l + o
+// (0 outside the stencil and past the last row).
 void imm_batch_windows(int Ny, int p, const int* j01, const double* w1, const int* j02,
                        const double* w2, std::vector<int>* base, std::vector<double>* w1x,
                        std::vector<double>* w2x) {
@@ -567,7 +567,7 @@ static cudaError_t solve_launch(const ImmBatch& bt, int op, double2* X, long lon
   // tiles it loses (128 x 129 x 128 193.7 -> 195.1 us), as it does at kl = 4 (32 x
   // 53 x 36 predict_and_correct 131.4 -> 133.7 us).
   constexpr int SC = kSplitCols<KL>;
-  const bool split = SC == 1 && grid <= kSplitTiles;
+  const bool split = SC == 1 && grid <= bt.sms;
   const int threads = 32 * ((split ? 2 : 1) * ncomp + 1);
   const void* kernel = imm_batch_scaled(Ny) ? imm_solve_fn<true>(KL, bt.nu, split)
                                             : imm_solve_plain(KL, bt.nu, split);
@@ -586,9 +586,10 @@ static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2*
   const long long cs = (long long)tiles * Ny * kLanes;
   const size_t sm = imm_batch_stage_smem(Ny), sm6 = imm_batch_assemble_smem(Ny);
   cudaError_t e;
-#define DNSB_STAGE013(YM)                                                                   \
-  case YM:                                                                                  \
-    launch_dep(a.dep, imm_stage013_kernel<K, YM>, grid, threads, sm, st, a, bt.paired, bt.w1x, bt.w2x, bt.base, vel_n, nl_n, nl_j, bt.F, bt.R, cs);                        \
+#define DNSB_STAGE013(YM)                                                              \
+  case YM:                                                                             \
+    launch_dep(a.dep, imm_stage013_kernel<K, YM>, grid, threads, sm, st, a, bt.paired, \
+               bt.w1x, bt.w2x, bt.base, vel_n, nl_n, nl_j, bt.F, bt.R, cs);            \
     break;
   switch (imm_batch_rows(Ny)) {
     DNSB_STAGE013(3) DNSB_STAGE013(5) DNSB_STAGE013(7) DNSB_STAGE013(9) DNSB_STAGE013(17)
@@ -598,16 +599,16 @@ static cudaError_t pipeline(const ImmArgs& a, const ImmBatch& bt, const double2*
   e = solve_launch<K>(bt, 0, bt.F, 0, 1, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
   const dim3 gg((Ny - 2 + kGradRows - 1) / kGradRows, tiles);
-  launch_dep(a.dep, imm_grad_kernel<K>, gg, kLanes * kGradRows, 0, st, a, bt.paired, bt.NP, bt.F, bt.R, cs);
+  launch_dep(a.dep, imm_grad_kernel<K>, gg, kLanes * kGradRows, 0, st, a, bt.paired, bt.NP, bt.F,
+             bt.R, cs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = solve_launch<K>(bt, 1, bt.R, cs, 3, Ny, a.skip, st);
   if (e != cudaSuccess) return e;
-  if (Ny <= 96)
-    launch_dep(a.dep, imm_stage6_kernel<K, 3>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
-  else if (Ny <= 160)
-    launch_dep(a.dep, imm_stage6_kernel<K, 5>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
-  else
-    launch_dep(a.dep, imm_stage6_kernel<K, 0>, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new, corr_out, partials);
+  auto* stage6 = Ny <= 96    ? imm_stage6_kernel<K, 3>
+                 : Ny <= 160 ? imm_stage6_kernel<K, 5>
+                             : imm_stage6_kernel<K, 0>;
+  launch_dep(a.dep, stage6, grid, threads, sm6, st, a, bt.paired, bt.R, cs, vel_j, vel_new,
+             corr_out, partials);
   return cudaGetLastError();
 }
 

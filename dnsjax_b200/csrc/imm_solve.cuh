@@ -11,10 +11,9 @@ namespace {
 constexpr int kTile = 16;       // items per substitution CTA (two sides per item)
 constexpr int kLanes = 2 * kTile;  // lanes of a tile row (two sides)
 constexpr int kRowDoubles = 2 * kLanes;
-// Substitution lanes of one real column: bandwidths and tiles (see solve_launch).
+// Real columns of a substitution lane on few tiles, by bandwidth (see solve_launch).
 template <int KL>
 constexpr int kSplitCols = KL >= 6 ? 1 : 2;
-constexpr int kSplitTiles = 148;
 
 }  // namespace
 

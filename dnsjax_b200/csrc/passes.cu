@@ -140,8 +140,9 @@ template <int M>
 struct ColShape {
   static constexpr int R1 = ColRadix<M>::R1, R2 = ColRadix<M>::R2, C = col_columns(M);
   static constexpr int NT = R2 * C;
-  // CTAs per SM that the registers are held to: 24 warps where at most 16 complex
-  // values a thread fit 80 registers, else 16
+  // CTAs per SM that the registers are held to: 768 threads' worth where at most 16
+  // complex values a thread fit 80 registers (24 warps, 25 at 108 points), else 512
+  // (12 to 16 warps)
   static constexpr int MINB = (R1 <= 16 && R2 <= 16 ? 768 : 512) / NT;
   // the same for the Couette z inverse, whose curl takes more
   static constexpr int ZB = M == 36 || M == 54                             ? 5
@@ -298,12 +299,12 @@ col_pass2_kernel(ColPassArgs a) {
   col_pass2_body<ML, SIGN, T, OUT32, CURL, SLAB>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// The FP64 pass with its registers held to ColShape::MINB CTAs per SM
-// (ColPassArgs::occ4: the periodic flows' column passes; the lengths compiled for
-// FP64 alone take it always).
+// The FP64 pass with its registers held to ColShape::MINB CTAs per SM: the inverse
+// passes, the forward ones with ColPassArgs::held and at the lengths compiled for
+// FP64 alone.
 template <int ML, int SIGN, bool CURL>
 __global__ void __launch_bounds__(ColShape<ML>::NT, ColShape<ML>::MINB)
-col_pass2_occ4_kernel(ColPassArgs a) {
+col_pass2_held_kernel(ColPassArgs a) {
   grid_dep_sync();
   if (a.skip && *a.skip) return;
   if (CURL && a.fields_fast)
@@ -327,7 +328,8 @@ cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
       constexpr int LL = decltype(len)::value, NT = ColShape<LL>::NT;
       if constexpr (fp32_length(LL)) {
         if (slab)
-          launch_dep(a.dep, col_pass2_kernel<LL, 1, double, false, false, true>, g2, NT, sm2, st, a);
+          launch_dep(a.dep, col_pass2_kernel<LL, 1, double, false, false, true>, g2, NT, sm2, st,
+                     a);
         else if (a.curl && a.fp32 == 2)
           launch_dep(a.dep, col_pass2_kernel<LL, 1, fcomp, true, true>, g2, NT, sm2, st, a);
         else if (a.fp32 == 2 && a.inverse)
@@ -344,21 +346,17 @@ cudaError_t launch_col_pass(const ColPassArgs& a, int nfields, int nO,
           launch_dep(a.dep, col_pass2_kernel<LL, -1, float, true>, g2, NT, sm2, st, a);
         else if (a.fp32)
           launch_dep(a.dep, col_pass2_kernel<LL, -1, float>, g2, NT, sm2, st, a);
-        else if (!a.occ4 && a.curl)
-          launch_dep(a.dep, col_pass2_kernel<LL, 1, double, false, true>, g2, NT, sm2, st, a);
-        else if (!a.occ4 && a.inverse)
-          launch_dep(a.dep, col_pass2_kernel<LL, 1>, g2, NT, sm2, st, a);
-        else if (!a.occ4)
+        else if (!a.inverse && !a.held)
           launch_dep(a.dep, col_pass2_kernel<LL, -1>, g2, NT, sm2, st, a);
-        if (slab || a.fp32 || !a.occ4) return cudaGetLastError();
+        if (slab || a.fp32 || (!a.inverse && !a.held)) return cudaGetLastError();
       }
       if (a.curl) {
         const dim3 gf = a.fields_fast ? dim3(g2.z, g2.x, g2.y) : g2;
-        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, true>, gf, NT, sm2, st, a);
+        launch_dep(a.dep, col_pass2_held_kernel<LL, 1, true>, gf, NT, sm2, st, a);
       } else if (a.inverse)
-        launch_dep(a.dep, col_pass2_occ4_kernel<LL, 1, false>, g2, NT, sm2, st, a);
+        launch_dep(a.dep, col_pass2_held_kernel<LL, 1, false>, g2, NT, sm2, st, a);
       else
-        launch_dep(a.dep, col_pass2_occ4_kernel<LL, -1, false>, g2, NT, sm2, st, a);
+        launch_dep(a.dep, col_pass2_held_kernel<LL, -1, false>, g2, NT, sm2, st, a);
       return cudaGetLastError();
     });
   }
@@ -797,8 +795,9 @@ cudaError_t launch_x_fwd(const XPhysArgs& a, const double* phys, double2* spec,
 // ---------------------------------------------------------------------------
 // Periodic first inverse pass (y) with the spectral curl fused.
 // ---------------------------------------------------------------------------
-// FP32 form: the state columns and the curl stay FP64 (su); the transform
-// buffers, twiddles and the output pass buffer are FP32.
+// FP32 form (a Stockham variant chosen for the FP64 passes before the precision was
+// set): the state columns and the curl stay FP64 (su); the transform buffers,
+// twiddles and the output pass buffer are FP32.
 size_t yinv_smem(int My, int NY1, int fp32) {
   const size_t cb = fp32 ? sizeof(float2) : sizeof(double2);
   return sizeof(double2) * (size_t)(3 * NY1 * kTile) + cb * (size_t)(2 * My * kTile + My);
@@ -1315,14 +1314,13 @@ cudaError_t set_pass_attributes(int max_smem) {
         allow({(const void*)yinv_kernel<LL, float>, (const void*)yfwd_kernel<LL, float>});
     }
     if (col_pass2_smem(LL) <= kDefaultSmem) return;
-    allow({(const void*)col_pass2_occ4_kernel<LL, 1, true>,
-           (const void*)col_pass2_occ4_kernel<LL, 1, false>,
-           (const void*)col_pass2_occ4_kernel<LL, -1, false>,
+    allow({(const void*)col_pass2_held_kernel<LL, 1, true>,
+           (const void*)col_pass2_held_kernel<LL, 1, false>,
+           (const void*)col_pass2_held_kernel<LL, -1, false>,
            (const void*)zinv_curl2_kernel<LL>});
     if constexpr (fp32_length(LL))
       allow({(const void*)zinv_curl2_kernel<LL, double, true>,
-             (const void*)col_pass2_kernel<LL, 1>, (const void*)col_pass2_kernel<LL, -1>,
-             (const void*)col_pass2_kernel<LL, 1, double, false, true>,
+             (const void*)col_pass2_kernel<LL, -1>,
              (const void*)col_pass2_kernel<LL, 1, double, false, false, true>});
   });
 #undef DNSB_STOCKHAM

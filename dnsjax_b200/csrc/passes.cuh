@@ -113,10 +113,10 @@ struct ColPassArgs {
   const double* kx;
   const double* ky;
   const double* kz;
-  // curl, occ4: the blocks of a column tile's six fields next to one another, so
+  // curl in FP64: the blocks of a column tile's six fields next to one another, so
   // that the components that several fields read come from L2
   int fields_fast;
-  int occ4;  // FP64 two-stage pass with its registers held (always beyond fp32_length)
+  int held;  // FP64 two-stage forward pass at fp32_length with its registers held
   // Slab store (inverse, FP64 two-stage pass): position t goes to
   // slab.buf[t / blk] + f*fs + o*out_os + (t % blk)*ts + off + i, instead of
   // out + f*out_fs + o*out_os + t*out_ts + i.
@@ -312,7 +312,7 @@ __device__ __forceinline__ int ens_find(const int* __restrict__ base, int n, int
   return lo;
 }
 size_t ens_col_smem(int maxL);
-size_t ens_x_smem(int maxL, int maxNKX);
+size_t ens_x_smem(int maxL);
 // kind 0: inverse pass with the spectral curl, 1: inverse, 2: forward
 // (column passes); 3: the x pass; 4: the y forward pass with the projection.
 // wide: a member's padded length is 192.  base[k]: first virtual block of item k.

@@ -141,7 +141,8 @@ cudaError_t launch_periodic_correct(const PeriodicPointArgs& a,
                                     const double2* rhs_next, double2* pred_out,
                                     double2* corr_out, double* partials,
                                     cudaStream_t st) {
-  launch_dep(a.dep, periodic_correct_kernel, kRedBlocks, kRedThreads, 0, st,  a, pred, rhs_prev, rhs_next, pred_out, corr_out, partials);
+  launch_dep(a.dep, periodic_correct_kernel, kRedBlocks, kRedThreads, 0, st, a, pred, rhs_prev,
+             rhs_next, pred_out, corr_out, partials);
   return cudaGetLastError();
 }
 
@@ -197,9 +198,9 @@ cudaError_t launch_periodic_stats(const PeriodicPointArgs& a,
   return cudaGetLastError();
 }
 
-// u - grad(inv_lapl div u), then (zero_mean) the mean mode set to zero.
+// u - grad(inv_lapl div u), then the mean mode set to zero.
 __device__ __forceinline__ void periodic_cv_body(const PeriodicPointArgs& a, const double2* in,
-                                                 double2* out, int divergence, int zero_mean,
+                                                 double2* out, int divergence,
                                                  int vb, int vgrid) {
   const int S = a.S;
   for (int s = vb * blockDim.x + threadIdx.x; s < S; s += vgrid * blockDim.x) {
@@ -210,7 +211,7 @@ __device__ __forceinline__ void periodic_cv_body(const PeriodicPointArgs& a, con
       const int iy = s / (a.NKX * a.NZ1);
       project_mode(u, a.kx[ix], a.ky[iy], a.kz[iz], a.inv_lapl[s]);
     }
-    if (s == 0 && zero_mean && a.kx0) {
+    if (s == 0 && a.kx0) {
       u[0] = u[1] = u[2] = make_double2(0.0, 0.0);
     }
     out[s] = u[0];
@@ -221,15 +222,14 @@ __device__ __forceinline__ void periodic_cv_body(const PeriodicPointArgs& a, con
 
 __global__ void periodic_cv_kernel(PeriodicPointArgs a,
                                    const double2* in, double2* out,
-                                   int divergence, int zero_mean) {
-  if (a.skip && *a.skip) return;
-  periodic_cv_body(a, in, out, divergence, zero_mean, blockIdx.x, gridDim.x);
+                                   int divergence) {
+  periodic_cv_body(a, in, out, divergence, blockIdx.x, gridDim.x);
 }
 
 cudaError_t launch_periodic_correct_velocity(const PeriodicPointArgs& a,
                                              const double2* in, double2* out,
                                              int divergence, cudaStream_t st) {
-  periodic_cv_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(a, in, out, divergence, 1);
+  periodic_cv_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(a, in, out, divergence);
   return cudaGetLastError();
 }
 
@@ -244,7 +244,7 @@ __device__ __forceinline__ bool ens_skip(const int* active, int m) {
 
 __global__ void __launch_bounds__(kRedThreads)
 ens_point_kernel(const EnsPointItem* __restrict__ items, int n, const int* __restrict__ active,
-                 int op, int divergence, int zero_mean) {
+                 int op, int divergence) {
   const int total = n * kRedBlocks;
   for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
     const int k = vb / kRedBlocks, b = vb % kRedBlocks;
@@ -256,7 +256,7 @@ ens_point_kernel(const EnsPointItem* __restrict__ items, int n, const int* __res
         periodic_correct_body(it.a, it.in0, it.in1, it.in2, it.out, nullptr, it.partials, b,
                               kRedBlocks);
       else
-        periodic_cv_body(it.a, it.in0, it.out, divergence, zero_mean, b, kRedBlocks);
+        periodic_cv_body(it.a, it.in0, it.out, divergence, b, kRedBlocks);
     }
     __syncthreads();
   }
@@ -271,8 +271,8 @@ ens_finalize_kernel(const EnsPointItem* __restrict__ items, const int* __restric
 }
 
 cudaError_t launch_ens_point(const EnsPointItem* items, int n, const int* active, int op,
-                             int divergence, int zero_mean, int grid, cudaStream_t st) {
-  ens_point_kernel<<<grid, kRedThreads, 0, st>>>(items, n, active, op, divergence, zero_mean);
+                             int divergence, int grid, cudaStream_t st) {
+  ens_point_kernel<<<grid, kRedThreads, 0, st>>>(items, n, active, op, divergence);
   return cudaGetLastError();
 }
 

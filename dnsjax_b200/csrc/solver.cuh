@@ -30,17 +30,16 @@ struct PeriodicPointArgs {
   const double* lapl;
   double c;
   int kx0;  // 1: local kx index 0 is the kx = 0 mode (weight 1 in the norms; else 2)
-  // Unrolled step-graph iterations: when non-null and *skip != 0, the
-  // correct and projection kernels return at once (the work-list forms
-  // ignore it).
+  // Unrolled step-graph iterations: when non-null and *skip != 0, the correct
+  // kernel returns at once (the work-list form ignores it).
   const int* skip = nullptr;
   int dep = 0;  // launch_dep
 };
 
 // One member's pointwise call in an ensemble work list: predict (op 0:
 // out = (in0 ldt_1 + in1) ildt_2), correct (op 1: out = in0 + c (in2 - in1)
-// ildt_2, the norm partials into `partials`), correct_velocity / projection
-// (op 2: in0 -> out).
+// ildt_2, the norm partials into `partials`), correct_velocity (op 2:
+// in0 -> out).
 struct EnsPointItem {
   PeriodicPointArgs a;
   const double2* in0;
@@ -51,7 +50,7 @@ struct EnsPointItem {
   int member;
 };
 cudaError_t launch_ens_point(const EnsPointItem* items, int n, const int* active, int op,
-                             int divergence, int zero_mean, int grid, cudaStream_t st);
+                             int divergence, int grid, cudaStream_t st);
 // err[member] = sqrt(sum of the member's kRedBlocks partials), one block each.
 cudaError_t launch_ens_finalize(const EnsPointItem* items, int n, const int* active,
                                 double* err, cudaStream_t st);
@@ -149,7 +148,8 @@ struct ImmBatch {
   int NP;        // items: (nz-1+1)/2 * nx/2 when paired, else all modes
   int nu;        // stored superdiagonals (kl+1 or 2 kl)
   int paired;    // mirror mode (nz-1-s, kx) reads item (s, kx)'s factors
-  int max_smem;  // per-CTA shared-memory limit of the device
+  int max_smem;
+  int sms;  // multiprocessors  // per-CTA shared-memory limit of the device
   int* status;   // bit 1: bad pivot, bit 2: a substitution ring wait timed out
   int wait_limit;  // polls of a ring slot's mbarrier before the wait gives up
   double2* F;

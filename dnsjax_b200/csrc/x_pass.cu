@@ -476,8 +476,7 @@ int ens_x_blocks(const XPassArgs& a) {
   return (a.nrows + R - 1) / R;
 }
 
-size_t ens_x_smem(int maxL, int maxNKX) {
-  (void)maxNKX;  // maxL / 3
+size_t ens_x_smem(int maxL) {
   return maxL == 48   ? XLayout<48>::bytes
          : maxL == 72 ? XLayout<72>::bytes
          : maxL == 96 ? XLayout<96>::bytes

@@ -48,7 +48,7 @@ __device__ __forceinline__ ColumnRows column_rows(int col) {
   return {2, 2 * (col - NR), 2, 2 * (col - NR) + 1};
 }
 
-template <int NR, int NT>
+template <int NR>
 __device__ __forceinline__ int row_offsets(const XPhysArgs& a, long long* s_spec,
                                            long long* s_phys) {
   const int r0 = blockIdx.x * NR;
@@ -73,7 +73,7 @@ x_phys2_kernel(XPhysArgs a) {
   double2* tw = sm + LY::SZ_I;
   __shared__ long long s_spec[NR], s_phys[NR];
   const int tid = threadIdx.x;
-  const int nr = row_offsets<NR, NT>(a, s_spec, s_phys);
+  const int nr = row_offsets<NR>(a, s_spec, s_phys);
   for (int i = tid; i < M; i += NT) cp_async16(tw + i, a.tw + i);
   __syncthreads();
   const unsigned long long drop = l2_drop();
@@ -203,7 +203,7 @@ x_fwd2_kernel(XPhysArgs a, const double* __restrict__ phys, double2* __restrict_
   double2* tw = sm + LY::SZ_F;
   __shared__ long long s_spec[NR], s_phys[NR];
   const int tid = threadIdx.x;
-  const int nr = row_offsets<NR, NT>(a, s_spec, s_phys);
+  const int nr = row_offsets<NR>(a, s_spec, s_phys);
   for (int i = tid; i < M; i += NT) cp_async16(tw + i, a.tw + i);
   cp_async_commit();
   cp_async_wait_all();

@@ -25,10 +25,12 @@ struct YShape {
   // FP32 at 192: 24 x 8 in 192 threads (128^3 RHS 213.8 us; 12 x 16: 215.6)
   static constexpr int R1 = F32 && M == 192 ? 24 : ColRadix<M>::R1, R2 = M / R1;
   static constexpr int NF = R2 * C, NT = 3 * NF;
-  // registers: 24 warps per SM where at most 16 FP64 values a thread fit 80 of
-  // them and the CTA is not small anyway (192 points against 12 warps of 24 x 8:
-  // 128^3 RHS 328.1 -> 320.2 us; 108 points: 96 x 72 x 144 RHS 179.5 -> 176.8 us;
-  // at 72 points 90 registers are better, 48 x 48 x 96 RHS 55.4 us against 56.1)
+  // registers: held to as many whole CTAs as 768 threads hold where at most 16 FP64
+  // values a thread fit (192 points: 2 CTAs, 24 warps per SM, against 12 warps of 24 x
+  // 8: 128^3 RHS 328.1 -> 320.2 us; 108 points: 3 CTAs, 21 warps: 96 x 72 x 144 RHS
+  // 179.5 -> 176.8 us; 144 points: 2 CTAs, 18 warps).  CTAs of up to 192 threads need
+  // no more than 2 asked for: at 72 points 90 registers are better, 48 x 48 x 96 RHS
+  // 55.4 us against 56.1
   static constexpr int MINB = NT <= 192 ? 2 : !F32 && R1 <= 16 ? 768 / NT : 1;
 };
 
@@ -181,7 +183,9 @@ int ens_y_blocks(EnsYItem* it, bool wide) {
   return wide && it->L != 192 ? (it->blocks + 1) / 2 : it->blocks;
 }
 
-size_t ens_y_smem(int maxL) { return sizeof(double2) * (size_t)(3 * maxL * YShape<192, double>::C); }
+size_t ens_y_smem(int maxL) {
+  return sizeof(double2) * (size_t)(3 * maxL * YShape<192, double>::C);
+}
 
 int ens_y_threads(bool wide) { return ens_y_shape(wide); }
 
