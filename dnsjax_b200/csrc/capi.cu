@@ -138,14 +138,15 @@ struct dnsb_periodic {
 
   bool graph = false;  // a step graph is being captured
 
-  // Dependent launches for the kernels of a call on small grids, where the gaps
-  // between kernels count (24 x 36 x 48 predict_and_correct 81 -> 70 us, 96 x 72 x
-  // 144 RHS 199 -> 190 us, 128^3 FP32 RHS 225 -> 218 us); on larger ones the early
-  // blocks of the next kernel cost more than the gap (128^3 FP64 RHS 332 -> 337
-  // us, 256^3 3.28 -> 3.39 ms).  Not inside step graphs, whose edges are as short
-  // without (32^3 step 173 us without, 176 with).
+  // Dependent launches for the kernels of a call, where the gaps between kernels
+  // count.  FP64 RHS: 72 x 96 x 96 137.2 -> 127.1 us, 96 x 72 x 144 (3.4 million padded
+  // points) 183.0 -> 175.4, 96 x 128 x 128 (5.3) 260.4 -> 251.6, 108 x 128 x 144 (6.7)
+  // 406.3 -> 400.0, 128^3 (7.1) 318.7 -> 326.2, 256^3 3.28 -> 3.39 ms: on large grids the
+  // early blocks of the next kernel cost more than the gap, which the line keeps clear
+  // of.  FP32, at most 128^3: 64^3 43.4 -> 39.9 us, 128^3 221.0 -> 212.5.  Not inside
+  // step graphs, whose edges are as short without (32^3 step 173 us without, 176 with).
   int dep() const {
-    return !graph && (long long)Mx * My * Mz <= (rhs_fp32 ? 192LL * 192 * 192 : 4000000LL);
+    return !graph && (rhs_fp32 || (long long)Mx * My * Mz <= 4000000);
   }
 
   PeriodicPointArgs point() const {
@@ -342,9 +343,12 @@ static ColPassArgs periodic_ycurl(const dnsb_periodic* p, const void* state) {
   yc.kx = p->kx;
   yc.ky = p->ky;
   yc.kz = p->kz;
-  // beyond a few waves of blocks (128^3 RHS 359 -> 347 us, 256^3 3285 -> 3193; a
-  // 32^3 step took 174 -> 177 us so)
-  yc.fields_fast = (long long)p->NKX * p->NZ1 >= 4096;
+  // Where the state and the six fields together are beyond what L2 holds of them
+  // beside the rest: RHS at 20 MB (256 x 24 x 36) 52.3 -> 53.2 us so, at 37 MB (128 x
+  // 32 x 72) 56.4 -> 56.8, at 49 MB (128 x 64 x 64) 87.6 -> 87.8; at 74 MB (64 x 192 x
+  // 64) 161.9 -> 144.6, (192 x 64 x 64) 144.7 -> 142.7, at 112 MB (128 x 96 x 96) 185.1
+  // -> 182.5, at 128^3 328 -> 317, 256^3 3282 -> 3166.
+  yc.fields_fast = 16LL * p->NKX * p->NZ1 * (3LL * p->NY1 + 6LL * p->My) > 64000000LL;
   return yc;
 }
 
@@ -1369,10 +1373,16 @@ struct dnsb_couette {
 
   bool graph = false;  // a step graph is being captured
 
-  // Dependent launches, as dnsb_periodic::dep (128 x 129 x 128 RHS 203 us without,
-  // 207 with; 64 x 65 x 64 predict_and_correct 221 -> 200 us).
+  // Dependent launches, as dnsb_periodic::dep.  FP64 RHS: 64 x 129 x 96 86.2 -> 81.2
+  // us, 96 x 129 x 128 (3.6 million padded points) 154.0 -> 150.2, 128 x 97 x 128 (3.6)
+  // 144.7 -> 144.8, 128 x 113 x 128 (4.2) 165.5 -> 166.4, 128 x 129 x 128 185.9 -> 187.6.
+  // FP32 RHS: 64 x 129 x 64 43.6 -> 42.0, 128 x 129 x 128 135.7 -> 130.5, 128 x 161 x 128
+  // 165.9 -> 159.1, 128 x 385 x 128 367.2 -> 364.1.  Influence-matrix iteration: 64 x 65 x
+  // 64 68.1 -> 61.0, 128 x 129 x 128 198.7 -> 192.8; beyond the line the iteration by
+  // itself gains 2% (144 x 111 x 192: 257.5 -> 252.3), though predict_and_correct there
+  // took 1298 -> 1310 us with it.
   int dep_rhs() const {
-    return !graph && (long long)Mx * Mz * Ny <= (rhs_fp32 ? 192LL * 192 * 129 : 4000000LL);
+    return !graph && (rhs_fp32 || (long long)Mx * Mz * Ny <= 4000000);
   }
   int dep_imm() const { return !graph && (long long)NM * Ny <= 1200000; }
 
@@ -1711,9 +1721,16 @@ static int couette_rhs_impl(dnsb_couette* p, const void* state, void* rhs, unsig
   zi.NKX = p->NKX;
   zi.Ny = p->Ny;
   zi.curl = 1;
-  // as in periodic_ycurl (128 x 129 x 128 RHS 200.7 -> 190.6 us, 144 x 113 x 144
-  // predict_and_correct 989 -> 937); tiles are the grid's y extent then
-  zi.fields_fast = (long long)p->NKX * p->Ny >= 4096 && (long long)p->NKX * p->Ny <= 8 * 65535LL;
+  // As in periodic_ycurl, the line further out: the stencils of neighbouring columns
+  // share rows.  RHS at 86 MB (96 x 97 x 96) 86.7 -> 89.3 us so, at 101 MB (128 x 129 x
+  // 64) 96.9 -> 97.3, at 115 MB (128 x 73 x 128) 111.0 -> 112.2; at 126 MB (108 x 113 x
+  // 108) 152.6 -> 149.4, at 203 MB (128 x 129 x 128) 197.1 -> 185.6.  FP32 fields: at 64
+  // MB (128 x 65 x 128) 70.0 -> 72.1, at 79 MB (128 x 81 x 128) 88.2 -> 86.9, at 126 MB
+  // (128 x 129 x 128) 139.6 -> 130.6.  Tiles are the grid's y extent then.
+  const long long cols = (long long)p->NKX * p->Ny;
+  zi.fields_fast = cols * (48LL * p->NZ1 + (p->rhs_fp32 ? 48LL : 96LL) * p->Mz) >
+                       (p->rhs_fp32 ? 72000000LL : 120000000LL) &&
+                   cols <= 8 * 65535LL;
   zi.s1 = p->s1;
   zi.d1_j0 = p->d1j0;
   zi.d1_w = p->d1w;

@@ -26,13 +26,14 @@ def dev(a):
 
 # grid of each flow family: several column tiles, a partly filled last one
 PERIODIC_GRIDS = [
-    (36, 24, 72), (36, 72, 24), (72, 96, 144), (108, 36, 108),
-    (128, 24, 72),   # a tile's fields next to one another: (nx / 2)(nz - 1) >= 4096
+    (36, 24, 72), (36, 72, 24), (108, 36, 108), (128, 24, 72),
+    # a tile's fields next to one another: state and pass buffer beyond 64 MB
+    (72, 96, 144),
     (72, 192, 128),  # the same with the 8-column tiles of 288 points
 ]
 COUETTE_GRIDS = [
     (36, 33, 72), (108, 21, 96), (72, 19, 256),
-    (144, 65, 144),  # a tile's fields next to one another: (nx / 2) ny >= 4096
+    (144, 65, 144),  # a tile's fields next to one another: beyond 120 MB
     (96, 97, 192),   # the same with 8-column tiles
 ]
 
