@@ -462,7 +462,10 @@ static size_t imm_batch_assemble_smem(int Ny) {
   return sizeof(double2) * (size_t)(assemble_stride(Ny) * kStageWarps);
 }
 
-// Rows per lane of the stage kernel (odd): 32 lanes cover Ny rows.
+// Rows per lane of the stage kernel (odd): 32 lanes cover Ny rows.  17 rows (289 to
+// 512 points) do not fit the registers (255, 1.9 KB of spills); the iteration is still
+// far ahead of the single-kernel form there: 64 x 301 x 64 at order 6 2487 -> 573 us, 48
+// x 401 x 48 at order 4 2390 -> 432, 24 x 511 x 24 at order 4 1302 -> 327.
 constexpr int kMaxNy = 512;  // four modes' rows fit in shared memory
 // Back substitution with pre-scaled U (see the substitution kernel's comment).
 constexpr int kMaxScaled = 160;

@@ -18,10 +18,10 @@ constexpr int kTile = 8;     // columns per CTA in the column passes
 constexpr int kXRows = 4;    // physical rows per CTA in the x pass
 constexpr int kPassThreads = 256;
 
-// Padded lengths with two-stage register passes in FP64: 3 m for every m =
-// 2^a 3^b from 12 to 72 and 96, 128 (mode counts 24 to 256); the others run
-// Stockham stages.  The FP32, slab and work-list forms are compiled for
-// fp32_length alone.
+// Padded lengths with two-stage register passes in FP64: those of 3/2 padding from 24
+// to 256 modes (3 x 2^a 3^b points; odd lengths, 81 and 243, are refused) but 324 (216
+// modes); the others run Stockham stages (216^3 RHS 7.75 ms).  The FP32, slab
+// and work-list forms are compiled for fp32_length alone.
 __host__ __device__ constexpr bool fp32_length(int L) {
   return L == 48 || L == 72 || L == 96 || L == 192;
 }

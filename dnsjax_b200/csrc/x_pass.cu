@@ -17,8 +17,11 @@
 // output: each stage reads its input into registers, waits for every thread,
 // then writes its output over it.
 //
-// Bound (128^3 Kolmogorov, M = 192): shared-memory wavefronts, then FP64 issue
-// and latency at 15 warps per SM; the 340 MB it moves would take 51 us.
+// Bound (128^3 Kolmogorov, M = 192, 132 us cold): latency.  Nothing is saturated at
+// the 15 warps per SM that 128 registers leave: shared-memory data pipe 56% busy, FP64
+// pipe 40%, issue slots 44%, DRAM 24% (the 340 MB it moves would take 51 us); a warp
+// waits on shared-memory loads, fixed latencies and barriers alike.  FP32 (8 CTAs per
+// SM, 85 us): shared memory 67%, issue 69%.
 // Twiddles applied where they are already at hand (they had cost stage C 23
 // loads a thread beside its 24 values), the zero-padded third left out of the
 // inverse DFTs and the truncated third out of the forward ones, the third
